@@ -106,10 +106,8 @@ extern "C" int vcpcu_igemm_noalloc_dev(int m, int n, int k, const double* A, int
   OzWorkspace ws;
   oz_carve_workspace(plan.pb, base, &ws);
   if ((st = oz_run_product(plan, ws, A, lda, B, ldb, C, ldc, s))) return st;
-  // The reassembly already writes NaN everywhere after a non-finite input or
-  // a timed-out wait; the status words go into the per-device status that
-  // vcpcu_status reports, as for vcpcu_igemm_dev.
-  oz_merge_status(ws.flag, s);
-  VCPCU_LAUNCH_CHECK("oz_status_merge");
+  // The reassembly writes NaN everywhere after a non-finite input or a
+  // timed-out wait and merges the status words into the per-device status
+  // that vcpcu_status reports, as for vcpcu_igemm_dev.
   return VCPCU_OK;
 }

@@ -88,16 +88,6 @@ void choose_scaling(const OzPairList& pl, int nchunks, int* t_ref, int* R) {
 
 size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Sticky per-device status of the Ozaki form: bit 0 non-finite input, bit 1
-// a bounded device wait timed out.  Merged after every product, read and
-// cleared by oz_take_status.
-__device__ int g_oz_status;
-
-__global__ void oz_status_merge(const int* flag) {
-  int v = (flag[0] ? 1 : 0) | (flag[1] ? 2 : 0);
-  if (v) atomicOr(&g_oz_status, v);
-}
-
 // Optional per-phase timing (CUDA events recorded on the call's stream).
 struct OzProfile {
   bool on = false;
@@ -180,37 +170,7 @@ int oz_selftest_timeout(long long limit, cudaStream_t s) {
   return VCPCU_OK;
 }
 
-void oz_merge_status(const int* flag, cudaStream_t s) {
-  oz_status_merge<<<1, 1, 0, s>>>(flag);
-  count_launch();
-}
-
-int* oz_status_ptr() {
-  static std::mutex mu;
-  static int* ptr[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!ptr[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_oz_status) != cudaSuccess) return nullptr;
-    ptr[dev] = (int*)p;
-  }
-  return ptr[dev];
-}
-
-int oz_take_status(cudaStream_t s, int* status) {
-  int zero = 0;
-  VCPCU_CUDA_TRY(cudaMemcpyFromSymbolAsync(status, g_oz_status, sizeof(int), 0,
-                                           cudaMemcpyDeviceToHost, s));
-  VCPCU_CUDA_TRY(cudaStreamSynchronize(s));
-  VCPCU_CUDA_TRY(cudaMemcpyToSymbolAsync(g_oz_status, &zero, sizeof(int), 0,
-                                         cudaMemcpyHostToDevice, s));
-  VCPCU_CUDA_TRY(cudaStreamSynchronize(s));
-  return VCPCU_OK;
-}
-
-// CRT form: number of moduli L and basis Q_l for w-bit operands and inner
+// CRT form: number of moduli L and their basis for w-bit operands and inner
 // dimension K: the product A'B' satisfies |A'B'| <= K 2^(2w-2); the moduli
 // are taken with prod m_l > K 2^(2w) = 4 max |A'B'|, so the centred value
 // lies within a quarter of M of zero and the reassembly's quotient needs no
@@ -222,22 +182,7 @@ int crt_setup(int K, int w, OzPlan* plan) {
   int L = 0;
   while (L < OZ_MAX_MODULI_128 && bits <= need) bits += std::log2((double)OZ_MODULI[L++]);
   if (bits <= need) return -1;
-  unsigned __int128 Mv = 1;
-  for (int l = 0; l < L; ++l) Mv *= (unsigned __int128)OZ_MODULI[l];
-  for (int l = 0; l < L; ++l) {
-    const int m = OZ_MODULI[l];
-    const unsigned __int128 Ml = Mv / (unsigned __int128)m;
-    const int r = (int)(Ml % (unsigned __int128)m);
-    int inv = 0;
-    for (int x = 1; x < m; ++x)
-      if ((r * x) % m == 1) {
-        inv = x;
-        break;
-      }
-    const unsigned __int128 Q = Ml * (unsigned __int128)inv;  // < M
-    for (int t = 0; t < 4; ++t) plan->Q[l][t] = (uint32_t)(Q >> (32 * t));
-  }
-  for (int t = 0; t < 4; ++t) plan->Mlimb[t] = (uint32_t)(Mv >> (32 * t));
+  crt_basis(L, &plan->basis);
   plan->pb.L = L;
   return 0;
 }
@@ -416,7 +361,10 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const double* A, long ld
   }
   if (plan.pb.crt) {
     PhaseTimer t(4, s);
-    if ((st = oz_crt_assemble(plan, ws, C, ldc, s))) return st;
+    if ((st = oz_crt_assemble(plan, ws, C, ldc, s, true))) return st;
+  } else {
+    oz_merge_status(ws.flag, s);
+    VCPCU_LAUNCH_CHECK("oz_status_merge");
   }
   return VCPCU_OK;
 }
@@ -599,7 +547,6 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
     v.delta = ws.delta + i0;
     v.asum = ws.asum + 4 * (size_t)i0;
     v.F2 = ws.F2 + 2 * (size_t)j0;
-    v.beta = ws.beta + j0;
     v.bsum = ws.bsum + 4 * (size_t)j0;
     const bool odd = (nblk++ & 1) != 0;
     cudaStream_t c = odd ? c1 : c0;
@@ -611,7 +558,7 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
     if ((e = pipe_event(g, s, c))) return e;
     if ((e = oz_run_gemm(pj, OZ_ALL, v, nullptr, 0, c))) return e;
     double* cblk = dC + 2 * ((size_t)i0 + (size_t)j0 * m);
-    if ((e = oz_crt_assemble(pj, v, cblk, m, c))) return e;
+    if ((e = oz_crt_assemble(pj, v, cblk, m, c, false))) return e;
     if ((e = pipe_event(g, c, down))) return e;
     VCPCU_CUDA_TRY(cudaMemcpy2DAsync(C + 2 * ((size_t)i0 + (size_t)j0 * m), m * rowb, cblk,
                                      m * rowb, mv * rowb, wj, cudaMemcpyDeviceToHost, down));
@@ -690,8 +637,6 @@ int ozaki_igemm(int m, int n, int k, const double* A, long lda, const double* B,
   oz_profile_add_flops(2LL * m * n * (long long)(k > 0 ? k : 0) *
                        ((plan.pb.crt ? plan.pb.L : plan.mid.npairs) +
                         (long long)(!(point_mask & 2) + !(point_mask & 1)) * plan.rad.npairs));
-  oz_status_merge<<<1, 1, 0, s>>>(ws.flag);
-  VCPCU_LAUNCH_CHECK("oz_status_merge");
   return VCPCU_OK;
 }
 

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "ozaki_crt.cuh"
+
 namespace vcpcu {
 
 constexpr int OZ_MAX_SLICES = 12;
@@ -36,7 +38,7 @@ struct OzWorkspace {
   int* E3;                            // [Mp][3] exponents Em, Ep, Er
   unsigned long long* delta;          // [Mp] sum of |midpoint digits| per row
   int* F2;                            // [Np][2] exponents Fm, Fr
-  double* beta;                       // [Np] sum_k |mB(k,j)| rounded up
+  double* beta;                       // [Np] sum_k |mB(k,j)| rounded up (slice form)
   unsigned long long* asum;           // [Mp][4] CRT form: sum_k |A'(i,k)| as (bits >= 32, bits < 32);
                                       // sum_k lo^2 of the low radius digits of P, of rA
   uint8_t* res;                       // [L][Np][Mp] CRT form: residues of A'B' mod m_l
@@ -118,8 +120,7 @@ struct OzPlan {
   OzProblem pb;
   OzPairList mid, rad, crt;
   int t_ref_mid, R_mid, t_ref_rad, R_rad;
-  uint32_t Q[16][4];   // CRT basis: Q_l = (M/m_l) * ((M/m_l)^-1 mod m_l), 32-bit limbs
-  uint32_t Mlimb[4];   // M = prod m_l
+  CrtBasis basis;      // of the L moduli (CRT form)
   // bit 0: A is a point matrix (rA = 0), bit 1: B is (rB = 0).  The radius
   // product with a zero factor is skipped; it would add exactly 0 to T.
   int point_mask = 0;
@@ -149,8 +150,9 @@ int oz_radius_T(const OzPlan& plan, const OzWorkspace& ws, cudaStream_t st);
 // s may carry OZ_FAST_RADIUS (CRT form: the radius products leave out
 // their low x low digit pair) and is then 0 for the default 8.
 int oz_make_plan(int M, int N, int K, int s, int sr, OzPlan* plan, int crt = 0);
+// merge_status: the kernel also merges ws.flag into the sticky status.
 int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long ldc,
-                    cudaStream_t st);
+                    cudaStream_t st, bool merge_status);
 int oz_prepare(const OzProblem& pb, const double* A, long lda, const double* B, long ldb,
                OzWorkspace& ws, cudaStream_t st);
 // oz_prepare in parts: clear the row maxima, sums and status words; midrad
@@ -185,9 +187,6 @@ int oz_take_status(cudaStream_t s, int* status);
 int oz_selftest_timeout(long long limit, cudaStream_t s);
 // Merge a product's status words into the sticky device status.
 void oz_merge_status(const int* flag, cudaStream_t s);
-// Device address of the sticky status word of the current device (kernels
-// that merge statuses themselves atomicOr into it); null on error.
-int* oz_status_ptr();
 
 // dd GEMM (pddblas semantics) by the CRT form: C, Cerr as documented in
 // include/vcpcuda.h.  static_scratch != nullptr: use that device buffer of
@@ -240,10 +239,9 @@ struct OzGProb {
   int tiles_m, tiles_n;
   long long res_off, P_off;    // element offsets into the bucket's res / P
   int orig;                    // index in the caller's problem table
-  uint32_t Q[16][4];           // CRT basis of this problem's L moduli
-  uint32_t Mlimb[4];
-  float invMf;                 // 2^64 / M rounded to float
 };
+
+constexpr int OZ_GASM_COLS = 16;  // columns of a reassembly block of a bucket
 
 // Device view of one bucket (all pointers device memory).
 struct OzGBucket {
@@ -255,7 +253,7 @@ struct OzGBucket {
   const int* item_crt;     // [nprob + 1] prefix of residue work items (L x tiles)
   const int* prob_rad;     // [radius items] the problem of each item
   const int* prob_crt;     // [residue items] the problem of each item
-  const int* blk_asm;      // [nprob + 1] prefix of reassembly blocks
+  const int* blk_asm;      // [nprob + 1] prefix of reassembly blocks (128 rows x OZ_GASM_COLS)
   const int* prob_asm;     // [reassembly blocks] the problem of each block
   const int* col_prob;     // [Ntot] problem of each stacked B column
   uint16_t* planesA;       // [Lmax + 4][Mtot][Kp]: residues, |mA|+rA digits, rA digits
@@ -263,7 +261,6 @@ struct OzGBucket {
   unsigned long long* rowmax;  // [Mtot][3]
   int* E3;                 // [Mtot][3]
   int* F2;                 // [Ntot][2]
-  double* beta;            // [Ntot]
   double *midB, *radB;     // [Ntot][Kp] midrad of the stacked B columns
   double *midA, *radA;     // [Kp][Mtot] midrad of the stacked A rows (column-major)
   unsigned long long* bsum;  // [Ntot][4] as OzWorkspace::bsum

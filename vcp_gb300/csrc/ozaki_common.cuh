@@ -214,6 +214,7 @@ OZ_HD uint16_t oz_bf16_of_int(int v) {
   return (uint16_t)(sign | ((unsigned)(e + 127) << 7) | frac);
 }
 
+#ifdef __CUDACC__
 // Paired FP32 arithmetic (sm_100 and later): two floats in one 64-bit
 // register pair, the first in the low half; each instruction rounds each
 // half to nearest exactly as the scalar instruction does, so a pair gives
@@ -244,5 +245,6 @@ __device__ __forceinline__ unsigned long long sub_x2(unsigned long long a, unsig
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+#endif
 
 }  // namespace vcpcu

@@ -13,17 +13,22 @@
 #include "common.cuh"
 #include "ozaki.cuh"
 #include "ozaki_common.cuh"
+#include "ozaki_crt.cuh"
 #include "swfp.cuh"
 
 namespace vcpcu {
 
 namespace {
 
-struct CrtConst {
-  uint32_t Q[16][4];
-  uint32_t M[4];
-  float invMf;  // 2^64 / M rounded to float: the quotient estimate of the reduction
-};
+// Sticky per-device status of the Ozaki form: bit 0 non-finite input, bit 1
+// a bounded device wait timed out.  The reassembly kernels merge their
+// product's status words; read and cleared by oz_take_status.
+__device__ int g_oz_status;
+
+__global__ void oz_status_merge(const int* flag) {
+  int v = (flag[0] ? 1 : 0) | (flag[1] ? 2 : 0);
+  if (v) atomicOr(&g_oz_status, v);
+}
 
 __device__ __forceinline__ double scale_dir2(double x, int e, bool up) {
   while (e > 1023) {
@@ -109,73 +114,6 @@ __device__ __forceinline__ void big_to_dir(const uint32_t (&mag)[4], int neg, in
   }
 }
 
-// Nearest integer of |x| < 2^22 on the FP32 pipe (ties to even).
-__device__ __forceinline__ float rint_f(float x) {
-  return __fsub_rn(__fadd_rn(x, 12582912.0f), 12582912.0f);
-}
-
-// u32 -> float rounded to nearest (equal to __uint2float_rn) on the FP32
-// pipe: the two 16-bit halves are exact floats, one FMA rounds their sum.
-__device__ __forceinline__ float u32_to_f(uint32_t v) {
-  const float h = __fsub_rn(__uint_as_float(0x4B000000u | (v >> 16)), 8388608.0f);
-  const float l = __fsub_rn(__uint_as_float(0x4B000000u | (v & 0xffffu)), 8388608.0f);
-  return __fmaf_rn(h, 65536.0f, l);
-}
-
-// Exact X = (A'B')(i, j) from its residues (see the file comment); returns
-// the magnitude in mag[4] and the sign.
-// c[l] = 0 and Q_l = 0 for l >= L.  S = sum_l c_l Q_l < 2^12 M is formed
-// exactly in five 32-bit limbs; the plan keeps |X| <= K 2^(2w-2) < M / 4
-// (prod m_l > K 2^(2w)), so S / M lies within 1/4 of the integer q with
-// S = q M + X, and the fp32 estimate of S / M (relative error below 2^-20,
-// absolute below 2^-8) rounds to exactly that q: X = S - q M in one
-// multiply-subtract, already centred, with no correction step.
-__device__ __forceinline__ int crt_value(const uint32_t (&c)[16], const uint32_t (&Q)[16][4],
-                                         const uint32_t (&Mm)[4], float invMf,
-                                         uint32_t (&mag)[4]) {
-  unsigned long long s[4] = {0, 0, 0, 0};
-#pragma unroll
-  for (int l = 0; l < 16; ++l) {
-#pragma unroll
-    for (int t = 0; t < 4; ++t) s[t] += (unsigned long long)c[l] * Q[l][t];
-  }
-  uint32_t r[5];
-  unsigned long long carry = 0;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const unsigned long long v = s[t] + carry;
-    r[t] = (uint32_t)v;
-    carry = v >> 32;
-  }
-  r[4] = (uint32_t)carry;
-  const float Sf = u32_to_f(r[4]) * 0x1p64f + u32_to_f(r[3]) * 0x1p32f + u32_to_f(r[2]) +
-                   u32_to_f(r[1]) * 0x1p-32f + u32_to_f(r[0]) * 0x1p-64f;
-  const unsigned int q = (unsigned int)rint_f(Sf * invMf);  // nearest integer to S / M
-  unsigned long long c2 = 0, borrow = 0;
-#pragma unroll
-  for (int t = 0; t < 5; ++t) {  // r = S - q M in five-limb two's complement
-    const unsigned long long v = (t < 4 ? (unsigned long long)q * Mm[t] : 0ULL) + c2;
-    c2 = v >> 32;
-    const unsigned long long d = (unsigned long long)r[t] - (uint32_t)v - borrow;
-    r[t] = (uint32_t)d;
-    borrow = (d >> 63) & 1ULL;
-  }
-  const int neg = (int)(r[4] >> 31);  // |X| < 2^125: the top limb is 0 or all ones
-  if (neg) {  // magnitude = -r
-    unsigned long long cy = 1;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const unsigned long long v = (unsigned long long)(~r[t]) + cy;
-      mag[t] = (uint32_t)v;
-      cy = v >> 32;
-    }
-  } else {
-#pragma unroll
-    for (int t = 0; t < 4; ++t) mag[t] = r[t];
-  }
-  return neg;
-}
-
 // The radius sums of both products for 4 consecutive rows (e0 = j Mp + i0):
 // one fp32 fold per product (slot 0 and slot nslot = 1), the slice GEMM
 // epilogue's upward sum of every chunk weighted by its digit pair -- an
@@ -257,202 +195,384 @@ oz_radius_T_kernel(int M, int N, int Mp, size_t plane, const int32_t* __restrict
   }
 }
 
-// Per-row data of 4 consecutive rows: the exponents, sA = RU(sum_k
-// |A'(i,k)|) (asum_hi 2^32 + asum_lo, exact below 2^96) and the 2^-8-scaled
-// roots of the low radius digits' squares of P and rA, computed once per
-// thread and reused for every column it assembles.
-struct QuadRows {
-  int E[4], Ep[4], Er[4];
-  double sA[4];
-  float qp[4], qr[4];
+// ---------------------------------------------------------------- reassembly
+//
+// A block of 256 threads takes a tile of up to 128 rows and CB columns of one
+// product; a thread owns 4 consecutive rows (their residue bytes are one
+// 32-bit word per modulus, their folds one 16-byte load per product) of every
+// CW-th column.  The per-row and per-column data -- exponents, sA = RU(sum_k
+// |A'(i,k)|), beta_j = RU((sum_k |B'(k,j)| + ceil(K/2)) 2^(F - w)), the roots
+// of the low radius digits' squares -- are formed once per block in shared
+// memory.
+//
+// Bound: five FP64 additions per entry (64 cycles of a sub-partition's FP64
+// unit per warp instruction) beside the integer arithmetic of the residues;
+// DRAM moves 40 bytes per entry.  Values that every entry of a tile shares
+// are scaled once (t1 and t2 below are an exponent add each), three residues
+// meet in one 32-bit value before the multi-limb products (ozaki_crt.cuh),
+// and the double results are put together from words.  Measured against one
+// 128-bit product per residue, 8 columns a thread and a branch per entry:
+// n = 8192 1.49 -> 0.76 ms, n = 512 48 -> 10 us (64 blocks before), 17 chunks
+// of a 256-problem batch 1.30 -> 0.54 ms summed.  80 registers (three blocks
+// per SM, a few words spilled) 756 us at n = 8192, 128 registers 815 us.
+
+constexpr int ASM_ROWS = 128, ASM_COLS = 64, ASM_NT = 256;
+// Exponents within +-ASM_EXP keep every value of an entry a normal double:
+// the path below that adds to exponent fields without looking.
+constexpr int ASM_EXP = 400;
+
+// (rows as one array per quantity: a thread reads its 4 as one vector, a
+// warp's vectors lie side by side, free of bank conflicts)
+struct alignas(16) AsmRows {
+  double sA[ASM_ROWS];                       // RU(sum_k |A'(i,k)|)
+  int E[ASM_ROWS], Ep[ASM_ROWS], Er[ASM_ROWS];  // exponents of mA, |mA| + rA, rA
+  float qp[ASM_ROWS], qr[ASM_ROWS];          // 2^-8 roots of the low digits' squares of P, rA
+};
+struct AsmCol {
+  double beta;
+  int Fm, Fr;
+  float q1, q2;     // roots of the low digits' squares of rB, |mB|
+};
+struct AsmTile {
+  AsmRows row;
+  AsmCol col[ASM_COLS];
 };
 
-__device__ __forceinline__ void quad_rows(int i0, int M, const int* __restrict__ E3,
-                                          const unsigned long long* __restrict__ asum,
-                                          QuadRows& r) {
+__device__ __forceinline__ bool asm_exp_ok(int e) { return e >= -ASM_EXP && e <= ASM_EXP; }
+// a zero radius row or column has zero folds: any exponent gives its 0
+__device__ __forceinline__ bool asm_rad_ok(int e) { return e == OZ_ZERO_EXP || asm_exp_ok(e); }
+
+// RU of asum_hi 2^32 + asum_lo (exact below 2^96).
+__device__ __forceinline__ double asum_ru(unsigned long long ah, unsigned long long al) {
+  const unsigned __int128 sx = ((unsigned __int128)ah << 32) + al;
+  if (!sx) return 0.0;
+  double dn, up;
+  const unsigned long long hi64 = (unsigned long long)(sx >> 64);
+  if (hi64 == 0) {
+    u64_to_dir((unsigned long long)sx, 0, dn, up);
+  } else {
+    const int sh = 64 - __clzll(hi64);
+    unsigned long long t = (unsigned long long)(sx >> sh);
+    if ((unsigned long long)sx & ((1ULL << sh) - 1)) t |= 1ULL;
+    u64_to_dir(t, sh, dn, up);
+  }
+  return up;
+}
+
+// The rows [i0, i0 + nr) and columns [j0, j0 + nc) of the tile.  E3, asum, F2
+// and bsum point at row / column 0 of the product.
+__device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j0, int nc, int K,
+                                               int w, int lowb, const int* __restrict__ E3,
+                                               const unsigned long long* __restrict__ asum,
+                                               const int* __restrict__ F2,
+                                               const unsigned long long* __restrict__ bsum) {
+  for (int x = threadIdx.x; x < ASM_ROWS + ASM_COLS; x += ASM_NT) {
+    if (x < ASM_ROWS) {
+      double sA = 0.0;
+      int E = OZ_ZERO_EXP, Ep = OZ_ZERO_EXP, Er = OZ_ZERO_EXP;
+      float qp = 0.0f, qr = 0.0f;
+      if (x < nr) {
+        const int i = i0 + x;
+        E = E3[3 * i];
+        Ep = E3[3 * i + 1];
+        Er = E3[3 * i + 2];
+        sA = asum_ru(asum[4 * i], asum[4 * i + 1]);
+        if (lowb) {
+          qp = lowpair_root(asum[4 * i + 2], 0x1p-8f);
+          qr = lowpair_root(asum[4 * i + 3], 0x1p-8f);
+        }
+      }
+      t.row.sA[x] = sA;
+      t.row.E[x] = E;
+      t.row.Ep[x] = Ep;
+      t.row.Er[x] = Er;
+      t.row.qp[x] = qp;
+      t.row.qr[x] = qr;
+    } else if (x - ASM_ROWS < nc) {
+      const int j = j0 + x - ASM_ROWS;
+      AsmCol c;
+      c.Fm = F2[2 * j];
+      c.Fr = F2[2 * j + 1];
+      c.beta = 0.0;
+      if (c.Fm != OZ_ZERO_EXP) {
+        const double v =
+            __fma_ru((double)bsum[4 * j], 0x1p32,
+                     (double)(bsum[4 * j + 1] + (unsigned long long)(K + 1) / 2));
+        c.beta = scale_dir2(v, c.Fm - w, true);
+      }
+      c.q1 = lowb ? lowpair_root(bsum[4 * j + 2], 1.0f) : 0.0f;
+      c.q2 = lowb ? lowpair_root(bsum[4 * j + 3], 1.0f) : 0.0f;
+      t.col[x - ASM_ROWS] = c;
+    }
+  }
+  __syncthreads();
+}
+
+// What the entries of a product read and write.  res and P point at row /
+// column 0 of the product (plane = Np Mp of its layout).
+struct AsmArgs {
+  int M, Mp, L, w;
+  const uint8_t* res;
+  size_t plane;
+  const int32_t* P;
+  double* C;
+  long ldc;
+  bool nonfinite, al16;
+};
+
+// One entry (row x of the tile, column *col, element e of its planes) whose
+// exponents leave the direct path: the same operations with every range
+// looked at, from its residues again.  Out of line, so that neither its
+// registers nor its FP64 instructions weigh on the direct path.
+static __device__ __noinline__ double2 asm_entry_general(const AsmArgs* a, size_t e,
+                                                         const AsmRows* row, int x,
+                                                         const AsmCol* col, const CrtBasis* cc,
+                                                         const OzRadConst* rc) {
+  double lo = 0.0, up = 0.0, tr = 0.0;
+  const int E = row->E[x], F = col->Fm, w = a->w;
+  if (E != OZ_ZERO_EXP && F != OZ_ZERO_EXP) {
+    uint32_t V[OZ_CRT_GROUPS], mag[4];
+#pragma unroll
+    for (int g = 0; g < OZ_CRT_GROUPS; ++g) {
+      V[g] = 0;
+#pragma unroll
+      for (int l = 0; l < 3; ++l)
+        if (3 * g + l < a->L) V[g] += a->res[(size_t)(3 * g + l) * a->plane + e] * cc->a[g][l];
+    }
+    crt_reduce(V, *cc, mag);
+    const int neg = crt_abs(mag);
+    big_to_dir(mag, neg, E + F - 2 * w - cc->z, lo, up);
+    const double t1 = scale_pow2(col->beta, E - w - 1, true);
+    const double t2 = scale_pow2(row->sA[x], E + F - 2 * w - 1, true);
+    tr = __dadd_ru(t1, t2);
+  }
+  const float S1 = rc->run1 ? __int_as_float(a->P[e]) : 0.0f,
+              S2 = rc->run2 ? __int_as_float(a->P[(size_t)rc->nslot * a->plane + e]) : 0.0f;
+  const double T = rad_T(S1, S2, row->Ep[x], row->Er[x], F, col->Fr, *rc,
+                         __fmul_ru(row->qp[x], col->q1), __fmul_ru(row->qr[x], col->q2));
+  const double err = __dadd_ru(tr, T);
+  return make_double2(__dsub_rd(lo, err), __dadd_ru(up, err));
+}
+
+// RU(s) 2^x of a fold s >= 0 as a double (0 for 0): e20 = (x + 896) << 20.
+__device__ __forceinline__ double asm_fold(float s, int e20) {
+  const unsigned u = __float_as_uint(s);
+  const bool pos = s > 0.0f;
+  const int hi = (int)(u >> 3) + e20;
+  return __hiloint2double(pos ? hi : 0, pos ? (int)(u << 29) : 0);
+}
+
+// All entries of a thread: rows i0 + 4 q .. + 3 (q = thread % Rq) of the
+// columns j0 + thread / Rq + CW c of its block.  The 4 entries of a column run
+// the direct path together without a branch between them (their FP64
+// additions overlap); where exponents leave its range they are redone.
+template <bool LOWB>
+__device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int i0, int nr,
+                                         int j0, int nc, const CrtBasis& cc,
+                                         const OzRadConst& rc) {
+  const int Rq = (nr + 3) >> 2, CW = ASM_NT / Rq;
+  const int slot = (int)threadIdx.x / Rq, q4 = 4 * ((int)threadIdx.x - slot * Rq);
+  if (slot >= CW) return;
+  const int i = i0 + q4;
+  // per-row words of the direct path
+  int E20[4], P20[4], R20[4], sAh[4], sAl[4];
+  float qp[4], qr[4];
+  bool rows_ok = rc.R == 0;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const int i = i0 + u;
-    r.E[u] = r.Ep[u] = r.Er[u] = OZ_ZERO_EXP;
-    r.sA[u] = 0.0;
-    r.qp[u] = r.qr[u] = 0.0f;
-    if (i >= M) continue;
-    r.E[u] = E3[3 * i];
-    r.Ep[u] = E3[3 * i + 1];
-    r.Er[u] = E3[3 * i + 2];
-    r.qp[u] = lowpair_root(asum[4 * i + 2], 0x1p-8f);
-    r.qr[u] = lowpair_root(asum[4 * i + 3], 0x1p-8f);
-    const unsigned long long ah = asum[4 * i + 0], al = asum[4 * i + 1];
-    const unsigned __int128 sx = ((unsigned __int128)ah << 32) + al;
-    if (sx) {
-      double sAdn;
-      const unsigned long long hi64 = (unsigned long long)(sx >> 64);
-      if (hi64 == 0) {
-        u64_to_dir((unsigned long long)sx, 0, sAdn, r.sA[u]);
-      } else {
-        const int sh = 64 - __clzll(hi64);
-        unsigned long long t = (unsigned long long)(sx >> sh);
-        if ((unsigned long long)sx & ((1ULL << sh) - 1)) t |= 1ULL;
-        u64_to_dir(t, sh, sAdn, r.sA[u]);
+    const int E = t.row.E[q4 + u], Ep = t.row.Ep[q4 + u], Er = t.row.Er[q4 + u];
+    // (rows past M hold the zero exponent; they are not stored)
+    rows_ok = rows_ok && ((asm_exp_ok(E) && asm_rad_ok(Ep) && asm_rad_ok(Er)) || i + u >= a.M);
+    E20[u] = E << 20;
+    P20[u] = ((Ep == OZ_ZERO_EXP ? 0 : Ep) - 8 * rc.t_ref + 896) << 20;
+    R20[u] = ((Er == OZ_ZERO_EXP ? 0 : Er) - 8 * rc.t_ref + 896) << 20;
+    const long long sb = __double_as_longlong(t.row.sA[q4 + u]);
+    sAh[u] = (int)(sb >> 32) + ((E - 2 * a.w - 1) << 20);  // sA 2^(E - 2 w - 1)
+    sAl[u] = (int)sb;
+    qp[u] = LOWB ? t.row.qp[q4 + u] : 0.0f;
+    qr[u] = LOWB ? t.row.qr[q4 + u] : 0.0f;
+  }
+  const int cX = (1149 - 2 * a.w - cc.z) << 20;
+  for (int c = slot; c < nc; c += CW) {
+    const int j = j0 + c;
+    const AsmCol& col = t.col[c];
+    const size_t e0 = (size_t)j * a.Mp + i;
+    uint32_t pk[3 * OZ_CRT_GROUPS];
+#pragma unroll
+    for (int l = 0; l < 3 * OZ_CRT_GROUPS; ++l)
+      pk[l] = l < a.L ? *reinterpret_cast<const uint32_t*>(a.res + (size_t)l * a.plane + e0) : 0u;
+    float S1[4], S2[4];
+    rad_folds(a.P, a.plane, e0, rc, S1, S2);
+    // group values of the 4 rows
+    uint32_t V[4][OZ_CRT_GROUPS];
+#pragma unroll
+    for (int g = 0; g < OZ_CRT_GROUPS; ++g) {
+      const uint32_t a0 = cc.a[g][0], a1 = cc.a[g][1], a2 = cc.a[g][2];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        V[u][g] = ((pk[3 * g] >> (8 * u)) & 255u) * a0 + ((pk[3 * g + 1] >> (8 * u)) & 255u) * a1 +
+                  ((pk[3 * g + 2] >> (8 * u)) & 255u) * a2;
+    }
+    const int Fm = col.Fm, Fr = col.Fr;
+    const bool direct = rows_ok && asm_exp_ok(Fm) && asm_rad_ok(Fr);
+    const int F20 = Fm << 20, Fr20 = (Fr == OZ_ZERO_EXP ? 0 : Fr) << 20;
+    const long long bb = __double_as_longlong(col.beta);
+    const int bh = (int)(bb >> 32) - ((a.w + 1) << 20), bl = (int)bb;  // beta 2^(-w - 1)
+    double2 r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      uint32_t mag[4], dn[2], up[2];
+      crt_reduce(V[u], cc, mag);
+      const int neg = crt_abs(mag);
+      crt_to_dir(mag, E20[u] + F20 + cX, dn, up);
+      // [lo, hi] = neg ? [-up, -dn] : [dn, up]
+      const uint32_t sg = (uint32_t)neg << 31;
+      const double lo = __hiloint2double((int)((neg ? up[0] : dn[0]) | sg),
+                                         (int)(neg ? up[1] : dn[1])),
+                   hi = __hiloint2double((int)((neg ? dn[0] : up[0]) | sg),
+                                         (int)(neg ? dn[1] : up[1]));
+      const double t1 = __hiloint2double(bh + E20[u], bl),
+                   t2 = __hiloint2double(sAh[u] + F20, sAl[u]);
+      double err = __dadd_ru(t1, t2);
+      float s1 = S1[u], s2 = S2[u];
+      if (LOWB) {
+        s1 = __fadd_ru(s1, __fmul_ru(qp[u], col.q1));
+        s2 = __fadd_ru(s2, __fmul_ru(qr[u], col.q2));
+      }
+      const double b1 = asm_fold(s1, P20[u] + Fr20), b2 = asm_fold(s2, R20[u] + F20);
+      // (a product that did not run adds nothing)
+      if (rc.run1 && rc.run2)
+        err = __dadd_ru(err, __dadd_ru(b1, b2));
+      else if (rc.run1)
+        err = __dadd_ru(err, b1);
+      else if (rc.run2)
+        err = __dadd_ru(err, b2);
+      r[u] = make_double2(__dsub_rd(lo, err), __dadd_ru(hi, err));
+    }
+    if (!direct) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u < a.M)
+          r[u] = asm_entry_general(&a, e0 + u, &t.row, q4 + u, &col, &cc, &rc);
+    }
+    double* cp = a.C + 2 * ((size_t)i + (size_t)j * a.ldc);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (a.nonfinite) r[u].x = r[u].y = __longlong_as_double(0x7ff8000000000000LL);
+      if (i + u >= a.M) continue;
+      if (a.al16) {
+        *reinterpret_cast<double2*>(cp + 2 * u) = r[u];
+      } else {  // C may be only 8-byte aligned
+        cp[2 * u] = r[u].x;
+        cp[2 * u + 1] = r[u].y;
       }
     }
   }
 }
 
-// The 4 entries (i0 .. i0+3, j): the residue planes are read 4 bytes at a
-// time, the radius folds 16 bytes, C written as 4 consecutive pairs.  Only
-// the final error sum and the two outward roundings use the FP64 pipe on the
-// common path.  res and P point at row / column 0 of this product; plane =
-// Np Mp of its layout; Fj, Frj the column's exponents, bj its beta, qj its
-// sums of squared low radius digits (of rB and |mB|).
-__device__ __forceinline__ void assemble_quad_col(
-    const QuadRows& rw, int i0, int j, int M, int Mp, int L, int w,
-    const uint8_t* __restrict__ res, size_t plane, int Fj, int Frj, double bj,
-    const unsigned long long* __restrict__ qj, const int32_t* __restrict__ P,
-    double* __restrict__ C, long ldc, bool nonfinite, const uint32_t (&Q)[16][4],
-    const uint32_t (&Mm)[4], float invMf, const OzRadConst& rc) {
-  const size_t e0 = (size_t)j * Mp + i0;
-  uint32_t pk[16];
-#pragma unroll
-  for (int l = 0; l < 16; ++l)
-    pk[l] = l < L ? *reinterpret_cast<const uint32_t*>(res + (size_t)l * plane + e0) : 0u;
-  float W1[4], W2[4];
-  rad_folds(P, plane, e0, rc, W1, W2);
-  const float qb1 = rc.lowb ? lowpair_root(qj[0], 1.0f) : 0.0f;
-  const float qb2 = rc.lowb ? lowpair_root(qj[1], 1.0f) : 0.0f;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = i0 + u;
-    if (i >= M) break;
-    const int Ei = rw.E[u];
-    double lo = 0.0, up = 0.0, tr = 0.0;
-    if (Ei != OZ_ZERO_EXP && Fj != OZ_ZERO_EXP) {
-      uint32_t c[16], mag[4];
-#pragma unroll
-      for (int l = 0; l < 16; ++l) c[l] = (pk[l] >> (8 * u)) & 0xffu;
-      const int neg = crt_value(c, Q, Mm, invMf, mag);
-      big_to_dir(mag, neg, Ei + Fj - 2 * w, lo, up);
-      const double t1 = scale_pow2(bj, Ei - w - 1, true);
-      const double t2 = scale_pow2(rw.sA[u], Ei + Fj - 2 * w - 1, true);
-      tr = __dadd_ru(t1, t2);
-    }
-    const double Tu = rad_T(W1[u], W2[u], rw.Ep[u], rw.Er[u], Fj, Frj, rc,
-                            __fmul_ru(rw.qp[u], qb1), __fmul_ru(rw.qr[u], qb2));
-    const double err = __dadd_ru(tr, Tu);
-    double clo = __dsub_rd(lo, err), cup = __dadd_ru(up, err);
-    if (nonfinite) clo = cup = __longlong_as_double(0x7ff8000000000000LL);
-    double* cp = C + 2 * ((size_t)i + (size_t)j * ldc);  // C may be only 8-byte aligned
-    cp[0] = clo;
-    cp[1] = cup;
-  }
-}
-
-// Thread = 4 consecutive rows of about 8 columns; blockIdx.y strides over the
-// columns (no 64-bit index division).  At most 80 registers: three blocks per
-// SM (measured at n = 8192: 1.88 ms; 2.10 ms at the unbounded 94 registers).
-__global__ void __launch_bounds__(256, 3)
-oz_crt_assemble_kernel(int M, int N, int Mp, int L, int w, const uint8_t* __restrict__ res,
-                       size_t plane, const int* __restrict__ E3, const int* __restrict__ F2,
-                       const unsigned long long* __restrict__ asum,
-                       const unsigned long long* __restrict__ bsum,
-                       const double* __restrict__ beta, const int32_t* __restrict__ P,
-                       double* __restrict__ C, long ldc, const int* __restrict__ flag,
-                       const __grid_constant__ CrtConst cc, const __grid_constant__ OzRadConst rc) {
-  const bool nonfinite = flag[0] != 0 || flag[1] != 0;
-  const int Mq = (M + 3) >> 2;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= Mq) return;
-  QuadRows rw;
-  quad_rows(4 * q, M, E3, asum, rw);
-  for (int j = blockIdx.y; j < N; j += gridDim.y)
-    assemble_quad_col(rw, 4 * q, j, M, Mp, L, w, res, plane, F2[2 * j], F2[2 * j + 1], beta[j],
-                      bsum + 4 * (size_t)j + 2, P, C, ldc, nonfinite, cc.Q, cc.M, cc.invMf, rc);
+// One product: blockIdx.x over the column ranges of CB columns, blockIdx.y
+// over the 128-row tiles.  Block (0, 0) merges the status words.
+template <bool LOWB>
+__global__ void __launch_bounds__(ASM_NT, 3)
+oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
+                       const uint8_t* __restrict__ res, size_t plane, const int* __restrict__ E3,
+                       const int* __restrict__ F2, const unsigned long long* __restrict__ asum,
+                       const unsigned long long* __restrict__ bsum, const int32_t* __restrict__ P,
+                       double* __restrict__ C, long ldc, const int* __restrict__ flag, int merge,
+                       const __grid_constant__ CrtBasis cc, const __grid_constant__ OzRadConst rc) {
+  __shared__ AsmTile t;
+  const int f0 = flag[0], f1 = flag[1];
+  if (merge && (f0 | f1) && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+    atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
+  const int i0 = blockIdx.y * ASM_ROWS, nr = min(ASM_ROWS, M - i0);
+  const int j0 = blockIdx.x * CB, nc = min(CB, N - j0);
+  asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, E3, asum, F2, bsum);
+  const AsmArgs a{M, Mp, L, w, res, plane, P, C, ldc, f0 != 0 || f1 != 0,
+                  (((uintptr_t)C) & 15) == 0};
+  asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
 }
 
 // Grouped reassembly.  The problems of a bucket share one CRT plan (the
 // bucket is keyed by padded K, modulus count and operand width), so the
-// basis comes in the launch parameters as for one product.  A thread takes 4
-// consecutive rows of one problem and the columns cg, cg + NG, cg + 2 NG, ...
-// (NG = ceil(n / 8) column groups): its rows' exponents and sums are set up
-// once for about 8 columns, and consecutive threads take consecutive row
-// quads (coalesced residue and fold reads).  A block finds its problem with
-// one load (prob_asm), stamps the problem's end and merges its status words
-// into the sticky status.  A device-wait timeout of the slice
-// GEMM (flag[1] of problem 0) poisons every output of the bucket.  117
-// registers: two blocks per SM (the problem's pointers and sizes stay in
-// registers where one product has them in the launch parameters; at 80
-// registers they spill).
-__global__ void __launch_bounds__(256, 2)
-oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ CrtConst cc,
-                  const __grid_constant__ OzRadConst rc, int* __restrict__ status) {
+// basis comes in the launch parameters as for one product.  A block takes a
+// tile of up to 128 rows and OZ_GASM_COLS columns of one problem, found with
+// one load (prob_asm); it stamps the problem's end and merges its status
+// words into the sticky status.  A device-wait timeout of the slice
+// GEMM (flag[1] of problem 0) poisons every output of the bucket.
+template <bool LOWB>
+__global__ void __launch_bounds__(ASM_NT, 3)
+oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ CrtBasis cc,
+                  const __grid_constant__ OzRadConst rc) {
+  __shared__ AsmTile t;
   const int p = b.prob_asm[blockIdx.x];
   const OzGProb& q = b.probs[p];
   const int m = q.m, n = q.n;
-  const int Mq = (m + 3) >> 2;
-  const int NG = (n + 7) >> 3;
-  const long u = (long)(blockIdx.x - b.blk_asm[p]) * blockDim.x + threadIdx.x;
+  const int tm = (m + ASM_ROWS - 1) / ASM_ROWS, local = blockIdx.x - b.blk_asm[p];
+  const int i0 = (local % tm) * ASM_ROWS, nr = min(ASM_ROWS, m - i0);
+  const int j0 = (local / tm) * OZ_GASM_COLS, nc = min(OZ_GASM_COLS, n - j0);
   const int f0 = b.flag[4 * p], f1 = b.flag[4 * p + 1];
-  if (u < (long)Mq * NG) {
-    const bool nonfinite = f0 != 0 || b.flag[1] != 0;
-    const int qd = (int)(u % Mq), cg = (int)(u / Mq);
-    const int* E3 = b.E3 + 3 * (size_t)q.rowoff;
-    const unsigned long long* asum = b.asum + 4 * (size_t)q.rowoff;
-    const unsigned long long* bsum = b.bsum + 4 * (size_t)q.coloff;
-    const int* F2 = b.F2 + 2 * (size_t)q.coloff;
-    const double* beta = b.beta + q.coloff;
-    const uint8_t* res = b.res + q.res_off;
-    const int32_t* P = b.P + q.P_off;
-    const size_t plane = (size_t)q.Np * q.Mp;
-    QuadRows rw;
-    quad_rows(4 * qd, m, E3, asum, rw);
-    for (int j = cg; j < n; j += NG)
-      assemble_quad_col(rw, 4 * qd, j, m, q.Mp, q.L, q.w, res, plane, F2[2 * j], F2[2 * j + 1],
-                        beta[j], bsum + 4 * (size_t)j + 2, P, q.C, q.ldc, nonfinite, cc.Q, cc.M,
-                        cc.invMf, rc);
-  }
-  if (threadIdx.x == 0 && (f0 | f1)) atomicOr(status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
+  asm_tile_setup(t, i0, nr, j0, nc, q.k, q.w, LOWB, b.E3 + 3 * (size_t)q.rowoff,
+                 b.asum + 4 * (size_t)q.rowoff, b.F2 + 2 * (size_t)q.coloff,
+                 b.bsum + 4 * (size_t)q.coloff);
+  const AsmArgs a{m, q.Mp, q.L, q.w, b.res + q.res_off, (size_t)q.Np * q.Mp, b.P + q.P_off, q.C,
+                  q.ldc, f0 != 0 || b.flag[1] != 0, (((uintptr_t)q.C) & 15) == 0};
+  asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
+  if (threadIdx.x == 0 && (f0 | f1)) atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
   if (b.t_last) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      atomicMax(&b.t_last[q.orig], t);
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      atomicMax(&b.t_last[q.orig], now);
     }
   }
 }
 
+static_assert(OZ_GASM_COLS <= ASM_COLS, "column data of a grouped tile");
+
 }  // namespace
 
-namespace {
-// The CRT basis of a plan's L moduli (Q_l = 0 past L), M and 2^64 / M.
-CrtConst crt_const(const OzPlan& plan) {
-  CrtConst cc;
-  memset(&cc, 0, sizeof(cc));
-  for (int l = 0; l < plan.pb.L; ++l)
-    for (int t = 0; t < 4; ++t) cc.Q[l][t] = plan.Q[l][t];
-  for (int t = 0; t < 4; ++t) cc.M[t] = plan.Mlimb[t];
-  const double Md = (double)cc.M[3] * 0x1p96 + (double)cc.M[2] * 0x1p64 +
-                    (double)cc.M[1] * 0x1p32 + (double)cc.M[0];
-  cc.invMf = (float)(0x1p64 / Md);
-  return cc;
+void oz_merge_status(const int* flag, cudaStream_t s) {
+  oz_status_merge<<<1, 1, 0, s>>>(flag);
+  count_launch();
 }
-}  // namespace
+
+int oz_take_status(cudaStream_t s, int* status) {
+  int zero = 0;
+  VCPCU_CUDA_TRY(cudaMemcpyFromSymbolAsync(status, g_oz_status, sizeof(int), 0,
+                                           cudaMemcpyDeviceToHost, s));
+  VCPCU_CUDA_TRY(cudaStreamSynchronize(s));
+  VCPCU_CUDA_TRY(cudaMemcpyToSymbolAsync(g_oz_status, &zero, sizeof(int), 0,
+                                         cudaMemcpyHostToDevice, s));
+  VCPCU_CUDA_TRY(cudaStreamSynchronize(s));
+  return VCPCU_OK;
+}
 
 int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long ldc,
-                    cudaStream_t st) {
+                    cudaStream_t st, bool merge_status) {
   const OzProblem& pb = plan.pb;
-  const CrtConst cc = crt_const(plan);
   if (pb.M <= 0 || pb.N <= 0) return VCPCU_OK;
-  const int Mq = (pb.M + 3) / 4;
-  // about 8 columns per thread: its rows' exponents and sums are set up once
-  const int gy = (pb.N + 7) / 8;
-  // 128-thread blocks: a row count that is not a multiple of 1024 leaves at
-  // most 127 idle threads per column group (the blocks of a host-pointer
-  // product have 768 - 1536 rows)
-  dim3 grid((Mq + 127) / 128, gy < 65535 ? gy : 65535);
-  oz_crt_assemble_kernel<<<grid, 128, 0, st>>>(
-      pb.M, pb.N, pb.Mp, pb.L, pb.w, ws.res, (size_t)pb.Np * pb.Mp, ws.E3, ws.F2, ws.asum,
-      ws.bsum, ws.beta, ws.P, C, ldc, ws.flag, cc, oz_rad_const(plan));
+  const int tm = (pb.M + ASM_ROWS - 1) / ASM_ROWS;
+  // columns per block: as many as leave four blocks for each of the 152 SMs
+  // (a block's row and column data are formed once), 64 at most
+  int CB = ASM_COLS;
+  while (CB > 8 && (long)tm * ((pb.N + CB - 1) / CB) < 608) CB >>= 1;
+  // (row tiles past the 65535 of grid.y: more than 8 million rows)
+  if (tm > 65535) {
+    set_error("reassembly: %d rows are more than it takes", pb.M);
+    return VCPCU_ERR_UNSUPPORTED;
+  }
+  const dim3 grid((pb.N + CB - 1) / CB, tm);
+  const OzRadConst rc = oz_rad_const(plan);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, ASM_NT, 0, st>>>(pb.M, pb.N, pb.K, pb.Mp, pb.L, pb.w, CB, ws.res,
+                                    (size_t)pb.Np * pb.Mp, ws.E3, ws.F2, ws.asum, ws.bsum, ws.P,
+                                    C, ldc, ws.flag, merge_status ? 1 : 0, plan.basis, rc);
+  };
+  if (rc.lowb)
+    launch(oz_crt_assemble_kernel<true>);
+  else
+    launch(oz_crt_assemble_kernel<false>);
   VCPCU_LAUNCH_CHECK("oz_crt_assemble_kernel");
   return VCPCU_OK;
 }
@@ -460,12 +580,10 @@ int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long l
 int oz_gassemble(const OzGBucket& b, const OzPlan& shape, const OzRadConst& rc, int nblk,
                  cudaStream_t st) {
   if (nblk <= 0) return VCPCU_OK;
-  int* status = oz_status_ptr();
-  if (!status) {
-    set_error("igemm_batched: no device address of the status word");
-    return VCPCU_ERR_CUDA;
-  }
-  oz_crt_assemble_g<<<nblk, 256, 0, st>>>(b, crt_const(shape), rc, status);
+  if (rc.lowb)
+    oz_crt_assemble_g<true><<<nblk, ASM_NT, 0, st>>>(b, shape.basis, rc);
+  else
+    oz_crt_assemble_g<false><<<nblk, ASM_NT, 0, st>>>(b, shape.basis, rc);
   VCPCU_LAUNCH_CHECK("oz_crt_assemble_g");
   return VCPCU_OK;
 }

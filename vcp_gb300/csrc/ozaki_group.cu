@@ -43,7 +43,7 @@ struct BucketHost {
   int wmax = 0;  // largest operand width w of the bucket's problems
   // workspace layout (byte offsets; the first zero_bytes are cleared per run)
   size_t offRowmax = 0, offAsum = 0, offFlag = 0, zero_bytes = 0;
-  size_t offE3 = 0, offF2 = 0, offBeta = 0, offA = 0, offB = 0, offRes = 0, offP = 0;
+  size_t offE3 = 0, offF2 = 0, offA = 0, offB = 0, offRes = 0, offP = 0;
   size_t offMidB = 0, offRadB = 0, offBsum = 0, offMidA = 0, offRadA = 0;
   size_t ws_bytes = 0;
 };
@@ -192,12 +192,6 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       gp.res_off = res;
       gp.P_off = P;
       gp.orig = id;
-      for (int l = 0; l < 16; ++l)
-        for (int c = 0; c < 4; ++c) gp.Q[l][c] = l < pl.pb.L ? pl.Q[l][c] : 0u;
-      for (int c = 0; c < 4; ++c) gp.Mlimb[c] = pl.Mlimb[c];
-      const double Md = (double)pl.Mlimb[3] * 0x1p96 + (double)pl.Mlimb[2] * 0x1p64 +
-                        (double)pl.Mlimb[1] * 0x1p32 + (double)pl.Mlimb[0];
-      gp.invMf = (float)(0x1p64 / Md);
       memcpy(host.data() + o.probs + sizeof(OzGProb) * t, &gp, sizeof(gp));
       int* v;
       v = (int*)(host.data() + o.brow); v[t] = (int)brow;
@@ -212,7 +206,7 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       bspl += (long long)(Kp / 64) * (gp.Mp / 32);
       irad += b.shape.rad.ngroups * tiles;
       icrt += gp.L * tiles;
-      basm += (((long long)(q.m + 3) / 4) * ((q.n + 7) / 8) + 255) / 256;
+      basm += (long long)((q.m + 127) / 128) * ((q.n + OZ_GASM_COLS - 1) / OZ_GASM_COLS);
       res += (long long)gp.L * gp.Np * gp.Mp;
       P += 2LL * b.shape.rad_slots * gp.Np * gp.Mp;
       rowoff += gp.Mp;
@@ -268,7 +262,6 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     b.zero_bytes = w;
     b.offE3 = take(sizeof(int) * 3 * Mtot);
     b.offF2 = take(sizeof(int) * 2 * Ntot);
-    b.offBeta = take(sizeof(double) * Ntot);
     b.offMidB = take(sizeof(double) * (size_t)Ntot * Kp);
     b.offRadB = take(sizeof(double) * (size_t)Ntot * Kp);
     b.offBsum = take(sizeof(unsigned long long) * 4 * Ntot);
@@ -337,7 +330,6 @@ int record_chunk(const BucketHost& b, uint8_t* ws, unsigned long long* t_first,
   d.flag = (int*)(ws + b.offFlag);
   d.E3 = (int*)(ws + b.offE3);
   d.F2 = (int*)(ws + b.offF2);
-  d.beta = (double*)(ws + b.offBeta);
   d.midB = (double*)(ws + b.offMidB);
   d.radB = (double*)(ws + b.offRadB);
   d.bsum = (unsigned long long*)(ws + b.offBsum);

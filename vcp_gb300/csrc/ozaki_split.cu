@@ -419,20 +419,6 @@ __device__ __forceinline__ uint32_t res_pair(const float (&h0)[NL], const float 
   return __byte_perm((uint32_t)r, (uint32_t)(r >> 32), 0x7632);
 }
 
-// x * 2^e rounded up (up) or down, in steps that stay in the double range.
-__device__ __forceinline__ double dev_scale_dir(double x, int e, bool up) {
-  while (e > 1023) {
-    x = up ? __dmul_ru(x, 0x1p1023) : __dmul_rd(x, 0x1p1023);
-    e -= 1023;
-  }
-  while (e < -1022) {
-    x = up ? __dmul_ru(x, 0x1p-1022) : __dmul_rd(x, 0x1p-1022);
-    e += 1022;
-  }
-  const double p = __longlong_as_double((long long)(e + 1023) << 52);
-  return up ? __dmul_ru(x, p) : __dmul_rd(x, p);
-}
-
 // w-bit integer of x (|x| <= 2^(E-1)): round to nearest even, |result| <= 2^(w-1).
 // x 2^(w-E) is formed exactly by power-of-two multiplications (no overflow:
 // it stays below 2^(w-1); a subnormal intermediate is below 2^-1022 and
@@ -869,21 +855,6 @@ __global__ void __launch_bounds__(256) oz_split_right2_g(const __grid_constant__
   }
 }
 
-// Pass 3: beta_j = RU((sum_k |B'| + ceil(K/2)) 2^(Fm - w)) per stacked column.
-__global__ void oz_beta_right_g(const __grid_constant__ OzGBucket b) {
-  const int jst = blockIdx.x * blockDim.x + threadIdx.x;
-  if (jst >= b.Ntot) return;
-  const OzGProb& q = b.probs[b.col_prob[jst]];
-  const int j = jst - q.coloff, Fm = b.F2[2 * jst];
-  double bj = 0.0;
-  if (j < q.n && Fm != OZ_ZERO_EXP) {
-    const double v = __fma_ru((double)b.bsum[4 * jst], 0x1p32,
-                              (double)(b.bsum[4 * jst + 1] + (unsigned long long)(q.k + 1) / 2));
-    bj = dev_scale_dir(v, Fm - q.w, true);
-  }
-  b.beta[jst] = bj;
-}
-
 int oz_gprep(const OzGBucket& b, int nblk_rowmax, int nblk_split, int wmax, cudaStream_t st) {
   if (nblk_rowmax > 0) {
     oz_rowmax_left_g<<<nblk_rowmax, 256, 0, st>>>(b);
@@ -916,9 +887,8 @@ int oz_gprep(const OzGBucket& b, int nblk_rowmax, int nblk_split, int wmax, cuda
   }
 #undef OZ_GRIGHT
   VCPCU_LAUNCH_CHECK("oz_split_right2_g");
-  // (the exponents of the left factor come from its split)
-  oz_beta_right_g<<<(b.Ntot + 255) / 256, 256, 0, st>>>(b);
-  VCPCU_LAUNCH_CHECK("oz_beta_right_g");
+  // (the exponents of the left factor come from its split, the columns'
+  // beta from the reassembly)
   return VCPCU_OK;
 }
 
@@ -1089,23 +1059,6 @@ oz_split_right_crt2(int K, int N, int Kp, int cols, int colbase, size_t pstride,
   }
 }
 
-// beta_j = RU((sum_k |B'| + ceil(K/2)) 2^(Fm - w)) >= sum_k |mB(k, j)|.
-__global__ void oz_beta_right(int K, int N, int cols, int colbase, int w,
-                              const int* __restrict__ F2,
-                              const unsigned long long* __restrict__ bsum,
-                              double* __restrict__ beta) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= cols) return;
-  const int jst = colbase + j, Fm = F2[2 * jst];
-  double bj = 0.0;
-  if (j < N && Fm != OZ_ZERO_EXP) {
-    const double v = __fma_ru((double)bsum[4 * jst], 0x1p32,
-                              (double)(bsum[4 * jst + 1] + (unsigned long long)(K + 1) / 2));
-    bj = dev_scale_dir(v, Fm - w, true);
-  }
-  beta[jst] = bj;
-}
-
 int oz_prepare_left_begin(const OzProblem& pb, OzWorkspace& ws, cudaStream_t st) {
   VCPCU_CUDA_TRY(cudaMemsetAsync(ws.rowmax, 0, sizeof(unsigned long long) * 3 * (size_t)pb.Mp, st));
   VCPCU_CUDA_TRY(cudaMemsetAsync(ws.delta, 0, sizeof(unsigned long long) * (size_t)pb.Mp, st));
@@ -1213,9 +1166,6 @@ int oz_prepare_right_crt(const OzProblem& pb, const double* B, long ldb, OzWorks
     OZ_RIGHT_CRT(6);
 #undef OZ_RIGHT_CRT
   VCPCU_LAUNCH_CHECK("oz_split_right_crt2");
-  oz_beta_right<<<(cols + 255) / 256, 256, 0, st>>>(pb.K, nv, cols, colbase, pb.w, ws.F2,
-                                                    ws.bsum, ws.beta);
-  VCPCU_LAUNCH_CHECK("oz_beta_right");
   return VCPCU_OK;
 }
 
