@@ -240,7 +240,7 @@ int autotune_pick(int m, int n, int k, const double* A, long lda, const double* 
   // probe: the plain form and every candidate on the sampled block
   if ((st = igemm_any(Sr, Sc, k, As, Sr, Bs, k, Cs, Sr, VCPCU_FORM_PLAIN, 0, s))) return st;
   for (int c = 0; c < NCAND; ++c)
-    if ((st = ozaki_igemm(Sr, Sc, k, As, Sr, Bs, k, Cs + (c + 1) * nc, Sr, VCPCU_FORM_OZAKI,
+    if ((st = ozaki_igemm(Sr, Sc, k, OzOperand{As, Sr}, OzOperand{Bs, k}, Cs + (c + 1) * nc, Sr, VCPCU_FORM_OZAKI,
                           cand[c], s)))
       return st;
   std::vector<double> hc((NCAND + 1) * nc);

@@ -172,7 +172,8 @@ int vcpcu::igemm_any(int m, int n, int k, const double* A, long lda, const doubl
     if (st) return st;
     return launch_interval_gemm_plain(m, n, k, A, lda, B, ldb, C, ldc, (double*)ws.ptr, s);
   }
-  return ozaki_igemm(m, n, k, A, lda, B, ldb, C, ldc, form, slices, s, point_mask);
+  return ozaki_igemm(m, n, k, OzOperand{A, lda}, OzOperand{B, ldb}, C, ldc, form, slices, s,
+                     point_mask);
 }
 
 namespace {

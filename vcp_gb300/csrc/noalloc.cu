@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "ozaki.cuh"
 
+#include <algorithm>
 #include <mutex>
 
 namespace vcpcu {
@@ -58,6 +59,18 @@ int scratch_for_current_device(void** out) {
   return VCPCU_OK;
 }
 
+// The scratch by which the entry point has always measured a problem: what the
+// kernels take now plus room for midpoint and radius planes of both factors,
+// so that the same problems are accepted.
+size_t noalloc_bytes(const OzProblem& pb) {
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t np = (size_t)(pb.mplanes + 2 * pb.sr), Mp = pb.Mp, Np = pb.Np, Kp = pb.Kp;
+  return al(np * Mp * Kp * 2) + al(np * Np * Kp * 2) + al(24 * Mp) + al(12 * Mp) + al(8 * Mp) +
+         2 * al(8 * Np) + al(8 * Mp * Np) + al(16) +
+         2 * al(8 * (size_t)pb.M * (pb.K > 0 ? pb.K : 1)) + 2 * al(8 * Np * Kp) + al(32 * Np) +
+         al(32 * Mp) + al((size_t)pb.L * Np * Mp);
+}
+
 }  // namespace
 
 }  // namespace vcpcu
@@ -91,7 +104,7 @@ extern "C" int vcpcu_igemm_noalloc_dev(int m, int n, int k, const double* A, int
   }
   OzPlan plan;
   oz_make_plan(m, n, k, slices, 2, &plan, /*crt=*/1);
-  const size_t need = oz_workspace_bytes(plan.pb);
+  const size_t need = std::max(noalloc_bytes(plan.pb), oz_workspace_bytes(plan.pb));
   if (need > (size_t)VCPCU_NOALLOC_SCRATCH_BYTES) {
     set_error("igemm_noalloc: %d x %d x %d with %d slices needs %zu bytes of scratch, more than "
               "the %u-byte static scratch; use vcpcu_igemm_dev",
@@ -105,7 +118,7 @@ extern "C" int vcpcu_igemm_noalloc_dev(int m, int n, int k, const double* A, int
   cudaStream_t s = (cudaStream_t)stream;
   OzWorkspace ws;
   oz_carve_workspace(plan.pb, base, &ws);
-  if ((st = oz_run_product(plan, ws, A, lda, B, ldb, C, ldc, s))) return st;
+  if ((st = oz_run_product(plan, ws, OzOperand{A, lda}, OzOperand{B, ldb}, C, ldc, s))) return st;
   // The reassembly writes NaN everywhere after a non-finite input or a
   // timed-out wait and merges the status words into the per-device status
   // that vcpcu_status reports, as for vcpcu_igemm_dev.

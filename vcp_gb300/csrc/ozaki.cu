@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -250,92 +251,76 @@ namespace {
 int rad_slot_count(const OzProblem&) { return 1; }
 }  // namespace
 
-size_t oz_workspace_bytes(const OzProblem& pb) {
+namespace {
+// The parts of a workspace, in order: with a base, each pointer; the size
+// either way.
+size_t workspace_layout(const OzProblem& pb, uint8_t* base, OzWorkspace* ws) {
+  size_t off = 0;
+  auto take = [&](auto** ptr, size_t bytes) {
+    if (ws) *ptr = reinterpret_cast<std::remove_pointer_t<decltype(ptr)>>(base + off);
+    off += al256(bytes);
+  };
+  OzWorkspace none;
+  OzWorkspace& w = ws ? *ws : none;
+  const size_t mk = (size_t)pb.Mp * pb.Kp, nk = (size_t)pb.Np * pb.Kp,
+               mn = (size_t)pb.Mp * pb.Np;
   const size_t np = (size_t)(pb.mplanes + 2 * pb.sr);
-  size_t b = 0;
-  b += al256(np * pb.Mp * pb.Kp * 2);
-  b += al256(np * pb.Np * pb.Kp * 2);
-  b += al256(sizeof(unsigned long long) * 3 * pb.Mp);
-  b += al256(sizeof(int) * 3 * pb.Mp);
-  b += al256(sizeof(unsigned long long) * pb.Mp);
-  b += al256(sizeof(int) * 2 * pb.Np);
-  b += al256(sizeof(double) * pb.Np);
-  if (!pb.crt) {  // T and the midpoint fold buffer: slice form only
-    b += al256(sizeof(double) * (size_t)pb.Mp * pb.Np);
-    b += al256(sizeof(long long) * (size_t)pb.Mp * pb.Np);
+  take(&w.a_mid, np * mk * 2);
+  take(&w.b_mid, np * nk * 2);
+  if (ws) {
+    w.a_p = w.a_mid + pb.mplanes * mk;
+    w.a_r = w.a_p + pb.sr * mk;
+    w.b_r = w.b_mid + pb.mplanes * nk;
+    w.b_s = w.b_r + pb.sr * nk;
   }
-  b += al256(sizeof(int32_t) * 2 * (size_t)rad_slot_count(pb) * pb.Mp * pb.Np);
-  b += al256(sizeof(int) * 4);
-  b += 2 * al256(sizeof(double) * (size_t)pb.M * (pb.K > 0 ? pb.K : 1));
-  b += 2 * al256(sizeof(double) * (size_t)pb.Np * pb.Kp);
-  if (pb.crt) b += al256(sizeof(unsigned long long) * 4 * pb.Np);
-  b += al256(sizeof(unsigned long long) * 4 * pb.Mp);
-  if (pb.crt) b += al256((size_t)pb.L * pb.Np * pb.Mp);
-  return b;
+  take(&w.P, sizeof(int32_t) * 2 * (size_t)rad_slot_count(pb) * mn);
+  if (pb.crt) {
+    const size_t z0 = off;
+    take(&w.eA, sizeof(uint32_t) * 3 * pb.Mp);
+    take(&w.eB, sizeof(uint32_t) * 2 * pb.Np);
+    take(&w.asum, sizeof(unsigned long long) * 4 * pb.Mp);
+    take(&w.bsum, sizeof(unsigned long long) * 4 * pb.Np);
+    take(&w.flag, sizeof(int) * 4);
+    if (ws) {
+      w.zero = base + z0;
+      w.zero_bytes = off - z0;
+    }
+    take(&w.res, (size_t)pb.L * mn);
+  } else {
+    const size_t mk1 = (size_t)pb.M * (pb.K > 0 ? pb.K : 1);
+    take(&w.flag, sizeof(int) * 4);
+    take(&w.rowmax, sizeof(unsigned long long) * 3 * pb.Mp);
+    take(&w.E3, sizeof(int) * 3 * pb.Mp);
+    take(&w.delta, sizeof(unsigned long long) * pb.Mp);
+    take(&w.F2, sizeof(int) * 2 * pb.Np);
+    take(&w.beta, sizeof(double) * pb.Np);
+    take(&w.T, sizeof(double) * mn);
+    take(&w.W, sizeof(long long) * mn);
+    take(&w.midA, sizeof(double) * mk1);
+    take(&w.radA, sizeof(double) * mk1);
+    take(&w.midB, sizeof(double) * nk);
+    take(&w.radB, sizeof(double) * nk);
+  }
+  return off;
 }
+}  // namespace
+
+size_t oz_workspace_bytes(const OzProblem& pb) { return workspace_layout(pb, nullptr, nullptr); }
 
 int oz_carve_workspace(const OzProblem& pb, void* base, OzWorkspace* ws) {
-  uint8_t* p = (uint8_t*)base;
-  const size_t mk = (size_t)pb.Mp * pb.Kp, nk = (size_t)pb.Np * pb.Kp;
-  const size_t np = (size_t)(pb.mplanes + 2 * pb.sr);
-  uint16_t* a = (uint16_t*)p;
-  ws->a_mid = a;
-  ws->a_p = a + pb.mplanes * mk;
-  ws->a_r = ws->a_p + pb.sr * mk;
-  p += al256(np * mk * 2);
-  uint16_t* b = (uint16_t*)p;
-  ws->b_mid = b;
-  ws->b_r = b + pb.mplanes * nk;
-  ws->b_s = ws->b_r + pb.sr * nk;
-  p += al256(np * nk * 2);
-  ws->rowmax = (unsigned long long*)p;
-  p += al256(sizeof(unsigned long long) * 3 * pb.Mp);
-  ws->E3 = (int*)p;
-  p += al256(sizeof(int) * 3 * pb.Mp);
-  ws->delta = (unsigned long long*)p;
-  p += al256(sizeof(unsigned long long) * pb.Mp);
-  ws->F2 = (int*)p;
-  p += al256(sizeof(int) * 2 * pb.Np);
-  ws->beta = (double*)p;
-  p += al256(sizeof(double) * pb.Np);
-  ws->T = nullptr;
-  ws->W = nullptr;
-  if (!pb.crt) {
-    ws->T = (double*)p;
-    p += al256(sizeof(double) * (size_t)pb.Mp * pb.Np);
-    ws->W = (long long*)p;
-    p += al256(sizeof(long long) * (size_t)pb.Mp * pb.Np);
-  }
-  ws->P = (int32_t*)p;
-  p += al256(sizeof(int32_t) * 2 * (size_t)rad_slot_count(pb) * pb.Mp * pb.Np);
-  ws->flag = (int*)p;
-  p += al256(sizeof(int) * 4);
-  const size_t mk1 = sizeof(double) * (size_t)pb.M * (pb.K > 0 ? pb.K : 1);
-  ws->midA = (double*)p;
-  p += al256(mk1);
-  ws->radA = (double*)p;
-  p += al256(mk1);
-  ws->midB = (double*)p;
-  p += al256(sizeof(double) * (size_t)pb.Np * pb.Kp);
-  ws->radB = (double*)p;
-  p += al256(sizeof(double) * (size_t)pb.Np * pb.Kp);
-  ws->bsum = nullptr;
-  if (pb.crt) {
-    ws->bsum = (unsigned long long*)p;
-    p += al256(sizeof(unsigned long long) * 4 * pb.Np);
-  }
-  ws->asum = (unsigned long long*)p;
-  p += al256(sizeof(unsigned long long) * 4 * pb.Mp);
-  ws->res = pb.crt ? (uint8_t*)p : nullptr;
+  *ws = OzWorkspace();
+  workspace_layout(pb, (uint8_t*)base, ws);
   return VCPCU_OK;
 }
 
-int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const double* A, long lda,
-                   const double* B, long ldb, double* C, long ldc, cudaStream_t s) {
+int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, const OzOperand& B,
+                   double* C, long ldc, cudaStream_t s, double* Cup) {
   int st;
   {
     PhaseTimer t(0, s);
-    if ((st = oz_prepare(plan.pb, A, lda, B, ldb, ws, s))) return st;
+    st = plan.pb.crt ? oz_prepare(plan.pb, plan.point_mask, A, B, ws, s)
+                     : oz_prepare_slices(plan.pb, A.x, A.ld, B.x, B.ld, ws, s);
+    if (st) return st;
   }
   // T = (|mA| + rA) * rB + rA * |mB|: each product leaves its folds in its
   // half of ws.P.  A product with a zero factor would give exactly 0 (its
@@ -361,7 +346,7 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const double* A, long ld
   }
   if (plan.pb.crt) {
     PhaseTimer t(4, s);
-    if ((st = oz_crt_assemble(plan, ws, C, ldc, s, true))) return st;
+    if ((st = oz_crt_assemble(plan, ws, C, ldc, s, true, Cup))) return st;
   } else {
     oz_merge_status(ws.flag, s);
     VCPCU_LAUNCH_CHECK("oz_status_merge");
@@ -495,7 +480,8 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
   if ((st = pipe_event(g, s, up)) || (st = pipe_event(g, s, down)) ||
       (st = pipe_event(g, s, c0)) || (st = pipe_event(g, s, c1)))
     return st;
-  if ((st = oz_prepare_left_begin(pb, ws, s))) return st;
+  if ((st = oz_prepare_begin(ws, s))) return st;
+  const OzOperand opA{dA, m}, opB{dB, k > 0 ? k : 1};
 
   // uploads, interleaved: A's row block t, then B's column block t
   const size_t rowb = 2 * sizeof(double);  // bytes of one interval
@@ -542,11 +528,9 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
     v.b_r = ws.b_r + (size_t)j0 * Kp;
     v.b_s = ws.b_s + (size_t)j0 * Kp;
     v.b_pstride = (size_t)pb.Np * Kp;
-    v.rowmax = ws.rowmax + 3 * (size_t)i0;
-    v.E3 = ws.E3 + 3 * (size_t)i0;
-    v.delta = ws.delta + i0;
+    v.eA = ws.eA + 3 * (size_t)i0;
     v.asum = ws.asum + 4 * (size_t)i0;
-    v.F2 = ws.F2 + 2 * (size_t)j0;
+    v.eB = ws.eB + 2 * (size_t)j0;
     v.bsum = ws.bsum + 4 * (size_t)j0;
     const bool odd = (nblk++ & 1) != 0;
     cudaStream_t c = odd ? c1 : c0;
@@ -575,7 +559,7 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
     if (t < row_panels) {
       const int i0 = rb[t], rows = (t + 1 < row_panels ? rb[t + 1] : pb.Mp) - i0;
       VCPCU_CUDA_TRY(cudaStreamWaitEvent(s, evA[t], 0));
-      if ((st = oz_prepare_left_rows(pb, dA, m, i0, rows, ws, s))) return st;
+      if ((st = oz_prepare_left_rows(pb, opA, i0, rows, ws, s))) return st;
       const int nj = t < panels ? t : panels;
       if (!last_is_b && t == row_panels - 1) {
         for (int J = 0; J < nj; ++J)
@@ -587,9 +571,7 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
     if (t < panels) {
       const int j0 = cb[t], cols = (t + 1 < panels ? cb[t + 1] : pb.Np) - j0;
       VCPCU_CUDA_TRY(cudaStreamWaitEvent(s, evB[t], 0));
-      if ((st = oz_prepare_right_crt(pb, dB, k > 0 ? k : 1, ws, s, j0, cols,
-                                     (size_t)pb.Np * pb.Kp)))
-        return st;
+      if ((st = oz_prepare_right_cols(pb, opB, j0, cols, ws, s))) return st;
       const int ni = t + 1 < row_panels ? t + 1 : row_panels;
       if (last_is_b && t == panels - 1) {
         for (int I = 0; I < ni; ++I)
@@ -617,8 +599,8 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
   return VCPCU_OK;
 }
 
-int ozaki_igemm(int m, int n, int k, const double* A, long lda, const double* B, long ldb,
-                double* C, long ldc, int form, int slices, cudaStream_t s, int point_mask) {
+int ozaki_igemm(int m, int n, int k, const OzOperand& A, const OzOperand& B, double* C, long ldc,
+                int form, int slices, cudaStream_t s, int point_mask, double* Cup) {
   const int nslices = slices > 0 ? slices : 8;
   const int sr = 2;
   if (k > (1 << 20)) {
@@ -633,7 +615,7 @@ int ozaki_igemm(int m, int n, int k, const double* A, long lda, const double* B,
   if (st) return st;
   OzWorkspace ws;
   oz_carve_workspace(plan.pb, buf.ptr, &ws);
-  if ((st = oz_run_product(plan, ws, A, lda, B, ldb, C, ldc, s))) return st;
+  if ((st = oz_run_product(plan, ws, A, B, C, ldc, s, Cup))) return st;
   oz_profile_add_flops(2LL * m * n * (long long)(k > 0 ? k : 0) *
                        ((plan.pb.crt ? plan.pb.L : plan.mid.npairs) +
                         (long long)(!(point_mask & 2) + !(point_mask & 1)) * plan.rad.npairs));

@@ -30,26 +30,41 @@ struct OzProblem {
   int mplanes;     // midpoint planes per operand: s (slice form) or L (CRT form)
 };
 
+// One factor of a product: kv intervals (ld in intervals) or, raw, a point
+// matrix as plain doubles.
+struct OzOperand {
+  const double* x;
+  long ld;
+  int raw = 0;
+};
+
 // Device scratch of one Ozaki-form product (pointers into one allocation).
 struct OzWorkspace {
   uint16_t *a_mid, *a_p, *a_r;        // left digit planes  [s|sr][Mp][Kp] (bf16)
   uint16_t *b_mid, *b_r, *b_s;        // right digit planes [s|sr][Np][Kp] (bf16)
+  int32_t* P;                         // [2 slots][Np][Mp] fp32 folds (bits) of the two radius products
+  int* flag;                          // [0] non-finite input, [1] device wait timeout
+  // CRT form.  zero .. zero_bytes: the words that the preparation
+  // accumulates into (exponents, sums, flag), cleared before it.
+  void* zero;
+  size_t zero_bytes;
+  uint32_t* eA;                       // [Mp][3] encoded exponents Em, Ep, Er (ozaki_prep.cuh)
+  uint32_t* eB;                       // [Np][2] encoded exponents Fm, Fr
+  unsigned long long* asum;           // [Mp][4] sum_k |A'(i,k)| as (bits >= 32, bits < 32);
+                                      // sum_k lo^2 of the low radius digits of P, of rA
+  unsigned long long* bsum;           // [Np][4] sum_k |B'(k,j)| as (bits >= 32, bits < 32);
+                                      // sum_k lo^2 of the low radius digits of rB, of |mB|
+  uint8_t* res;                       // [L][Np][Mp] residues of A'B' mod m_l
+  // slice form
   unsigned long long* rowmax;         // [Mp][3] maxima of |mA|, P, rA (double bits)
   int* E3;                            // [Mp][3] exponents Em, Ep, Er
   unsigned long long* delta;          // [Mp] sum of |midpoint digits| per row
   int* F2;                            // [Np][2] exponents Fm, Fr
-  double* beta;                       // [Np] sum_k |mB(k,j)| rounded up (slice form)
-  unsigned long long* asum;           // [Mp][4] CRT form: sum_k |A'(i,k)| as (bits >= 32, bits < 32);
-                                      // sum_k lo^2 of the low radius digits of P, of rA
-  uint8_t* res;                       // [L][Np][Mp] CRT form: residues of A'B' mod m_l
+  double* beta;                       // [Np] sum_k |mB(k,j)| rounded up
   double *midA, *radA;                // [K][M] midpoints / radii of A (column-major)
   double *midB, *radB;                // [Np][Kp] midpoints / radii of B (k contiguous)
-  unsigned long long* bsum;           // [Np][4] CRT form: sum_k |B'(k,j)| as (bits >= 32, bits < 32);
-                                      // sum_k lo^2 of the low radius digits of rB, of |mB|
-  double* T;                          // [N][Mp] upper bound of the radius product (slice form)
-  long long* W;                       // [Np][Mp] int64 fold buffer (slice form)
-  int32_t* P;                         // [2 slots][Np][Mp] fp32 folds (bits) of the two radius products
-  int* flag;                          // [0] non-finite input, [1] device wait timeout
+  double* T;                          // [N][Mp] upper bound of the radius product
+  long long* W;                       // [Np][Mp] int64 fold buffer
   // Plane strides (elements) of the left / right digit planes when they are
   // a row / column block of larger planes; 0: Mp Kp / Np Kp.
   size_t a_pstride = 0, b_pstride = 0;
@@ -152,27 +167,21 @@ int oz_radius_T(const OzPlan& plan, const OzWorkspace& ws, cudaStream_t st);
 int oz_make_plan(int M, int N, int K, int s, int sr, OzPlan* plan, int crt = 0);
 // merge_status: the kernel also merges ws.flag into the sticky status.
 int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long ldc,
-                    cudaStream_t st, bool merge_status);
-int oz_prepare(const OzProblem& pb, const double* A, long lda, const double* B, long ldb,
+                    cudaStream_t st, bool merge_status, double* Cup = nullptr);
+// Operand planes of the CRT form (ozaki_prep.cu): both factors of a product
+// whose radius products point_mask leaves out (OzPlan::point_mask), or, after
+// oz_prepare_begin, the rows [i0, i0 + rows) of the left one (i0 a multiple of
+// 128) or the columns [j0, j0 + cols) of the right one.
+int oz_prepare(const OzProblem& pb, int point_mask, const OzOperand& A, const OzOperand& B,
                OzWorkspace& ws, cudaStream_t st);
-// oz_prepare in parts: clear the row maxima, sums and status words; midrad
-// and row maxima of the columns [k0, k1) of A (any order of column ranges,
-// the maxima accumulate); row exponents and the left planes; the right
-// planes (CRT form) of B, whose columns may be any column panel of a larger
-// right factor.
-int oz_prepare_left_begin(const OzProblem& pb, OzWorkspace& ws, cudaStream_t st);
-int oz_prepare_left_rowmax(const OzProblem& pb, const double* A, long lda, int k0, int k1,
-                           OzWorkspace& ws, cudaStream_t st);
-int oz_prepare_left_finish(const OzProblem& pb, OzWorkspace& ws, cudaStream_t st);
-int oz_prepare_right_crt(const OzProblem& pb, const double* B, long ldb, OzWorkspace& ws,
-                         cudaStream_t st, int colbase = 0, int cols = -1, size_t pstride = 0);
-// Left planes of the row block [i0, i0 + rows) (i0 and rows multiples of
-// 128, padding rows included) from the rows of A alone: midrad, row maxima,
-// exponents and planes (CRT form), after oz_prepare_left_begin.  B's column
-// blocks: oz_prepare_right_crt with colbase = j0 and cols its padded width
-// (B points at column 0; planes, F2 and beta of the whole right factor).
-int oz_prepare_left_rows(const OzProblem& pb, const double* A, long lda, int i0, int rows,
+int oz_prepare_begin(OzWorkspace& ws, cudaStream_t st);
+int oz_prepare_left_rows(const OzProblem& pb, const OzOperand& A, int i0, int rows,
                          OzWorkspace& ws, cudaStream_t st);
+int oz_prepare_right_cols(const OzProblem& pb, const OzOperand& B, int j0, int cols,
+                          OzWorkspace& ws, cudaStream_t st);
+// Operand planes of the slice form (ozaki_split.cu).
+int oz_prepare_slices(const OzProblem& pb, const double* A, long lda, const double* B, long ldb,
+                      OzWorkspace& ws, cudaStream_t st);
 // t_set < 0: the radius product of OZ_RAD_SET writes T, that of OZ_RAD_ADD
 // adds to it; 0 / 1 force add / write.
 int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, long ldc,
@@ -212,8 +221,9 @@ void oz_profile_add_flops(long long f);
 
 // Operand preparation, the three slice-GEMM phases and the reassembly of
 // one planned product (shared by every entry point of the Ozaki form).
-int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const double* A, long lda,
-                   const double* B, long ldb, double* C, long ldc, cudaStream_t s);
+// (raw operands: CRT form only)
+int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, const OzOperand& B,
+                   double* C, long ldc, cudaStream_t s, double* Cup = nullptr);
 
 // ---------------------------------------------------------------------------
 // Grouped CRT-form products (a batch of uneven interval products in a few
@@ -224,8 +234,7 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const double* A, long ld
 // coloff + Np) of the B planes ([plane][Ntot][Kp]); its residue bytes and
 // radius folds live at res_off / P_off of the bucket's arrays, laid out as
 // in a single product.  Every kernel of the CRT form has a grouped twin
-// that finds its problem by a binary search over a prefix array of blocks,
-// or by one load from a block / item -> problem table.
+// that finds its problem by one load from a block / item -> problem table.
 struct OzGProb {
   int m, n, k;
   const double* A;
@@ -239,30 +248,30 @@ struct OzGProb {
   int tiles_m, tiles_n;
   long long res_off, P_off;    // element offsets into the bucket's res / P
   int orig;                    // index in the caller's problem table
+  int max_left, split_left;    // blocks of the left factor in the two preparation passes
 };
 
-constexpr int OZ_GASM_COLS = 16;  // columns of a reassembly block of a bucket
+constexpr int OZ_GASM_COLS = 16;   // columns of a reassembly block of a bucket
+constexpr int OZ_GMAX_SPAN = 256;  // k range of a block of its maxima pass
 
 // Device view of one bucket (all pointers device memory).
 struct OzGBucket {
   int nprob, Kp, Lmax, Mtot, Ntot;
   const OzGProb* probs;
-  const int* blk_rowmax;   // [nprob + 1] prefix of rowmax blocks
-  const int* blk_split;    // [nprob + 1] prefix of split_left blocks
+  const int* blk_max;      // [nprob + 1] prefix of the blocks of the maxima pass
+  const int* prob_max;     // [blocks] the problem of each
+  const int* blk_split;    // [nprob + 1] prefix of the blocks of the split pass
+  const int* prob_split;   // [blocks] the problem of each
   const int* item_rad;     // [nprob + 1] prefix of radius work items (groups x tiles)
   const int* item_crt;     // [nprob + 1] prefix of residue work items (L x tiles)
   const int* prob_rad;     // [radius items] the problem of each item
   const int* prob_crt;     // [residue items] the problem of each item
   const int* blk_asm;      // [nprob + 1] prefix of reassembly blocks (128 rows x OZ_GASM_COLS)
   const int* prob_asm;     // [reassembly blocks] the problem of each block
-  const int* col_prob;     // [Ntot] problem of each stacked B column
   uint16_t* planesA;       // [Lmax + 4][Mtot][Kp]: residues, |mA|+rA digits, rA digits
   uint16_t* planesB;       // [Lmax + 4][Ntot][Kp]: residues, rB digits, |mB| digits
-  unsigned long long* rowmax;  // [Mtot][3]
-  int* E3;                 // [Mtot][3]
-  int* F2;                 // [Ntot][2]
-  double *midB, *radB;     // [Ntot][Kp] midrad of the stacked B columns
-  double *midA, *radA;     // [Kp][Mtot] midrad of the stacked A rows (column-major)
+  uint32_t* eA;            // [Mtot][3] encoded exponents, as OzWorkspace::eA
+  uint32_t* eB;            // [Ntot][2]
   unsigned long long* bsum;  // [Ntot][4] as OzWorkspace::bsum
   unsigned long long* asum;  // [Mtot][4] as OzWorkspace::asum
   uint8_t* res;
@@ -272,9 +281,11 @@ struct OzGBucket {
   unsigned long long* t_last;
 };
 
-// Kernels of the grouped form (ozaki_split.cu, ozaki_gemm.cu, ozaki_crt.cu).
+// Kernels of the grouped form (ozaki_prep.cu, ozaki_gemm.cu, ozaki_crt.cu).
 // wmax: the largest operand width w of the bucket (selects the limb form)
-int oz_gprep(const OzGBucket& b, int nblk_rowmax, int nblk_split, int wmax, cudaStream_t st);
+int oz_gprep(const OzGBucket& b, int nblk_max, int nblk_split, int wmax, cudaStream_t st);
+// Blocks of one problem in the two passes; sets q's left counts.
+void oz_gprep_blocks(int m, int n, int k, int Kp, OzGProb* q, int* max_blocks, int* split_blocks);
 int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int mode, int nitems,
                  cudaStream_t st);
 // shape: the bucket's plan (every problem of a bucket has the same CRT basis)
@@ -315,7 +326,9 @@ int ozaki_igemm_host_pipelined(int m, int n, int k, const double* A, const doubl
                                cudaStream_t down);
 
 // point_mask as OzPlan::point_mask (the caller guarantees the zero radii).
-int ozaki_igemm(int m, int n, int k, const double* A, long lda, const double* B, long ldb,
-                double* C, long ldc, int form, int slices, cudaStream_t s, int point_mask = 0);
+// Cup (CRT form): the upper ends go there and the lower ones to C, both as
+// plain matrices with leading dimension ldc; null: C takes intervals.
+int ozaki_igemm(int m, int n, int k, const OzOperand& A, const OzOperand& B, double* C, long ldc,
+                int form, int slices, cudaStream_t s, int point_mask = 0, double* Cup = nullptr);
 
 }  // namespace vcpcu

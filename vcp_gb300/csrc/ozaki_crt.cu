@@ -14,6 +14,7 @@
 #include "ozaki.cuh"
 #include "ozaki_common.cuh"
 #include "ozaki_crt.cuh"
+#include "ozaki_prep.cuh"
 #include "swfp.cuh"
 
 namespace vcpcu {
@@ -259,12 +260,12 @@ __device__ __forceinline__ double asum_ru(unsigned long long ah, unsigned long l
   return up;
 }
 
-// The rows [i0, i0 + nr) and columns [j0, j0 + nc) of the tile.  E3, asum, F2
+// The rows [i0, i0 + nr) and columns [j0, j0 + nc) of the tile.  eA, asum, eB
 // and bsum point at row / column 0 of the product.
 __device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j0, int nc, int K,
-                                               int w, int lowb, const int* __restrict__ E3,
+                                               int w, int lowb, const uint32_t* __restrict__ eA,
                                                const unsigned long long* __restrict__ asum,
-                                               const int* __restrict__ F2,
+                                               const uint32_t* __restrict__ eB,
                                                const unsigned long long* __restrict__ bsum) {
   for (int x = threadIdx.x; x < ASM_ROWS + ASM_COLS; x += ASM_NT) {
     if (x < ASM_ROWS) {
@@ -273,9 +274,9 @@ __device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j
       float qp = 0.0f, qr = 0.0f;
       if (x < nr) {
         const int i = i0 + x;
-        E = E3[3 * i];
-        Ep = E3[3 * i + 1];
-        Er = E3[3 * i + 2];
+        E = exp_dec(eA[3 * i]);
+        Ep = exp_dec(eA[3 * i + 1]);
+        Er = exp_dec(eA[3 * i + 2]);
         sA = asum_ru(asum[4 * i], asum[4 * i + 1]);
         if (lowb) {
           qp = lowpair_root(asum[4 * i + 2], 0x1p-8f);
@@ -291,8 +292,8 @@ __device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j
     } else if (x - ASM_ROWS < nc) {
       const int j = j0 + x - ASM_ROWS;
       AsmCol c;
-      c.Fm = F2[2 * j];
-      c.Fr = F2[2 * j + 1];
+      c.Fm = exp_dec(eB[2 * j]);
+      c.Fr = exp_dec(eB[2 * j + 1]);
       c.beta = 0.0;
       if (c.Fm != OZ_ZERO_EXP) {
         const double v =
@@ -316,6 +317,7 @@ struct AsmArgs {
   size_t plane;
   const int32_t* P;
   double* C;
+  double* Cup;  // not null: plain matrices, lower ends to C, upper ends to Cup
   long ldc;
   bool nonfinite, al16;
 };
@@ -455,16 +457,19 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
         if (i + u < a.M)
           r[u] = asm_entry_general(&a, e0 + u, &t.row, q4 + u, &col, &cc, &rc);
     }
-    double* cp = a.C + 2 * ((size_t)i + (size_t)j * a.ldc);
+    const size_t c0 = (size_t)i + (size_t)j * a.ldc;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (a.nonfinite) r[u].x = r[u].y = __longlong_as_double(0x7ff8000000000000LL);
       if (i + u >= a.M) continue;
-      if (a.al16) {
-        *reinterpret_cast<double2*>(cp + 2 * u) = r[u];
+      if (a.Cup) {
+        a.C[c0 + u] = r[u].x;
+        a.Cup[c0 + u] = r[u].y;
+      } else if (a.al16) {
+        reinterpret_cast<double2*>(a.C)[c0 + u] = r[u];
       } else {  // C may be only 8-byte aligned
-        cp[2 * u] = r[u].x;
-        cp[2 * u + 1] = r[u].y;
+        a.C[2 * (c0 + u)] = r[u].x;
+        a.C[2 * (c0 + u) + 1] = r[u].y;
       }
     }
   }
@@ -475,10 +480,12 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
 template <bool LOWB>
 __global__ void __launch_bounds__(ASM_NT, 3)
 oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
-                       const uint8_t* __restrict__ res, size_t plane, const int* __restrict__ E3,
-                       const int* __restrict__ F2, const unsigned long long* __restrict__ asum,
+                       const uint8_t* __restrict__ res, size_t plane,
+                       const uint32_t* __restrict__ eA, const uint32_t* __restrict__ eB,
+                       const unsigned long long* __restrict__ asum,
                        const unsigned long long* __restrict__ bsum, const int32_t* __restrict__ P,
-                       double* __restrict__ C, long ldc, const int* __restrict__ flag, int merge,
+                       double* __restrict__ C, double* __restrict__ Cup, long ldc,
+                       const int* __restrict__ flag, int merge,
                        const __grid_constant__ CrtBasis cc, const __grid_constant__ OzRadConst rc) {
   __shared__ AsmTile t;
   const int f0 = flag[0], f1 = flag[1];
@@ -486,8 +493,8 @@ oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
     atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
   const int i0 = blockIdx.y * ASM_ROWS, nr = min(ASM_ROWS, M - i0);
   const int j0 = blockIdx.x * CB, nc = min(CB, N - j0);
-  asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, E3, asum, F2, bsum);
-  const AsmArgs a{M, Mp, L, w, res, plane, P, C, ldc, f0 != 0 || f1 != 0,
+  asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, eA, asum, eB, bsum);
+  const AsmArgs a{M, Mp, L, w, res, plane, P, C, Cup, ldc, f0 != 0 || f1 != 0,
                   (((uintptr_t)C) & 15) == 0};
   asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
 }
@@ -511,11 +518,11 @@ oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ C
   const int i0 = (local % tm) * ASM_ROWS, nr = min(ASM_ROWS, m - i0);
   const int j0 = (local / tm) * OZ_GASM_COLS, nc = min(OZ_GASM_COLS, n - j0);
   const int f0 = b.flag[4 * p], f1 = b.flag[4 * p + 1];
-  asm_tile_setup(t, i0, nr, j0, nc, q.k, q.w, LOWB, b.E3 + 3 * (size_t)q.rowoff,
-                 b.asum + 4 * (size_t)q.rowoff, b.F2 + 2 * (size_t)q.coloff,
+  asm_tile_setup(t, i0, nr, j0, nc, q.k, q.w, LOWB, b.eA + 3 * (size_t)q.rowoff,
+                 b.asum + 4 * (size_t)q.rowoff, b.eB + 2 * (size_t)q.coloff,
                  b.bsum + 4 * (size_t)q.coloff);
   const AsmArgs a{m, q.Mp, q.L, q.w, b.res + q.res_off, (size_t)q.Np * q.Mp, b.P + q.P_off, q.C,
-                  q.ldc, f0 != 0 || b.flag[1] != 0, (((uintptr_t)q.C) & 15) == 0};
+                  nullptr, q.ldc, f0 != 0 || b.flag[1] != 0, (((uintptr_t)q.C) & 15) == 0};
   asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
   if (threadIdx.x == 0 && (f0 | f1)) atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
   if (b.t_last) {
@@ -549,7 +556,7 @@ int oz_take_status(cudaStream_t s, int* status) {
 }
 
 int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long ldc,
-                    cudaStream_t st, bool merge_status) {
+                    cudaStream_t st, bool merge_status, double* Cup) {
   const OzProblem& pb = plan.pb;
   if (pb.M <= 0 || pb.N <= 0) return VCPCU_OK;
   const int tm = (pb.M + ASM_ROWS - 1) / ASM_ROWS;
@@ -566,8 +573,8 @@ int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long l
   const OzRadConst rc = oz_rad_const(plan);
   auto launch = [&](auto kernel) {
     kernel<<<grid, ASM_NT, 0, st>>>(pb.M, pb.N, pb.K, pb.Mp, pb.L, pb.w, CB, ws.res,
-                                    (size_t)pb.Np * pb.Mp, ws.E3, ws.F2, ws.asum, ws.bsum, ws.P,
-                                    C, ldc, ws.flag, merge_status ? 1 : 0, plan.basis, rc);
+                                    (size_t)pb.Np * pb.Mp, ws.eA, ws.eB, ws.asum, ws.bsum, ws.P,
+                                    C, Cup, ldc, ws.flag, merge_status ? 1 : 0, plan.basis, rc);
   };
   if (rc.lowb)
     launch(oz_crt_assemble_kernel<true>);

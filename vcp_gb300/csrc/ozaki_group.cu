@@ -39,12 +39,11 @@ struct BucketHost {
   OzGBucket dev;  // table pointers set at plan time, workspace pointers at record time
   OzPlan shape;   // radius pair list, Lmax-modulus pair list, fold count
   OzRadConst rc;
-  int nblk_rowmax = 0, nblk_split = 0, nitem_rad = 0, nitem_crt = 0, nblk_asm = 0;
+  int nblk_max = 0, nblk_split = 0, nitem_rad = 0, nitem_crt = 0, nblk_asm = 0;
   int wmax = 0;  // largest operand width w of the bucket's problems
   // workspace layout (byte offsets; the first zero_bytes are cleared per run)
-  size_t offRowmax = 0, offAsum = 0, offFlag = 0, zero_bytes = 0;
-  size_t offE3 = 0, offF2 = 0, offA = 0, offB = 0, offRes = 0, offP = 0;
-  size_t offMidB = 0, offRadB = 0, offBsum = 0, offMidA = 0, offRadA = 0;
+  size_t offEA = 0, offEB = 0, offAsum = 0, offBsum = 0, offFlag = 0, zero_bytes = 0;
+  size_t offA = 0, offB = 0, offRes = 0, offP = 0;
   size_t ws_bytes = 0;
 };
 
@@ -124,7 +123,7 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     host.resize(off + bytes);
     return off;
   };
-  struct Offs { size_t probs, brow, bspl, irad, icrt, basm, cols, prad, pcrt, pasm; };
+  struct Offs { size_t probs, bmax, bspl, irad, icrt, basm, pmax, pspl, prad, pcrt, pasm; };
   std::vector<Offs> toff;
   for (const std::vector<int>& ids : chunks) {
     const int n = (int)ids.size();
@@ -157,13 +156,12 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     b.dev.Lmax = Lmax;
     Offs o;
     o.probs = reserve(sizeof(OzGProb) * n);
-    o.brow = reserve(sizeof(int) * (n + 1));
+    o.bmax = reserve(sizeof(int) * (n + 1));
     o.bspl = reserve(sizeof(int) * (n + 1));
     o.irad = reserve(sizeof(int) * (n + 1));
     o.icrt = reserve(sizeof(int) * (n + 1));
     o.basm = reserve(sizeof(int) * (n + 1));
-    o.cols = reserve(sizeof(int) * (size_t)Ntot);
-    long long brow = 0, bspl = 0, irad = 0, icrt = 0, basm = 0, res = 0, P = 0;
+    long long bmax = 0, bspl = 0, irad = 0, icrt = 0, basm = 0, res = 0, P = 0;
     int rowoff = 0, coloff = 0;
     for (int t = 0; t < n; ++t) {
       const int id = ids[t];
@@ -192,18 +190,18 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       gp.res_off = res;
       gp.P_off = P;
       gp.orig = id;
+      int nmax, nspl;
+      oz_gprep_blocks(q.m, q.n, q.k, Kp, &gp, &nmax, &nspl);
       memcpy(host.data() + o.probs + sizeof(OzGProb) * t, &gp, sizeof(gp));
       int* v;
-      v = (int*)(host.data() + o.brow); v[t] = (int)brow;
+      v = (int*)(host.data() + o.bmax); v[t] = (int)bmax;
       v = (int*)(host.data() + o.bspl); v[t] = (int)bspl;
       v = (int*)(host.data() + o.irad); v[t] = (int)irad;
       v = (int*)(host.data() + o.icrt); v[t] = (int)icrt;
       v = (int*)(host.data() + o.basm); v[t] = (int)basm;
-      int* cols = (int*)(host.data() + o.cols);
-      for (int j = 0; j < gp.Np; ++j) cols[coloff + j] = t;
       const long long tiles = (long long)gp.tiles_m * gp.tiles_n;
-      brow += (long long)((q.m + 31) / 32) * ((q.k + 255) / 256);
-      bspl += (long long)(Kp / 64) * (gp.Mp / 32);
+      bmax += nmax;
+      bspl += nspl;
       irad += b.shape.rad.ngroups * tiles;
       icrt += gp.L * tiles;
       basm += (long long)((q.m + 127) / 128) * ((q.n + OZ_GASM_COLS - 1) / OZ_GASM_COLS);
@@ -212,39 +210,41 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       rowoff += gp.Mp;
       coloff += gp.Np;
     }
-    if (std::max({brow, bspl, irad, icrt, basm}) >= INT_MAX || Mtot >= INT_MAX ||
+    if (std::max({bmax, bspl, irad, icrt, basm}) >= INT_MAX || Mtot >= INT_MAX ||
         Ntot >= INT_MAX) {
       delete g;
       set_error("igemm_batched: the tensor-core batch is too large for one group");
       return VCPCU_ERR_INVALID_ARG;
     }
     int* v;
-    v = (int*)(host.data() + o.brow); v[n] = (int)brow;
+    v = (int*)(host.data() + o.bmax); v[n] = (int)bmax;
     v = (int*)(host.data() + o.bspl); v[n] = (int)bspl;
     v = (int*)(host.data() + o.irad); v[n] = (int)irad;
     v = (int*)(host.data() + o.icrt); v[n] = (int)icrt;
     v = (int*)(host.data() + o.basm); v[n] = (int)basm;
-    b.nblk_rowmax = (int)brow;
+    b.nblk_max = (int)bmax;
     b.nblk_split = (int)bspl;
     b.nitem_rad = (int)irad;
     b.nitem_crt = (int)icrt;
-    // item -> problem maps of the two kinds of slice GEMM launches (one load
-    // per work item instead of a binary search over the prefixes above)
+    // block / item -> problem maps (one load instead of a binary search over
+    // the prefixes above)
+    o.pmax = reserve(sizeof(int) * (size_t)(bmax > 0 ? bmax : 1));
+    o.pspl = reserve(sizeof(int) * (size_t)(bspl > 0 ? bspl : 1));
     o.prad = reserve(sizeof(int) * (size_t)(irad > 0 ? irad : 1));
     o.pcrt = reserve(sizeof(int) * (size_t)(icrt > 0 ? icrt : 1));
     o.pasm = reserve(sizeof(int) * (size_t)(basm > 0 ? basm : 1));
     {
-      const int* pr = (const int*)(host.data() + o.irad);
-      const int* pc = (const int*)(host.data() + o.icrt);
-      const int* pa = (const int*)(host.data() + o.basm);
-      int* mr = (int*)(host.data() + o.prad);
-      int* mc = (int*)(host.data() + o.pcrt);
-      int* ma = (int*)(host.data() + o.pasm);
-      for (int t = 0; t < n; ++t) {
-        for (int it = pr[t]; it < pr[t + 1]; ++it) mr[it] = t;
-        for (int it = pc[t]; it < pc[t + 1]; ++it) mc[it] = t;
-        for (int it = pa[t]; it < pa[t + 1]; ++it) ma[it] = t;
-      }
+      auto spread = [&](size_t prefix, size_t map) {
+        const int* p = (const int*)(host.data() + prefix);
+        int* m = (int*)(host.data() + map);
+        for (int t = 0; t < n; ++t)
+          for (int it = p[t]; it < p[t + 1]; ++it) m[it] = t;
+      };
+      spread(o.bmax, o.pmax);
+      spread(o.bspl, o.pspl);
+      spread(o.irad, o.prad);
+      spread(o.icrt, o.pcrt);
+      spread(o.basm, o.pasm);
     }
     b.nblk_asm = (int)basm;
     b.dev.Mtot = (int)Mtot;
@@ -256,17 +256,12 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       w = al256g(w + bytes);
       return off;
     };
-    b.offRowmax = take(sizeof(unsigned long long) * 3 * Mtot);
+    b.offEA = take(sizeof(uint32_t) * 3 * Mtot);
+    b.offEB = take(sizeof(uint32_t) * 2 * Ntot);
     b.offAsum = take(sizeof(unsigned long long) * 4 * Mtot);
+    b.offBsum = take(sizeof(unsigned long long) * 4 * Ntot);
     b.offFlag = take(sizeof(int) * 4 * (size_t)n);
     b.zero_bytes = w;
-    b.offE3 = take(sizeof(int) * 3 * Mtot);
-    b.offF2 = take(sizeof(int) * 2 * Ntot);
-    b.offMidB = take(sizeof(double) * (size_t)Ntot * Kp);
-    b.offRadB = take(sizeof(double) * (size_t)Ntot * Kp);
-    b.offBsum = take(sizeof(unsigned long long) * 4 * Ntot);
-    b.offMidA = take(sizeof(double) * (size_t)Mtot * Kp);
-    b.offRadA = take(sizeof(double) * (size_t)Mtot * Kp);
     b.offA = take(sizeof(uint16_t) * (size_t)(Lmax + 4) * Mtot * Kp);
     b.offB = take(sizeof(uint16_t) * (size_t)(Lmax + 4) * Ntot * Kp);
     b.offRes = take((size_t)res);
@@ -306,15 +301,16 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     OzGBucket& d = g->buckets[i].dev;
     const Offs& o = toff[i];
     d.probs = (const OzGProb*)(tb + o.probs);
-    d.blk_rowmax = (const int*)(tb + o.brow);
+    d.blk_max = (const int*)(tb + o.bmax);
+    d.prob_max = (const int*)(tb + o.pmax);
     d.blk_split = (const int*)(tb + o.bspl);
+    d.prob_split = (const int*)(tb + o.pspl);
     d.item_rad = (const int*)(tb + o.irad);
     d.item_crt = (const int*)(tb + o.icrt);
     d.prob_rad = (const int*)(tb + o.prad);
     d.prob_crt = (const int*)(tb + o.pcrt);
     d.blk_asm = (const int*)(tb + o.basm);
     d.prob_asm = (const int*)(tb + o.pasm);
-    d.col_prob = (const int*)(tb + o.cols);
   }
   *out = g;
   return VCPCU_OK;
@@ -325,16 +321,11 @@ namespace {
 int record_chunk(const BucketHost& b, uint8_t* ws, unsigned long long* t_first,
                  unsigned long long* t_last, cudaStream_t s) {
   OzGBucket d = b.dev;
-  d.rowmax = (unsigned long long*)(ws + b.offRowmax);
+  d.eA = (uint32_t*)(ws + b.offEA);
+  d.eB = (uint32_t*)(ws + b.offEB);
   d.asum = (unsigned long long*)(ws + b.offAsum);
-  d.flag = (int*)(ws + b.offFlag);
-  d.E3 = (int*)(ws + b.offE3);
-  d.F2 = (int*)(ws + b.offF2);
-  d.midB = (double*)(ws + b.offMidB);
-  d.radB = (double*)(ws + b.offRadB);
   d.bsum = (unsigned long long*)(ws + b.offBsum);
-  d.midA = (double*)(ws + b.offMidA);
-  d.radA = (double*)(ws + b.offRadA);
+  d.flag = (int*)(ws + b.offFlag);
   d.planesA = (uint16_t*)(ws + b.offA);
   d.planesB = (uint16_t*)(ws + b.offB);
   d.res = ws + b.offRes;
@@ -346,7 +337,7 @@ int record_chunk(const BucketHost& b, uint8_t* ws, unsigned long long* t_first,
   int st;
   {
     PhaseTimer t(0, s);
-    if ((st = oz_gprep(d, b.nblk_rowmax, b.nblk_split, b.wmax, s))) return st;
+    if ((st = oz_gprep(d, b.nblk_max, b.nblk_split, b.wmax, s))) return st;
   }
   {
     PhaseTimer t(1, s);
