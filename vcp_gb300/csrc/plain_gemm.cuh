@@ -21,16 +21,24 @@ int launch_interval_gemm_plain(int M, int N, int K, const double* A, long lda,
 size_t interval_gemm_plain_ws_bytes(int M, int N, int K);
 
 // Thin right factor: products with N <= kThinN columns run in
-// interval_gemm_thin_kernel (two lanes per row of C, no tile padding), with
-// the same chains and results as the tile kernel.  a_point / b_point: A / B
-// hold point entries (doubles, radius 0) instead of kv intervals.  ws holds
-// interval_gemm_thin_ws_bytes(M, N, K, a_point) bytes (with an interval A:
-// 32 bytes per entry of A for the operand pairs of the two lanes).
+// interval_gemm_thin_kernel (plain_thin.cu: one chain per lane, no tile
+// padding), with the same chains and results as the tile kernel.  The left
+// factor holds kv intervals, plain doubles (radius 0), or intervals E that
+// enter as kv |E| or |E - I|; b_point: B holds doubles instead of intervals.
+// ws holds interval_gemm_thin_ws_bytes(N, K) bytes.
 constexpr int kThinN = 16;
-int launch_interval_gemm_thin(int M, int N, int K, const double* A, long lda, bool a_point,
+enum ThinLeft { THIN_INTERVAL = 0, THIN_POINT = 1, THIN_ABS_SHIFT = 2 };
+int launch_interval_gemm_thin(int M, int N, int K, const double* A, long lda, ThinLeft left,
                               const double* B, long ldb, bool b_point, double* C, long ldc,
                               double* ws, cudaStream_t s);
-size_t interval_gemm_thin_ws_bytes(int M, int N, int K, bool a_point);
+size_t interval_gemm_thin_ws_bytes(int N, int K);
+
+// Row sums of kv |X| (shift: |X - I|) of an n x n interval matrix, columns
+// ascending: the upper ends rounded up to rows[i] and, with sums != NULL, the
+// lower ends rounded down and the upper ones rounded up to sums[2i],
+// sums[2i + 1] (kv interval sums).  X 16-byte aligned.
+int launch_abs_row_sums(int n, const double* X, long ldx, bool shift, double* rows, double* sums,
+                        cudaStream_t s);
 
 // R (M x N) = Y (M x K point) [C] (K x N kv) with imats::mul_m_im's loop
 // (vcp/imats.hpp:203-213): kv interval products and sums term by term.

@@ -93,61 +93,6 @@ __global__ void mirror_upper(int n, double* __restrict__ C, long ldc) {
 // The upper end of kv abs([lo, up]), on the integer pipe (swfp.cuh).
 __device__ __forceinline__ double abs_sup(double lo, double up) { return sw_abs_sup(lo, up); }
 
-// Row sums of |RA - I| rounded upward, column order ascending (one thread per
-// row; a warp reads 32 consecutive rows of one column).  The sums are
-// sequential chains, so there are only n threads: each keeps two groups of
-// PF columns in flight ahead of its additions.
-template <bool SHIFT = true>
-__global__ void norm_rows(int n, const double* __restrict__ C, long ldc,
-                          double* __restrict__ rows) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  constexpr int PF = 16;
-  const double2* c2 = reinterpret_cast<const double2*>(C);
-  auto load = [&](int j) -> double2 {
-    return j < n ? c2[i + (long)j * ldc] : make_double2(0.0, 0.0);
-  };
-  double2 cur[PF], nxt[PF];
-#pragma unroll
-  for (int p = 0; p < PF; ++p) cur[p] = load(p);
-  // the warp's rows i0 .. i0 + 31 meet the diagonal only in the column
-  // groups that overlap them (a warp-uniform test): elsewhere no FP64
-  // subtraction is issued, not even predicated off
-  const int i0 = i & ~31;
-  double s = 0.0;
-  for (int jb = 0; jb < n; jb += PF) {
-#pragma unroll
-    for (int p = 0; p < PF; ++p) nxt[p] = load(jb + PF + p);
-    if (!SHIFT || jb + PF <= i0 || jb >= i0 + 32) {
-#pragma unroll
-      for (int p = 0; p < PF; ++p) {
-        const int j = jb + p;
-        if (j < n) {
-          const double mg = abs_sup(cur[p].x, cur[p].y);
-          s = (j == 0) ? mg : __dadd_ru(s, mg);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int p = 0; p < PF; ++p) {
-        const int j = jb + p;
-        if (j < n) {
-          double lo = cur[p].x, up = cur[p].y;
-          if (i == j) {
-            lo = __dsub_rd(lo, 1.0);
-            up = __dsub_ru(up, 1.0);
-          }
-          const double mg = abs_sup(lo, up);
-          s = (j == 0) ? mg : __dadd_ru(s, mg);
-        }
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < PF; ++p) cur[p] = nxt[p];
-  }
-  rows[i] = s;
-}
-
 // largest entry (NaN propagates)
 __global__ void max_of(int n, const double* __restrict__ v, double* __restrict__ out) {
   __shared__ double red[256];
@@ -181,9 +126,10 @@ int igemm_point_dispatch(int interval_side, int m, int n, int k, const double* L
     // thin plain product: the kernel reads the point factor as is
     if (m <= 0 || n <= 0) return VCPCU_OK;
     Scratch ws;
-    int st = ws.alloc(interval_gemm_thin_ws_bytes(m, n, k, interval_side == 1), s);
+    int st = ws.alloc(interval_gemm_thin_ws_bytes(n, k), s);
     if (st) return st;
-    return launch_interval_gemm_thin(m, n, k > 0 ? k : 0, L, ldl, interval_side == 1, R, ldr,
+    return launch_interval_gemm_thin(m, n, k > 0 ? k : 0, L, ldl,
+                                     interval_side == 1 ? THIN_POINT : THIN_INTERVAL, R, ldr,
                                      interval_side == 0, C, ldc, (double*)ws.ptr, s);
   }
   if (form == VCPCU_FORM_OZAKI) {
@@ -278,8 +224,7 @@ int norm_dispatch(int n, const double* R, long ldr, const double* A, long lda, d
   double* rows = RA + 2 * (size_t)n * n;
   st = igemm_point_dispatch(1, n, n, n, R, ldr, A, lda, RA, n, form, slices, s);
   if (st) return st;
-  norm_rows<<<(n + 127) / 128, 128, 0, s>>>(n, RA, n, rows);
-  VCPCU_LAUNCH_CHECK("norm_rows");
+  if ((st = launch_abs_row_sums(n, RA, n, true, rows, nullptr, s))) return st;
   max_of<<<1, 256, 0, s>>>(n, rows, bound);
   VCPCU_LAUNCH_CHECK("max_of");
   return VCPCU_OK;
@@ -368,7 +313,7 @@ __global__ void max_last(int n, const double* __restrict__ v, double* __restrict
 
 // g = [t, t] / (1 - [G, G]) by kv's interval division with both operands
 // positive: [RD(t / RU(1 - G)), RU(t / RD(1 - G))]; then E -> |E| with the
-// diagonal shifted (E = RA - I) is done by abs_shift, and H's factor
+// diagonal shifted (E = RA - I) is done by abs_shift (or as the thin kernel reads E), and H's factor
 // (g ... g) by fill_iv.
 __global__ void lss_scale(const double* __restrict__ G, const double* __restrict__ t,
                           double* __restrict__ g) {
@@ -387,15 +332,14 @@ __global__ void lss_scale(const double* __restrict__ G, const double* __restrict
   g[1] = up;
 }
 
-// E(i, i) -= 1 (interval minus point; SHIFT), then E -> kv abs(E), in place.
-template <bool SHIFT = true>
+// E(i, i) -= 1 (interval minus point), then E -> kv abs(E), in place.
 __global__ void abs_shift(int n, double* __restrict__ E) {
   const long total = (long)n * n;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
     const long i = idx % n, j = idx / n;
     double2 e = reinterpret_cast<const double2*>(E)[idx];
-    if (SHIFT && i == j) {
+    if (i == j) {
       e.x = __dsub_rd(e.x, 1.0);
       e.y = __dsub_ru(e.y, 1.0);
     }
@@ -491,36 +435,6 @@ __global__ void sub_lambda(int n, double* __restrict__ C, const double* __restri
   }
 }
 
-// imats::mul_im_m 'M' x 'C' with the ones vector (vcp/imats.hpp:88-97): per row
-// c = X(i, 0), then c = X(i, j) + c outward, j ascending.
-__global__ void iv_row_sums(int n, const double* __restrict__ X, double* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  constexpr int PF = 16;
-  const double2* x2 = reinterpret_cast<const double2*>(X);
-  auto load = [&](int j) -> double2 { return j < n ? x2[i + (long)j * n] : make_double2(0.0, 0.0); };
-  double2 cur[PF], nxt[PF];
-#pragma unroll
-  for (int p = 0; p < PF; ++p) cur[p] = load(p);
-  double lo = 0.0, up = 0.0;
-  for (int jb = 0; jb < n; jb += PF) {
-#pragma unroll
-    for (int p = 0; p < PF; ++p) nxt[p] = load(jb + PF + p);
-#pragma unroll
-    for (int p = 0; p < PF; ++p) {
-      const int j = jb + p;
-      if (j < n) {
-        lo = j == 0 ? cur[p].x : __dadd_rd(cur[p].x, lo);
-        up = j == 0 ? cur[p].y : __dadd_ru(cur[p].y, up);
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < PF; ++p) cur[p] = nxt[p];
-  }
-  out[2 * i] = lo;
-  out[2 * i + 1] = up;
-}
-
 // lam_i = lambda_i + [-u, u], u = RU(sup Re_i + sup(g * Se_i)) (mulsm, addmm and
 // the symmetric widening of vcp/imats.hpp:488-499); g = sc[0..1].
 __global__ void eig_final(int n, const double* __restrict__ Re, const double* __restrict__ Se,
@@ -567,23 +481,14 @@ int ieig_stage2_dispatch(int n, const double* lambda, const double* Y, long ldy,
   else
     st = igemm_point_dispatch(1, n, n, n, Y, ldy, C, n, P, n, form, slices, s);
   if (st) return st;
-  norm_rows<false><<<(n + 127) / 128, 128, 0, s>>>(n, P, n, rows);
-  VCPCU_LAUNCH_CHECK("norm_rows");
+  // the upper ends of |R| e are the row sums of its norm: one pass for both
+  if ((st = launch_abs_row_sums(n, P, n, false, rows, Re, s))) return st;
   max_last<<<1, 256, 0, s>>>(n, rows, sc);
   VCPCU_LAUNCH_CHECK("max_last");
-  abs_shift<false><<<grid1((long)n * n), 256, 0, s>>>(n, P);
-  VCPCU_LAUNCH_CHECK("abs_shift");
-  iv_row_sums<<<(n + 127) / 128, 128, 0, s>>>(n, P, Re);
-  VCPCU_LAUNCH_CHECK("iv_row_sums");
   if ((st = igemm_point_dispatch(1, n, n, n, Y, ldy, BX, n, P, n, form, slices, s))) return st;
-  norm_rows<true><<<(n + 127) / 128, 128, 0, s>>>(n, P, n, rows);
-  VCPCU_LAUNCH_CHECK("norm_rows");
+  if ((st = launch_abs_row_sums(n, P, n, true, rows, Se, s))) return st;
   max_last<<<1, 256, 0, s>>>(n, rows, bound);
   VCPCU_LAUNCH_CHECK("max_last");
-  abs_shift<true><<<grid1((long)n * n), 256, 0, s>>>(n, P);
-  VCPCU_LAUNCH_CHECK("abs_shift");
-  iv_row_sums<<<(n + 127) / 128, 128, 0, s>>>(n, P, Se);
-  VCPCU_LAUNCH_CHECK("iv_row_sums");
   lss_scale<<<1, 1, 0, s>>>(bound, sc, sc + 1);  // g = [Rinf, Rinf] / (1 - [Sinf, Sinf])
   VCPCU_LAUNCH_CHECK("lss_scale");
   eig_final<<<(n + 127) / 128, 128, 0, s>>>(n, Re, Se, sc + 1, lambda, lam);
@@ -638,8 +543,7 @@ int ilss_verify_dispatch(int n, int nrhs, const double* A, long lda, const doubl
   VCPCU_LAUNCH_CHECK("iv_sub");
   if ((st = igemm_point_dispatch(1, n, nrhs, n, R, ldr, P, n, r, n, tf, slices, s))) return st;
   if ((st = igemm_point_dispatch(1, n, n, n, R, ldr, A, lda, E, n, form, slices, s))) return st;
-  norm_rows<<<(n + 127) / 128, 128, 0, s>>>(n, E, n, rows);
-  VCPCU_LAUNCH_CHECK("norm_rows");
+  if ((st = launch_abs_row_sums(n, E, n, true, rows, nullptr, s))) return st;
   max_of<<<1, 256, 0, s>>>(n, rows, bound);
   VCPCU_LAUNCH_CHECK("max_of");
   mag_rows<<<(n + 127) / 128, 128, 0, s>>>(n, nrhs, r, rows);
@@ -648,11 +552,19 @@ int ilss_verify_dispatch(int n, int nrhs, const double* A, long lda, const doubl
   VCPCU_LAUNCH_CHECK("max_last");
   lss_scale<<<1, 1, 0, s>>>(bound, sc, sc + 1);
   VCPCU_LAUNCH_CHECK("lss_scale");
-  abs_shift<<<grid1((long)n * n), 256, 0, s>>>(n, E);
-  VCPCU_LAUNCH_CHECK("abs_shift");
   fill_iv<<<grid1((long)n * nrhs), 256, 0, s>>>((long)n * nrhs, sc + 1, T);
   VCPCU_LAUNCH_CHECK("fill_iv");
-  if ((st = igemm_any(n, nrhs, n, E, n, T, n, H, n, tf, slices, s))) return st;
+  if (tf == VCPCU_FORM_PLAIN && nrhs <= kThinN) {  // |E| formed as its entries are read
+    Scratch tw;
+    if ((st = tw.alloc(interval_gemm_thin_ws_bytes(nrhs, n), s))) return st;
+    st = launch_interval_gemm_thin(n, nrhs, n, E, n, THIN_ABS_SHIFT, T, n, false, H, n,
+                                   (double*)tw.ptr, s);
+  } else {
+    abs_shift<<<grid1((long)n * n), 256, 0, s>>>(n, E);
+    VCPCU_LAUNCH_CHECK("abs_shift");
+    st = igemm_any(n, nrhs, n, E, n, T, n, H, n, tf, slices, s);
+  }
+  if (st) return st;
   lss_final<<<grid1((long)n * nrhs), 256, 0, s>>>(n, nrhs, r, H, mx, ldmx, x, ldx);
   VCPCU_LAUNCH_CHECK("lss_final");
   return VCPCU_OK;
