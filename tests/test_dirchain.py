@@ -80,10 +80,11 @@ int main() {
         auto value = [&](int p) { return vx[p]; };
         chain_add_n<true, 8>(bu, get, value);
         chain_add_n<false, 8>(bd, get, value);
-        chain_fma_n<8>(bf, [&](int p, ChainFactor* x, ChainFactor* y) {
+        auto factors = [&](int p, ChainFactor* x, ChainFactor* y) {
           *x = chain_factor(va[p]);
           *y = chain_factor(vb[p]);
-        });
+        };
+        chain_fma_n<8>(bf, factors, factors);
         if (!same(chain_value(bu), cu) || !same(chain_value(bd), cd) ||
             !same(chain_value(bf), cf)) ++bad;
       }

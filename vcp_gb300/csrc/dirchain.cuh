@@ -174,6 +174,18 @@ OZ_HD void chain_fma(DirChain& x, const ChainFactor& fa, const ChainFactor& fb) 
   chain_carry<true>(x);
 }
 
+// x >> s for any s >= 0 (the device instruction takes more than 63 for 63; a
+// negative s gives a value that its caller discards).
+OZ_HD long long chain_shr(long long x, int s) {
+#ifdef __CUDA_ARCH__
+  long long r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+  return r;
+#else
+  return x >> (s < 0 ? 0 : (s > 63 ? 63 : s));
+#endif
+}
+
 // N steps at once.  With every term below 2^53 units, the terms in units are
 // independent of one another, and where the sum with all of them stays below
 // 2^53 units no step doubles the unit: one sum is the whole batch (the common
@@ -182,9 +194,10 @@ OZ_HD void chain_fma(DirChain& x, const ChainFactor& fa, const ChainFactor& fb) 
 // floors again).  Away from both: one step after the other.
 constexpr int CHAIN_TOP = 2000;  // exponents from here on step singly
 
+// y[p]: floor of the term in units (RD), or one less than its ceiling (RU).
 template <bool UP, int N>
 OZ_HD void chain_batch(DirChain& x, const long long (&y)[N]) {
-  long long S = x.c;
+  long long S = x.c + (UP ? N : 0);
 #pragma unroll
   for (int p = 0; p < N; ++p) S += y[p];
   if ((uint32_t)((uint64_t)S >> 32) < (1u << 21)) {
@@ -194,7 +207,7 @@ OZ_HD void chain_batch(DirChain& x, const long long (&y)[N]) {
   int k = 0;
 #pragma unroll
   for (int p = 0; p < N; ++p) {
-    x.c += UP ? ((y[p] - 1) >> k) + 1 : y[p] >> k;
+    x.c += (y[p] >> k) + (UP ? 1 : 0);
     if ((uint32_t)((uint64_t)x.c >> 32) >= (1u << 21)) {
       x.c = (x.c + (UP ? 1 : 0)) >> 1;
       ++k;
@@ -214,10 +227,7 @@ OZ_HD void chain_add_n(DirChain& x, GET get, VALUE value) {
     int e;
     get(p, &y[p], &e);
     em = em > e ? em : e;
-    int d = x.U - e;
-    d = d < 63 ? d : 63;
-    d = d > 0 ? d : 0;
-    y[p] = UP ? ((y[p] - 1) >> d) + 1 : y[p] >> d;
+    y[p] = chain_shr(UP ? y[p] - 1 : y[p], x.U - e);
   }
   if (x.U < em || x.U > CHAIN_TOP || x.U < 1) {
 #pragma unroll 1
@@ -232,28 +242,28 @@ OZ_HD void chain_add_n(DirChain& x, GET get, VALUE value) {
   chain_batch<UP, N>(x, y);
 }
 
-// c = RU(c + a_p b_p), p ascending; get(p, &fa, &fb) gives the factors.
-template <int N, typename GET>
-OZ_HD void chain_fma_n(DirChain& x, GET get) {
+// c = RU(c + a_p b_p), p ascending; get(p, &fa, &fb) gives the factors, again
+// (p not a constant: from memory) for the single steps.
+template <int N, typename GET, typename AGAIN>
+OZ_HD void chain_fma_n(DirChain& x, GET get, AGAIN again) {
   long long y[N];
   int sm = 1;
+  const int U = x.U + 1023;
 #pragma unroll
   for (int p = 0; p < N; ++p) {
     ChainFactor fa, fb;
     get(p, &fa, &fb);
-    int s = x.U + 1023 - fa.e - fb.e;
+    const int s = U - fa.e - fb.e;
     sm = sm < s ? sm : s;
-    s = s < 63 ? s : 63;
-    s = s > 0 ? s : 0;
     const long long t0 = (long long)fa.l * fb.l - 1;
     const long long t1 = (long long)fa.h * fb.l + ((long long)fa.l * fb.h + (t0 >> 26));
-    y[p] = (((long long)fa.h * fb.h + (t1 >> 26)) >> s) + 1;
+    y[p] = chain_shr((long long)fa.h * fb.h + (t1 >> 26), s);
   }
   if (sm < 1 || x.U > CHAIN_TOP || x.U < 1) {
 #pragma unroll 1
     for (int p = 0; p < N; ++p) {
       ChainFactor fa, fb;
-      get(p, &fa, &fb);
+      again(p, &fa, &fb);
       chain_fma(x, fa, fb);
     }
     return;

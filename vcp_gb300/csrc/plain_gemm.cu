@@ -19,9 +19,10 @@
 //     t2 = chain_ru(rA*|mB|)        (:281)
 //     T  = t1 +ru t2 ; up = up +ru T ; lo = lo -rd T   (:283-286)
 // with mA, rA, mB, rB from kv-style midrad (pidblas.hpp:43-51).
-#include <type_traits>
+#include <mutex>
 
 #include "common.cuh"
+#include "dirchain.cuh"
 #include "plain_gemm.cuh"
 #include "swfp.cuh"
 
@@ -29,7 +30,7 @@ namespace vcpcu {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
+constexpr int BM = 64, BN = 64, BK = 16, NT = 256, BKI = 8;
 
 // Kinds of chains a kernel runs per C entry.
 enum Kind { K_RN = 0, K_RU = 1, K_RD = 2, K_UD = 3 };
@@ -41,49 +42,75 @@ __device__ __forceinline__ double fma_k(double a, double b, double c) {
   return __fma_rn(a, b, c);
 }
 
+// Tiles of the two products below: 32 rows (a row per lane) x 4 CW columns;
+// each of four warps -- one per SM sub-partition -- owns CW columns.  Both are
+// bound by the FP64 pipe (64 cycles per warp instruction), so what counts is
+// that the SMs' sub-partitions get the same number of (32-row, column) chain
+// sets: CW = 8, 4 or 2, whichever leaves the fullest one the least to do,
+// the widest of equals.
+constexpr int TROWS = 32;
+// The cost of a width in blocks on the fullest SM x CW, with `penalty` 32nds
+// more at CW = 4 and twice that at CW = 2 (a narrower block stages as much of
+// A), and a quarter more for a single block on an SM (nothing runs while it
+// waits at its barriers).  Interval product, us at CW = 8 / 4 / 2: 512^3 659 /
+// 683 / 684, 256^3 254 / 142 / 119, 300 x 200 x 700 591 / 321 / 271.
+inline int tile_cols(int M, int N, int penalty) {
+  const long mt = (M + TROWS - 1) / TROWS;
+  int best = 8;
+  double cost = 0.0;
+  for (int cw = 8, f = 32; cw >= 2; cw >>= 1, f += penalty) {
+    const long rounds = (mt * ((N + 4 * cw - 1) / (4 * cw)) + 151) / 152;
+    const double c = (rounds == 1 ? 1.25 : 1.0) * (double)rounds * cw * f;
+    if (cw == 8 || c < cost) {
+      best = cw;
+      cost = c;
+    }
+  }
+  return best;
+}
+
 // One-direction (KIND RN/RU/RD) or up+down (K_UD) point GEMM.
-// GEMM naming: C(M x N) = A(M x K) * B(K x N), column-major.
-template <int KIND>
-__global__ void __launch_bounds__(NT)
+// GEMM naming: C(M x N) = A(M x K) * B(K x N), column-major.  n = 1024, both
+// directions: 64 x 64 tiles 4.12 ms, these 3.47 ms (the FP64 rate).
+template <int KIND, int CW>
+__global__ void __launch_bounds__(128)
 point_gemm_kernel(int M, int N, int K, const double* __restrict__ A, long lda,
                   const double* __restrict__ B, long ldb, double* __restrict__ C0,
                   double* __restrict__ C1, long ldc) {
-  constexpr int NCH = (KIND == K_UD) ? 2 : 1;
-  __shared__ double As[2][BK][BM];
-  __shared__ double Bs[2][BK][BN];
+  constexpr int NCH = (KIND == K_UD) ? 2 : 1, COLS = 4 * CW;
+  constexpr int QA = TROWS * BK / 128, QB = COLS * BK / 128;
+  __shared__ double As[2][BK][TROWS];
+  __shared__ double Bs[2][BK][COLS];
 
-  const int tid = threadIdx.x;
-  const int tr = tid / 16, tc = tid % 16;
-  const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int mt = (M + TROWS - 1) / TROWS;
+  const int row0 = (blockIdx.x % mt) * TROWS, col0 = (blockIdx.x / mt) * COLS;
+  const int b_k = tid % BK, b_j = tid / BK;
 
-  // loader coordinates
-  const int a_i = tid % BM, a_k = tid / BM;        // A: 4 rows of k per pass
-  const int b_k = tid % BK, b_j = tid / BK;        // B: 16 columns per pass
-
-  double acc[NCH][4][4];
+  double acc[NCH][CW];
 #pragma unroll
   for (int c = 0; c < NCH; ++c)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[c][i][j] = 0.0;
+    for (int j = 0; j < CW; ++j) acc[c][j] = 0.0;
 
-  double ra[4], rb[4];
+  double ra[QA], rb[QB];
   auto load_tile = [&](int k0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int gi = row0 + a_i, gk = k0 + a_k + 4 * q;
+    for (int q = 0; q < QA; ++q) {
+      const int gi = row0 + lane, gk = k0 + warp + 4 * q;
       ra[q] = (gi < M && gk < K) ? A[gi + gk * lda] : 0.0;
-      int hk = k0 + b_k, hj = col0 + b_j + 16 * q;
+    }
+#pragma unroll
+    for (int q = 0; q < QB; ++q) {
+      const int hk = k0 + b_k, hj = col0 + b_j + (128 / BK) * q;
       rb[q] = (hk < K && hj < N) ? B[hk + hj * ldb] : 0.0;
     }
   };
   auto store_tile = [&](int buf) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      As[buf][a_k + 4 * q][a_i] = ra[q];
-      Bs[buf][b_k][b_j + 16 * q] = rb[q];
-    }
+    for (int q = 0; q < QA; ++q) As[buf][warp + 4 * q][lane] = ra[q];
+#pragma unroll
+    for (int q = 0; q < QB; ++q) Bs[buf][b_k][b_j + (128 / BK) * q] = rb[q];
   };
 
   const int nk = (K + BK - 1) / BK;
@@ -95,39 +122,44 @@ point_gemm_kernel(int M, int N, int K, const double* __restrict__ A, long lda,
     if (t + 1 < nk) load_tile((t + 1) * BK);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      double a[4], b[4];
+      const double a = As[buf][kk][lane];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk][tr + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk][tc + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (KIND == K_UD) {
-            acc[0][i][j] = __fma_ru(a[i], b[j], acc[0][i][j]);
-            acc[NCH - 1][i][j] = __fma_rd(a[i], b[j], acc[NCH - 1][i][j]);
-          } else {
-            acc[0][i][j] = fma_k<KIND>(a[i], b[j], acc[0][i][j]);
-          }
+      for (int j = 0; j < CW; ++j) {
+        const double b = Bs[buf][kk][warp * CW + j];
+        if (KIND == K_UD) {
+          acc[0][j] = __fma_ru(a, b, acc[0][j]);
+          acc[NCH - 1][j] = __fma_rd(a, b, acc[NCH - 1][j]);
+        } else {
+          acc[0][j] = fma_k<KIND>(a, b, acc[0][j]);
         }
+      }
     }
-    if (t + 1 < nk) {
-      store_tile(buf ^ 1);
-    }
+    if (t + 1 < nk) store_tile(buf ^ 1);
     __syncthreads();
   }
 
+  const int gi = row0 + lane;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int gi = row0 + tr + 16 * i, gj = col0 + tc + 16 * j;
-      if (gi < M && gj < N) {
-        C0[gi + gj * ldc] = acc[0][i][j];
-        if (KIND == K_UD) C1[gi + gj * ldc] = acc[NCH - 1][i][j];
-      }
+  for (int j = 0; j < CW; ++j) {
+    const int gj = col0 + warp * CW + j;
+    if (gi < M && gj < N) {
+      C0[gi + gj * ldc] = acc[0][j];
+      if (KIND == K_UD) C1[gi + gj * ldc] = acc[NCH - 1][j];
     }
+  }
+}
+
+template <int KIND>
+void point_launch(int M, int N, int K, const double* A, long lda, const double* B, long ldb,
+                  double* C0, double* C1, long ldc, cudaStream_t s) {
+  const int cw = tile_cols(M, N, 0);
+  const unsigned grid = (unsigned)((M + TROWS - 1) / TROWS) * (unsigned)((N + 4 * cw - 1) / (4 * cw));
+  if (cw == 8)
+    point_gemm_kernel<KIND, 8><<<grid, 128, 0, s>>>(M, N, K, A, lda, B, ldb, C0, C1, ldc);
+  else if (cw == 4)
+    point_gemm_kernel<KIND, 4><<<grid, 128, 0, s>>>(M, N, K, A, lda, B, ldb, C0, C1, ldc);
+  else
+    point_gemm_kernel<KIND, 2><<<grid, 128, 0, s>>>(M, N, K, A, lda, B, ldb, C0, C1, ldc);
 }
 
 // C = 0 for the n <= 0 (empty inner dimension) case of vblas rmatmul.
@@ -192,114 +224,168 @@ namespace {
 
 // Fused mid-rad interval GEMM over prepped planes (ld = M for A planes,
 // ld = K for B planes).  Writes C as {inf, sup} pairs (ld in intervals).
-// Five operand planes are staged per k step, so the k tile is BKI = 8 deep
-// (double-buffered: 40 KB of shared memory).
-constexpr int BKI = 8;
-__global__ void __launch_bounds__(NT)
+//
+// The two midpoint chains of an entry run on the FP64 pipe (warps 0 .. 3), the
+// two radius chains -- sums of non-negative products rounded up -- on the
+// integer pipe beside it (warps 4 .. 7 and 8 .. 11, dirchain.cuh, eight steps
+// at a time), each warp on CW columns of the block's 32 rows, a row per lane.  The FP64
+// pipe then has 2 instead of 4 instructions per entry and step: it is the
+// bound, the integer warps take about half the issue slots beside it.  The
+// radius chains' states live in shared memory between batches (their code is
+// one loop over the columns).  n = 512: 64 x 64 tiles with four FP64 chains
+// 2.07 ms, this 0.66; n = 1024 14.1 and
+// 4.4 ms (3.5 at the FP64 rate).
+constexpr int ITN = 384;  // threads
+template <int CW>
+struct ITile {
+  struct Stage {
+    double am[BKI][TROWS];
+    ChainFactor ap[BKI][TROWS], ar[BKI][TROWS];
+    double bm[BKI][4 * CW];
+    ChainFactor br[BKI][4 * CW], bs[BKI][4 * CW];
+  } st[2];
+  long long c[2][4 * CW][TROWS];
+  int U[2][4 * CW][TROWS];
+};
+
+template <int CW>
+__global__ void __launch_bounds__(ITN, 2)
 interval_gemm_kernel(int M, int N, int K, const double* __restrict__ mA,
                      const double* __restrict__ pA, const double* __restrict__ rA,
                      const double* __restrict__ mB, const double* __restrict__ rB,
                      double* __restrict__ C, long ldc) {
-  __shared__ double Am[2][BKI][BM], Ap[2][BKI][BM], Ar[2][BKI][BM];
-  __shared__ double Bm[2][BKI][BN], Br[2][BKI][BN];
+  extern __shared__ __align__(16) uint8_t plain_smem[];
+  ITile<CW>& sm = *reinterpret_cast<ITile<CW>*>(plain_smem);
+  constexpr int COLS = 4 * CW;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int mt = (M + TROWS - 1) / TROWS;
+  const int row0 = (blockIdx.x % mt) * TROWS, col0 = (blockIdx.x / mt) * COLS;
+  const int b_k = tid % BKI, b_j = tid / BKI;
 
-  const int tid = threadIdx.x;
-  const int tr = tid / 16, tc = tid % 16;
-  const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
-  const int a_i = tid % BM, a_k = tid / BM;    // 4 k rows per pass, 2 passes
-  const int b_k = tid % BKI, b_j = tid / BKI;  // 32 columns per pass, 2 passes
-  constexpr int QA = BKI / (NT / BM), QB = BN / (NT / BKI);
-
-  double lo[4][4], up[4][4], t1[4][4], t2[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) lo[i][j] = up[i][j] = t1[i][j] = t2[i][j] = 0.0;
-
-  double ram[QA], rap[QA], rar[QA], rbm[QB], rbr[QB];
-  auto load_tile = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      int gi = row0 + a_i, gk = k0 + a_k + (NT / BM) * q;
-      bool ok = gi < M && gk < K;
-      long o = gi + (long)gk * M;
-      ram[q] = ok ? mA[o] : 0.0;
-      rap[q] = ok ? pA[o] : 0.0;
-      rar[q] = ok ? rA[o] : 0.0;
+  double ram, rap, rar, rbm = 0.0, rbr = 0.0;
+  auto load_tile = [&](int k0) {  // by the first 256 threads
+    if (warp < 8) {
+      const int gi = row0 + lane, gk = k0 + warp;
+      const bool ok = gi < M && gk < K;
+      const long o = gi + (long)gk * M;
+      ram = ok ? mA[o] : 0.0;
+      rap = ok ? pA[o] : 0.0;
+      rar = ok ? rA[o] : 0.0;
     }
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      int hk = k0 + b_k, hj = col0 + b_j + (NT / BKI) * q;
-      bool okb = hk < K && hj < N;
-      long ob = hk + (long)hj * K;
-      rbm[q] = okb ? mB[ob] : 0.0;
-      rbr[q] = okb ? rB[ob] : 0.0;
+    if (b_j < COLS) {  // (COLS <= 32)
+      const int hk = k0 + b_k, hj = col0 + b_j;
+      const bool ok = hk < K && hj < N;
+      const long o = hk + (long)hj * K;
+      rbm = ok ? mB[o] : 0.0;
+      rbr = ok ? rB[o] : 0.0;
     }
   };
   auto store_tile = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      Am[buf][a_k + (NT / BM) * q][a_i] = ram[q];
-      Ap[buf][a_k + (NT / BM) * q][a_i] = rap[q];
-      Ar[buf][a_k + (NT / BM) * q][a_i] = rar[q];
+    auto& t = sm.st[buf];
+    if (warp < 8) {
+      t.am[warp][lane] = ram;
+      t.ap[warp][lane] = chain_factor(rap);
+      t.ar[warp][lane] = chain_factor(rar);
     }
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      Bm[buf][b_k][b_j + (NT / BKI) * q] = rbm[q];
-      Br[buf][b_k][b_j + (NT / BKI) * q] = rbr[q];
+    if (b_j < COLS) {
+      t.bm[b_k][b_j] = rbm;
+      t.br[b_k][b_j] = chain_factor(rbr);
+      t.bs[b_k][b_j] = chain_factor(oz_abs(rbm));
     }
   };
 
+  double lo[CW], up[CW];
+#pragma unroll
+  for (int j = 0; j < CW; ++j) lo[j] = up[j] = 0.0;
+  const int w0 = (warp & 3) * CW;  // the warp's first column
+  const int h = warp >= 8;               // the radius product of a chain warp
+  if (warp >= 4) {
+    for (int j = w0; j < w0 + CW; ++j) {
+      sm.c[h][j][lane] = 0;
+      sm.U[h][j][lane] = 1;
+    }
+  }
   const int nk = (K + BKI - 1) / BKI;
   load_tile(0);
   store_tile(0);
   __syncthreads();
   for (int t = 0; t < nk; ++t) {
-    const int buf = t & 1;
+    const auto& st = sm.st[t & 1];
     if (t + 1 < nk) load_tile((t + 1) * BKI);
-#pragma unroll 2
-    for (int kk = 0; kk < BKI; ++kk) {
-      double am[4], ap[4], ar[4], bm[4], br[4], bma[4];
+    if (warp < 4) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        am[i] = Am[buf][kk][tr + 16 * i];
-        ap[i] = Ap[buf][kk][tr + 16 * i];
-        ar[i] = Ar[buf][kk][tr + 16 * i];
-      }
+      for (int kk = 0; kk < BKI; ++kk) {
+        const double a = st.am[kk][lane];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        bm[j] = Bm[buf][kk][tc + 16 * j];
-        br[j] = Br[buf][kk][tc + 16 * j];
-        bma[j] = fabs(bm[j]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          lo[i][j] = __fma_rd(am[i], bm[j], lo[i][j]);
-          up[i][j] = __fma_ru(am[i], bm[j], up[i][j]);
-          t1[i][j] = __fma_ru(ap[i], br[j], t1[i][j]);
-          t2[i][j] = __fma_ru(ar[i], bma[j], t2[i][j]);
+        for (int j = 0; j < CW; ++j) {
+          const double b = st.bm[kk][w0 + j];
+          lo[j] = __fma_rd(a, b, lo[j]);
+          up[j] = __fma_ru(a, b, up[j]);
         }
+      }
+    } else {
+      // (|mA| + rA) rB or rA |mB|
+      const ChainFactor* a = (h ? &st.ar[0][0] : &st.ap[0][0]) + lane;
+      const ChainFactor(*fb)[COLS] = h ? st.bs : st.br;
+      ChainFactor fa[BKI];
+#pragma unroll
+      for (int kk = 0; kk < BKI; ++kk) fa[kk] = a[kk * TROWS];
+#pragma unroll 1
+      for (int j = w0; j < w0 + CW; ++j) {
+        DirChain x{sm.c[h][j][lane], sm.U[h][j][lane]};
+        chain_fma_n<BKI>(
+            x,
+            [&](int p, ChainFactor* u, ChainFactor* v) {
+              *u = fa[p];
+              *v = fb[p][j];
+            },
+            [&](int p, ChainFactor* u, ChainFactor* v) {
+              *u = a[p * TROWS];
+              *v = fb[p][j];
+            });
+        sm.c[h][j][lane] = x.c;
+        sm.U[h][j][lane] = x.U;
+      }
     }
-    if (t + 1 < nk) store_tile(buf ^ 1);
+    if (t + 1 < nk) store_tile((t + 1) & 1);
     __syncthreads();
   }
 
+  const int gi = row0 + lane;
+  if (warp >= 4 || gi >= M) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int gi = row0 + tr + 16 * i, gj = col0 + tc + 16 * j;
-      if (gi < M && gj < N) {
-        double T = __dadd_ru(t1[i][j], t2[i][j]);
-        double u = __dadd_ru(up[i][j], T);
-        double l = __dsub_rd(lo[i][j], T);
-        double* e = C + 2 * (gi + (long)gj * ldc);
-        e[0] = l;
-        e[1] = u;
-      }
+  for (int j = 0; j < CW; ++j) {
+    const int gj = col0 + w0 + j;
+    if (gj >= N) break;
+    const DirChain t1{sm.c[0][w0 + j][lane], sm.U[0][w0 + j][lane]},
+        t2{sm.c[1][w0 + j][lane], sm.U[1][w0 + j][lane]};
+    const double T = __dadd_ru(chain_value(t1), chain_value(t2));
+    double* e = C + 2 * (gi + (long)gj * ldc);
+    e[0] = __dsub_rd(lo[j], T);
+    e[1] = __dadd_ru(up[j], T);
+  }
+}
+
+template <int CW>
+int interval_launch(int M, int N, int K, const double* mA, const double* pA, const double* rA,
+                    const double* mB, const double* rB, double* C, long ldc, cudaStream_t s) {
+  static std::mutex mu;
+  static bool done[64] = {false};
+  int dev = 0;
+  VCPCU_CUDA_TRY(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+      VCPCU_CUDA_TRY(cudaFuncSetAttribute(interval_gemm_kernel<CW>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(ITile<CW>)));
+      if (dev >= 0 && dev < 64) done[dev] = true;
     }
+  }
+  const unsigned grid = (unsigned)((M + TROWS - 1) / TROWS) * (unsigned)((N + 4 * CW - 1) / (4 * CW));
+  interval_gemm_kernel<CW><<<grid, ITN, sizeof(ITile<CW>), s>>>(M, N, K, mA, pA, rA, mB, rB, C, ldc);
+  VCPCU_LAUNCH_CHECK("interval_gemm_kernel");
+  return VCPCU_OK;
 }
 
 // R = Y [C] with imats::mul_m_im's own loop (vcp/imats.hpp:203-213), the
@@ -530,19 +616,18 @@ int launch_point_gemm(int M, int N, int K, const double* A, long lda, const doub
     }
     return VCPCU_OK;
   }
-  dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
   switch (kind) {
     case PK_UP:
-      point_gemm_kernel<K_RU><<<grid, NT, 0, s>>>(M, N, K, A, lda, B, ldb, C0, nullptr, ldc);
+      point_launch<K_RU>(M, N, K, A, lda, B, ldb, C0, nullptr, ldc, s);
       break;
     case PK_DOWN:
-      point_gemm_kernel<K_RD><<<grid, NT, 0, s>>>(M, N, K, A, lda, B, ldb, C0, nullptr, ldc);
+      point_launch<K_RD>(M, N, K, A, lda, B, ldb, C0, nullptr, ldc, s);
       break;
     case PK_UPDOWN:
-      point_gemm_kernel<K_UD><<<grid, NT, 0, s>>>(M, N, K, A, lda, B, ldb, C0, C1, ldc);
+      point_launch<K_UD>(M, N, K, A, lda, B, ldb, C0, C1, ldc, s);
       break;
     default:
-      point_gemm_kernel<K_RN><<<grid, NT, 0, s>>>(M, N, K, A, lda, B, ldb, C0, nullptr, ldc);
+      point_launch<K_RN>(M, N, K, A, lda, B, ldb, C0, nullptr, ldc, s);
       break;
   }
   VCPCU_LAUNCH_CHECK("point_gemm_kernel");
@@ -564,10 +649,14 @@ int launch_interval_gemm_plain(int M, int N, int K, const double* A, long lda,
   VCPCU_LAUNCH_CHECK("interval_prep_left");
   interval_prep_right<<<grid_1d((long)K * N), 256, 0, s>>>(K, N, B, ldb, mB, rB);
   VCPCU_LAUNCH_CHECK("interval_prep_right");
-  dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
-  interval_gemm_kernel<<<grid, NT, 0, s>>>(M, N, K, mA, pA, rA, mB, rB, C, ldc);
-  VCPCU_LAUNCH_CHECK("interval_gemm_kernel");
-  return VCPCU_OK;
+  switch (tile_cols(M, N, 3)) {
+    case 8:
+      return interval_launch<8>(M, N, K, mA, pA, rA, mB, rB, C, ldc, s);
+    case 4:
+      return interval_launch<4>(M, N, K, mA, pA, rA, mB, rB, C, ldc, s);
+    default:
+      return interval_launch<2>(M, N, K, mA, pA, rA, mB, rB, C, ldc, s);
+  }
 }
 
 // (A k x n interval, lda) -> Aᵀ (n x k, ld = n) interval.

@@ -251,11 +251,13 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
 #pragma unroll 1
           for (int p0 = 0; p0 < TG; p0 += TB) {
 #pragma unroll
-            for (int j = 0; j < NB; ++j)
-              chain_fma_n<TB>(x[j], [&](int p, ChainFactor* u, ChainFactor* v) {
+            for (int j = 0; j < NB; ++j) {
+              auto get = [&](int p, ChainFactor* u, ChainFactor* v) {
                 *u = fa[(p0 + p) * TR];
                 *v = fb[p0 + p][j];
-              });
+              };
+              chain_fma_n<TB>(x[j], get, get);
+            }
           }
         }
       }
