@@ -13,19 +13,17 @@ namespace vcpcu {
 
 // Residues on the FP32 pipe (the integer multiply pipe is half as wide).
 // a is cut into b-bit limbs h_t, the last one signed (b = 12; b = 14 for the
-// four-limb form, which holds magnitudes <= 2^55; b = 13 for the eight-limb
-// form of the dd product, magnitudes < 2^103), exact as floats, and
+// four-limb form, which holds magnitudes <= 2^55, and the eight-limb form of
+// the dd product, magnitudes <= 2^111), exact as floats, and
 // x = sum_t h_t c_lt with c_lt = 2^(b t) mod m_l taken in [-m_l/2, m_l/2]:
-// |x| <= 128 sum_t |h_t| < 2^23 for every limb form used here (at most 16
-// twelve-bit limbs; four 14-bit limbs whose top one is <= 2^13; eight
-// 13-bit limbs whose top one is < 2^12), an exact
-// float.  The quotient q = rint(x RN(1/m)) is within 1/2 + |x / m| 2^-24 of
-// x / m (|x / m| 2^-24 m = |x| 2^-24 < 1/2; exact for m = 256), so
-// r = x - q m (one exact FMA) has |r| < m/2 + 1/2, i.e. |r| <= 128:
+// |x| <= h_0 + 128 sum_{t>0} |h_t| <= 2^14 + 128 (6 2^14 + 2^13) < 2^24 in the
+// longest form, an exact float.  The quotient q = rint(x RN(1/m)) is within
+// 1/2 + |x / m| 2^-24 of x / m (|x| 2^-24 <= 0.82; exact for m = 256), so the
+// integer r = x - q m (one exact FMA) has |r| <= m/2 + 0.82, i.e. |r| <= 128:
 // a residue of a in the range the slice GEMM's exact chunk sums allow
 // (|r_a r_b| <= 2^14 over 1024 terms), and exact in bf16.
 __host__ __device__ constexpr int oz_limb_bits(int NL) {
-  return NL == 4 ? 14 : (NL == 8 ? 13 : 12);
+  return NL == 4 || NL == 8 ? 14 : 12;
 }
 constexpr float oz_limb_c(unsigned long long m, int b, int t) {
   unsigned long long c = 1 % m;
@@ -40,18 +38,14 @@ constexpr OzPair oz_dup(float c) { return {c, c}; }
 constexpr OzPair oz_limb_cc(unsigned long long m, int b, int t) { return oz_dup(oz_limb_c(m, b, t)); }
 #define OZ_LIMB_ROW(m)                                                                     \
   {oz_limb_cc(m, 12, 0), oz_limb_cc(m, 12, 1), oz_limb_cc(m, 12, 2), oz_limb_cc(m, 12, 3), \
-   oz_limb_cc(m, 12, 4), oz_limb_cc(m, 12, 5), oz_limb_cc(m, 12, 6), oz_limb_cc(m, 12, 7), \
-   oz_limb_cc(m, 12, 8), oz_limb_cc(m, 12, 9)}
-#define OZ_LIMB14_ROW(m) \
-  {oz_limb_cc(m, 14, 0), oz_limb_cc(m, 14, 1), oz_limb_cc(m, 14, 2), oz_limb_cc(m, 14, 3)}
-#define OZ_LIMB13_ROW(m)                                                                   \
-  {oz_limb_cc(m, 13, 0), oz_limb_cc(m, 13, 1), oz_limb_cc(m, 13, 2), oz_limb_cc(m, 13, 3), \
-   oz_limb_cc(m, 13, 4), oz_limb_cc(m, 13, 5), oz_limb_cc(m, 13, 6), oz_limb_cc(m, 13, 7)}
+   oz_limb_cc(m, 12, 4), oz_limb_cc(m, 12, 5)}
+#define OZ_LIMB14_ROW(m)                                                                   \
+  {oz_limb_cc(m, 14, 0), oz_limb_cc(m, 14, 1), oz_limb_cc(m, 14, 2), oz_limb_cc(m, 14, 3), \
+   oz_limb_cc(m, 14, 4), oz_limb_cc(m, 14, 5), oz_limb_cc(m, 14, 6), oz_limb_cc(m, 14, 7)}
 #define OZ_NEGM(m) oz_dup(-(float)(m))
 #define OZ_INVF(m) oz_dup(1.0f / (float)(m))
-static __constant__ OzPair c_limb[OZ_MAX_MODULI][10] = {OZ_MOD_LIST(OZ_LIMB_ROW)};
-static __constant__ OzPair c_limb14[OZ_MAX_MODULI][4] = {OZ_MOD_LIST(OZ_LIMB14_ROW)};
-static __constant__ OzPair c_limb13[OZ_MAX_MODULI][8] = {OZ_MOD_LIST(OZ_LIMB13_ROW)};
+static __constant__ OzPair c_limb[OZ_MAX_MODULI][6] = {OZ_MOD_LIST(OZ_LIMB_ROW)};
+static __constant__ OzPair c_limb14[OZ_MAX_MODULI][8] = {OZ_MOD_LIST(OZ_LIMB14_ROW)};
 static __constant__ OzPair c_negm[OZ_MAX_MODULI] = {OZ_MOD_LIST(OZ_NEGM)};
 static __constant__ OzPair c_inv[OZ_MAX_MODULI] = {OZ_MOD_LIST(OZ_INVF)};
 __device__ __forceinline__ unsigned long long oz_pair(const OzPair& p) {
@@ -104,8 +98,7 @@ __device__ __forceinline__ uint32_t res_pair(const unsigned long long (&h)[NL], 
   unsigned long long x = h[0];
 #pragma unroll
   for (int t = 1; t < NL; ++t)
-    x = fma_x2(h[t],
-               oz_pair(NL == 4 ? c_limb14[l][t] : (NL == 8 ? c_limb13[l][t] : c_limb[l][t])), x);
+    x = fma_x2(h[t], oz_pair(oz_limb_bits(NL) == 14 ? c_limb14[l][t] : c_limb[l][t]), x);
   const unsigned long long q = sub_x2(fma_x2(x, oz_pair(c_inv[l]), magic), magic);
   const unsigned long long r = fma_x2(q, oz_pair(c_negm[l]), x);
   return __byte_perm((uint32_t)r, (uint32_t)(r >> 32), 0x7632);

@@ -1,6 +1,5 @@
 // ozaki_split.cu -- operand preparation of the slice form of the interval
-// product and of the dd product (the CRT form of the interval product:
-// ozaki_prep.cu).  Slice form: kv-style midrad of every interval entry (the
+// product (the CRT form's: ozaki_prep.cu): kv-style midrad of every interval entry (the
 // same arithmetic as the plain form and as pidblas_assist::midrad,
 // vcp/pidblas.hpp:43-51), per-row / per-column power-of-two exponents, and
 // the bf16 digit planes that the tcgen05 slice GEMM consumes.
@@ -311,34 +310,6 @@ oz_split_right(int K, int N, int Kp, int Np, const double* __restrict__ B, long 
   }
 }
 
-// Stores of a left split's plane tiles (32 rows x 64 k of bf16; lane = row,
-// warp q holds k 8q .. 8q + 7 as 16 bytes) through shared memory, so that
-// each warp writes 4 rows x 128 contiguous bytes instead of 32 separate
-// 16-byte pieces (the planes are k-contiguous, A row-contiguous).  Double
-// buffered: one barrier per tile; every thread of the block calls put() the
-// same number of times.
-struct TileStore {
-  uint4 (*T)[32][9];  // [2][32 rows][8 chunks + 1 pad]: conflict-free both ways
-  int buf;
-  __device__ __forceinline__ void put(uint4 v, uint16_t* tile, int Kp) {
-    const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-    T[buf][lane][wq] = v;
-    __syncthreads();
-    const int r = threadIdx.x >> 3, c = threadIdx.x & 7;
-    *reinterpret_cast<uint4*>(tile + (size_t)r * Kp + 8 * c) = T[buf][r][c];
-    buf ^= 1;
-  }
-};
-
-// Warp reduction of 64-bit maxima.
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
-    v = u > v ? u : v;
-  }
-  return v;
-}
 // ------------------------------------------------------------------ launchers
 template <int S, int SR>
 int launch_splits(const OzProblem& pb, const double* B, long ldb, OzWorkspace& ws,
@@ -390,198 +361,6 @@ int oz_prepare_slices(const OzProblem& pb, const double* A, long lda, const doub
       return VCPCU_ERR_INVALID_ARG;
   }
   return st_;
-}
-
-// ------------------------------------------------------------ dd (pddcuda)
-// w-bit integer of a dd value hi + lo against exponent E: the two words are
-// scaled and rounded to integers separately (|error| <= 1 unit).
-__device__ __forceinline__ __int128 dd_int(double hi, double lo, int E, int w) {
-  if (E == OZ_ZERO_EXP) return 0;
-  __int128 a = 0;
-  if (!oz_zero(hi)) a += oz_scaled_int_bits(hi, E, w, 0);
-  if (!oz_zero(lo)) a += oz_scaled_int_bits(lo, E, w, 0);
-  return a;
-}
-
-// Row maxima of |hi| of a dd matrix (kv pairs {a1, a2}, column-major).
-__global__ void __launch_bounds__(256)
-dd_rowmax(int M, int K, const double* __restrict__ A, long lda, int cols_per_block,
-          unsigned long long* __restrict__ mx, int* __restrict__ flag) {
-  __shared__ unsigned long long red[32];
-  const int lane = threadIdx.x & 31, ph = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
-  if (threadIdx.x < 32) red[lane] = 0;
-  __syncthreads();
-  unsigned long long am = 0;
-  bool bad = false;
-  if (i < M) {
-    const int c0 = blockIdx.y * cols_per_block, c1 = min(K, c0 + cols_per_block);
-    for (int c = c0 + ph; c < c1; c += 8) {
-      const double2 e = *reinterpret_cast<const double2*>(A + 2 * (i + (long)c * lda));
-      if (isfinite(e.x) && isfinite(e.y))
-        am = max(am, dbits(oz_abs(e.x)));
-      else
-        bad = true;
-    }
-  }
-  if (bad) atomicOr(flag, 1);
-  atomicMax(&red[lane], am);
-  __syncthreads();
-  if (threadIdx.x < 32 && i < M) atomicMax(&mx[i], red[lane]);
-}
-
-// Exponents of the dd form: one bit of headroom over max |hi| so that
-// |hi + lo| <= 2^(E-1).
-__global__ void dd_exponents(int R, const unsigned long long* __restrict__ mx,
-                             int* __restrict__ E) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= R) return;
-  const int e = oz_exponent(__longlong_as_double((long long)mx[i]));
-  E[i] = e == OZ_ZERO_EXP ? e : e + 1;
-}
-
-// Left dd factor -> residue planes [L][Mp][Kp].  Block: 32 rows x 64 k;
-// lane = row, warp q takes k0 + 8q .. k0 + 8q + 7 (coalesced loads across
-// the warp); the plane tiles go out through shared memory (TileStore).
-template <int NL>
-__global__ void __launch_bounds__(256)
-dd_split_left(int M, int K, int Mp, int Kp, const double* __restrict__ A, long lda, int L, int w,
-              const int* __restrict__ E, uint16_t* __restrict__ planes) {
-  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  const int i = blockIdx.y * 32 + lane;
-  const int k0 = blockIdx.x * 64 + wq * 8;
-  const int Ei = i < M ? E[i] : OZ_ZERO_EXP;
-  __int128 a[8];
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int k = k0 + t;
-    double hi = 0.0, lo = 0.0;
-    if (i < M && k < K) {
-      const double2 e = *reinterpret_cast<const double2*>(A + 2 * (i + (long)k * lda));
-      if (isfinite(e.x) && isfinite(e.y)) {
-        hi = e.x;
-        lo = e.y;
-      }
-    }
-    a[t] = dd_int(hi, lo, Ei, w);
-  }
-  __shared__ uint4 tile_smem[2][32][9];
-  TileStore ts{tile_smem, 0};
-  const size_t tile0 = (size_t)(blockIdx.y * 32) * Kp + blockIdx.x * 64;
-  const size_t pstride = (size_t)Mp * Kp;
-  unsigned long long hl[4][NL];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) limbs_pair<NL>(a[2 * t], a[2 * t + 1], hl[t]);
-#pragma unroll
-  for (int l = 0; l < OZ_MAX_MODULI; ++l) {
-    if (l >= L) break;
-    uint32_t h[4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) h[t] = res_pair<NL>(hl[t], l);
-    ts.put(make_uint4(h[0], h[1], h[2], h[3]), planes + l * pstride + tile0, Kp);
-  }
-}
-
-// Right dd factor, pass 1: one warp per column (8 per block), the column
-// maximum of |hi| (warp reduction) and its exponent; padding columns get
-// the zero exponent.
-__global__ void __launch_bounds__(256)
-dd_colmax(int K, int N, int Np, const double* __restrict__ B, long ldb, int* __restrict__ F,
-          int* __restrict__ flag) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (j >= Np) return;  // whole warps only
-  unsigned long long am = 0;
-  bool bad = false;
-  if (j < N) {
-    const double* bcol = B + 2 * (long)j * ldb;
-    for (int k = lane; k < K; k += 32) {
-      const double2 e = *reinterpret_cast<const double2*>(bcol + 2 * k);
-      if (sw_finite(e.x) && sw_finite(e.y))
-        am = max(am, dbits(oz_abs(e.x)));
-      else
-        bad = true;
-    }
-  }
-  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(flag, 1);
-  am = warp_max_u64(am);
-  int Fj = oz_exponent(__longlong_as_double((long long)am));
-  if (Fj != OZ_ZERO_EXP) Fj += 1;
-  if (lane == 0) F[j] = j < N ? Fj : OZ_ZERO_EXP;
-}
-
-// Right dd factor, pass 2 -> residue planes [L][Np][Kp].  Block: 8 columns x
-// 256 k; warp q takes column 8 bx.y + q, lane t the 8 consecutive k of
-// 256 bx.x + 8 t .. + 7 (each warp reads 4 KB of its column contiguously and
-// writes 512 contiguous bytes per plane).
-template <int NL>
-__global__ void __launch_bounds__(256)
-dd_split_right(int K, int N, int Kp, int Np, const double* __restrict__ B, long ldb, int L, int w,
-               const int* __restrict__ F, uint16_t* __restrict__ planes) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.y * 8 + (threadIdx.x >> 5);
-  const int k0 = blockIdx.x * 256 + 8 * lane;
-  if (j >= Np || k0 >= Kp) return;
-  const int Fj = F[j];
-  const double* bcol = B + 2 * (long)j * ldb;
-  __int128 b[8];
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int k = k0 + t;
-    double hi = 0.0, lo = 0.0;
-    if (j < N && k < K) {
-      const double2 e = *reinterpret_cast<const double2*>(bcol + 2 * k);
-      if (sw_finite(e.x) && sw_finite(e.y)) {
-        hi = e.x;
-        lo = e.y;
-      }
-    }
-    b[t] = dd_int(hi, lo, Fj, w);
-  }
-  unsigned long long hl[4][NL];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) limbs_pair<NL>(b[2 * t], b[2 * t + 1], hl[t]);
-  const size_t pstride = (size_t)Np * Kp, off = (size_t)j * Kp + k0;
-#pragma unroll
-  for (int l = 0; l < OZ_MAX_MODULI; ++l) {
-    if (l >= L) break;
-    uint32_t h[4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) h[t] = res_pair<NL>(hl[t], l);
-    *reinterpret_cast<uint4*>(planes + l * pstride + off) = make_uint4(h[0], h[1], h[2], h[3]);
-  }
-}
-
-int dd_prepare(int M, int N, int K, int Mp, int Np, int Kp, int L, int w, const double* A,
-               long lda, const double* B, long ldb, unsigned long long* rowmax, int* E, int* F,
-               uint16_t* planesA, uint16_t* planesB, int* flag, cudaStream_t st) {
-  VCPCU_CUDA_TRY(cudaMemsetAsync(rowmax, 0, sizeof(unsigned long long) * (size_t)Mp, st));
-  VCPCU_CUDA_TRY(cudaMemsetAsync(flag, 0, 4 * sizeof(int), st));
-  if (M > 0 && K > 0) {
-    const int cpb = 256;
-    dim3 g1((M + 31) / 32, (K + cpb - 1) / cpb);
-    dd_rowmax<<<g1, 256, 0, st>>>(M, K, A, lda, cpb, rowmax, flag);
-    VCPCU_LAUNCH_CHECK("dd_rowmax");
-  }
-  dd_exponents<<<(Mp + 255) / 256, 256, 0, st>>>(Mp, rowmax, E);
-  VCPCU_LAUNCH_CHECK("dd_exponents");
-  dim3 g2(Kp / 64, Mp / 32);
-  // |A'|, |B'| < 2^(w-1): eight 13-bit limbs up to w = 104, ten 12-bit ones
-  // up to w = 120
-  if (w <= 104)
-    dd_split_left<8><<<g2, 256, 0, st>>>(M, K, Mp, Kp, A, lda, L, w, E, planesA);
-  else
-    dd_split_left<10><<<g2, 256, 0, st>>>(M, K, Mp, Kp, A, lda, L, w, E, planesA);
-  VCPCU_LAUNCH_CHECK("dd_split_left");
-  dd_colmax<<<(Np + 7) / 8, 256, 0, st>>>(K, N, Np, B, ldb, F, flag);
-  VCPCU_LAUNCH_CHECK("dd_colmax");
-  dim3 g3((Kp + 255) / 256, Np / 8);
-  if (w <= 104)
-    dd_split_right<8><<<g3, 256, 0, st>>>(K, N, Kp, Np, B, ldb, L, w, F, planesB);
-  else
-    dd_split_right<10><<<g3, 256, 0, st>>>(K, N, Kp, Np, B, ldb, L, w, F, planesB);
-  VCPCU_LAUNCH_CHECK("dd_split_right");
-  return VCPCU_OK;
 }
 
 }  // namespace vcpcu

@@ -233,7 +233,7 @@ namespace {
 // bound, the integer warps take about half the issue slots beside it.  The
 // radius chains' states live in shared memory between batches (their code is
 // one loop over the columns).  n = 512: 64 x 64 tiles with four FP64 chains
-// 2.07 ms, this 0.66; n = 1024 14.1 and
+// 2.07 ms, this 0.66; n = 1024 8.24 and
 // 4.4 ms (3.5 at the FP64 rate).
 constexpr int ITN = 384;  // threads
 template <int CW>
