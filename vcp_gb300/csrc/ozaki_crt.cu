@@ -475,8 +475,9 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
   }
 }
 
-// One product: blockIdx.x over the column ranges of CB columns, blockIdx.y
-// over the 128-row tiles.  Block (0, 0) merges the status words.
+// One product: blocks over the column ranges of CB columns, then over the
+// 128-row tiles (one dimension: no limit on either).  Block 0 merges the
+// status words.
 template <bool LOWB>
 __global__ void __launch_bounds__(ASM_NT, 3)
 oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
@@ -489,10 +490,11 @@ oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
                        const __grid_constant__ CrtBasis cc, const __grid_constant__ OzRadConst rc) {
   __shared__ AsmTile t;
   const int f0 = flag[0], f1 = flag[1];
-  if (merge && (f0 | f1) && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+  if (merge && (f0 | f1) && blockIdx.x == 0 && threadIdx.x == 0)
     atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
-  const int i0 = blockIdx.y * ASM_ROWS, nr = min(ASM_ROWS, M - i0);
-  const int j0 = blockIdx.x * CB, nc = min(CB, N - j0);
+  const int ncb = (N + CB - 1) / CB;
+  const int i0 = (int)(blockIdx.x / ncb) * ASM_ROWS, nr = min(ASM_ROWS, M - i0);
+  const int j0 = (int)(blockIdx.x % ncb) * CB, nc = min(CB, N - j0);
   asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, eA, asum, eB, bsum);
   const AsmArgs a{M, Mp, L, w, res, plane, P, C, Cup, ldc, f0 != 0 || f1 != 0,
                   (((uintptr_t)C) & 15) == 0};
@@ -564,12 +566,7 @@ int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long l
   // (a block's row and column data are formed once), 64 at most
   int CB = ASM_COLS;
   while (CB > 8 && (long)tm * ((pb.N + CB - 1) / CB) < 608) CB >>= 1;
-  // (row tiles past the 65535 of grid.y: more than 8 million rows)
-  if (tm > 65535) {
-    set_error("reassembly: %d rows are more than it takes", pb.M);
-    return VCPCU_ERR_UNSUPPORTED;
-  }
-  const dim3 grid((pb.N + CB - 1) / CB, tm);
+  const unsigned grid = (unsigned)tm * (unsigned)((pb.N + CB - 1) / CB);
   const OzRadConst rc = oz_rad_const(plan);
   auto launch = [&](auto kernel) {
     kernel<<<grid, ASM_NT, 0, st>>>(pb.M, pb.N, pb.K, pb.Mp, pb.L, pb.w, CB, ws.res,
