@@ -8,9 +8,9 @@
 // (double-buffered TMEM accumulators, so draining overlaps the next chunk's
 // MMAs) and, per mode:
 //   OZ_CRT       group g = modulus m_g: the residue of the integer product
-//                mod m_g, one byte per entry in res[g][col][row] (one chunk:
-//                reduced on the FP32 pipe straight from TMEM; several: int32
-//                chunk sums, reduced per fold of 64 chunks);
+//                mod m_g, one byte per entry in res[g][col][row] (reduced on
+//                the FP32 pipe straight from TMEM; several chunks: the sum of
+//                their reductions, reduced again);
 //   OZ_RAD_SET / OZ_RAD_ADD  all digit pairs of one radius product form one
 //                group: every chunk is weighted by its pair's 2^(8 (t_ref - t))
 //                and summed upward in fp32, one fold per (product, tile) into
@@ -411,8 +411,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
         if (kind == OZ_CRT && nchunks == 1) {
           // residue group (one modulus) of one chunk: the residue goes
           // straight from TMEM to res on the FP32 pipe, for the valid rows
-          // and columns only (the reassembly reads no other); with several
-          // chunks the int32 accumulation below is cheaper per chunk
+          // and columns only (the reassembly reads no other)
           const int buf = acc & 1;
           const uint32_t par = (acc >> 1) & 1;
           ++acc;
@@ -468,6 +467,72 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
           if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
           continue;
         }
+        if (kind == OZ_CRT) {
+          // residue group of several chunks (one pair: the group's modulus):
+          // every chunk is reduced to |r| <= m/2 + 2 and summed on the FP32
+          // pipe, two columns per instruction; the sum is an exact integer
+          // (below 2^24 for any inner dimension under 10^8) and is reduced
+          // once more to the residue byte.  (As int32 sums -- conversions on
+          // the XU pipe, an integer remainder at the end -- the epilogue of
+          // two chunks outlasted their MMAs now and then: the product of
+          // 1225^3 took 109 us, now 88; 2048^3 288, now 279.)
+          const int ncb = (f.nb * 64 - half * 128) >> 5;  // column blocks multiplied
+          const float mf = (float)args.moduli[g];
+          const float invf = __frcp_rn(mf);
+          const unsigned long long inv2 = f32x2(invf, invf), negm2 = f32x2(-mf, -mf),
+                                   rnd2 = f32x2(12582912.0f, 12582912.0f);
+          auto reduce = [&](unsigned long long x) {
+            return fma_x2(sub_x2(add_x2(mul_x2(x, inv2), rnd2), rnd2), negm2, x);
+          };
+          unsigned long long S[64];
+#pragma unroll
+          for (int e = 0; e < 64; ++e) S[e] = 0;
+          for (int idx = 0; idx < nchunks; ++idx, ++acc) {
+            const int buf = acc & 1;
+            const uint32_t par = (acc >> 1) & 1;
+            if (*(volatile int*)&sm.abort || !ptx::mbar_wait(&sm.tfull[buf], par, lim)) {
+              if (!*(volatile int*)&sm.abort) raise_timeout(&sm, args.flag, 3);
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after();
+#pragma unroll
+            for (int c4 = 0; c4 < 4; ++c4) {
+              if (c4 < ncb) {
+                uint32_t r[32];
+                ptx::tmem_ld_32x32(tmem + lane_addr + buf * OZ_BN + half * 128 + c4 * 32, r);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                  S[c4 * 16 + e] = add_x2(
+                      S[c4 * 16 + e], reduce(f32x2(__uint_as_float(r[2 * e]),
+                                                   __uint_as_float(r[2 * e + 1]))));
+              }
+            }
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
+          }
+          if (!ok) break;
+          uint8_t* rp = f.res + (size_t)args.gres[g] * f.Np * f.Mp + (size_t)gj0 * f.Mp + gi;
+          const size_t ld = (size_t)f.Mp;
+          const int ncol = gi < f.M ? f.N - gj0 : 0;  // 0: a padding row
+          const unsigned long long off2 = f32x2(8388608.0f, 8388608.0f),
+                                   offm2 = f32x2(8388608.0f + mf, 8388608.0f + mf);
+#pragma unroll
+          for (int e = 0; e < 64; ++e) {
+            const unsigned long long rr = reduce(S[e]);
+            const unsigned long long a = add_x2(rr, off2), b = add_x2(rr, offm2);
+            const uint32_t r0 = __uint_as_float((uint32_t)rr) < 0.0f ? (uint32_t)b : (uint32_t)a;
+            const uint32_t r1 = __uint_as_float((uint32_t)(rr >> 32)) < 0.0f
+                                    ? (uint32_t)(b >> 32)
+                                    : (uint32_t)(a >> 32);
+            if (2 * e < ncol) rp[(2 * e) * ld] = (uint8_t)r0;
+            if (2 * e + 1 < ncol) rp[(2 * e + 1) * ld] = (uint8_t)r1;
+          }
+          continue;
+        }
+        // OZ_MID: the chunks of a digit group as int32 sums, folded into W
         const int t = args.pl.gt[g];
         const int sh = 8 * (args.t_ref - t);
         const int npg = args.pl.gstart[g + 1] - args.pl.gstart[g];
@@ -485,50 +550,20 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
             break;
           }
           ptx::tc_fence_after();
-          // columns past N were not multiplied
-          const int ncb = (f.nb * 64 - half * 128) >> 5;
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4) {
-            if (c4 < ncb) {
-              uint32_t r[32];
-              ptx::tmem_ld_32x32(tmem + lane_addr + buf * OZ_BN + half * 128 + c4 * 32, r);
-              ptx::tmem_ld_wait();
+            uint32_t r[32];
+            ptx::tmem_ld_32x32(tmem + lane_addr + buf * OZ_BN + half * 128 + c4 * 32, r);
+            ptx::tmem_ld_wait();
 #pragma unroll
-              for (int e = 0; e < 32; ++e) c[c4 * 32 + e] += __float2int_rn(__uint_as_float(r[e]));
-            }
+            for (int e = 0; e < 32; ++e) c[c4 * 32 + e] += __float2int_rn(__uint_as_float(r[e]));
           }
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
           ++cnt;
           const bool last_of_group = idx == total - 1;
-          if ((cnt == OZ_FOLD_CHUNKS || last_of_group) && kind == OZ_CRT) {
-            // CRT form: group g is modulus m_g; keep (A'B') mod m_g as a byte
-            // in its residue plane [col][row], adding to an earlier fold of the group
-            uint8_t* rp =
-                f.res + (size_t)args.gres[g] * f.Np * f.Mp + (size_t)gj0 * f.Mp + gi;
-            {
-              const uint32_t m = (uint32_t)args.moduli[g];
-              const uint32_t mg = 0xFFFFFFFFu / m;
-              const bool first = cnt == idx + 1;  // no earlier fold in this group
-#pragma unroll
-              for (int e = 0; e < 128; ++e) {
-                const int v = c[e];
-                const uint32_t a = (uint32_t)(v < 0 ? -v : v);
-                uint32_t r = a - __umulhi(a, mg) * m;
-                if (r >= m) r -= m;
-                if (r >= m) r -= m;
-                if (v < 0 && r) r = m - r;
-                if (!first) {
-                  r += rp[(size_t)e * f.Mp];
-                  if (r >= m) r -= m;
-                }
-                rp[(size_t)e * f.Mp] = (uint8_t)r;
-                c[e] = 0;
-              }
-            }
-            cnt = 0;
-          } else if (cnt == OZ_FOLD_CHUNKS || last_of_group) {
+          if (cnt == OZ_FOLD_CHUNKS || last_of_group) {
             // fold into W (global, column-major, ld = Mp); the first fold of
             // a tile stores, later folds add
 #pragma unroll
