@@ -27,12 +27,20 @@
 // multiplied (their columns are past N and never stored for reassembly).
 //
 // Warp roles (320 threads, one CTA per SM, persistent over tiles):
-//   warp 0      TMA producer (4-stage ring of 48 KB A+B k-blocks)
+//   warp 0      TMA producer (4-stage ring of 48 KB A+B k-blocks; pairs: 6 of 32)
 //   warp 1      TMEM owner + MMA issuer (one thread)
 //   warps 2..9  epilogue: warp w reads TMEM lanes 32*(w%4).. and columns
 //               128*((w-2)/4).. of each accumulator.
 // Every mbarrier wait is bounded; a timeout sets flag[1] and the CTA winds
 // down (waits for its copies and MMAs, frees TMEM, returns).
+//
+// CTA pairs (PAIR; use_pairs below says where): two CTAs work on a 256 x 256
+// tile with cta_group::2 MMAs.  Each still owns 128 rows of the result and its
+// epilogue, but loads only half of the B tile: 32 KB a k-block instead of 48,
+// so that the ring holds six stages in place of four, shared memory is read
+// less per MMA, and a third of the traffic from L2 goes away.  The issuer's
+// cycles per 1024-deep chunk (8192 at the tensor peak), single CTAs -> pairs:
+// 1225x1225x12544 11050 -> 9820, 4096^3 11430 -> 10830.
 #include "common.cuh"
 #include "ozaki.cuh"
 #include "ozaki_common.cuh"
@@ -50,19 +58,42 @@ constexpr int A_STAGE = OZ_BM * OZ_BK * 2;  // 16 KB
 constexpr int B_STAGE = OZ_BN * OZ_BK * 2;  // 32 KB
 constexpr int B_SUB = 64 * OZ_BK * 2;       // 8 KB: one 64-column block of B
 constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
+// A CTA of a pair: 128 rows of A, 128 of the tile's 256 columns of B
+constexpr int PAIR_STAGE_BYTES = A_STAGE + B_STAGE / 2;
+constexpr int PAIR_STAGES = 6;
+static_assert(PAIR_STAGES * PAIR_STAGE_BYTES == OZ_STAGES * STAGE_BYTES, "one ring size");
 constexpr int TMEM_COLS = 512;  // two 128 x 256 fp32 accumulators
 
+template <int STAGES>
 struct Smem {
-  uint64_t full[OZ_STAGES], empty[OZ_STAGES];
+  uint64_t full[STAGES], empty[STAGES];
   uint64_t tfull[2], tempty[2];
   uint64_t mma_done;
   uint32_t tmem_base;
   int abort;
 };
 
-__device__ __forceinline__ void raise_timeout(Smem* sm, int* flag, int where) {
+template <class S>
+__device__ __forceinline__ void raise_timeout(S* sm, int* flag, int where) {
   atomicOr(&flag[1], 1 << where);
   *(volatile int*)&sm->abort = 1;
+}
+
+// An epilogue warp hands an accumulator back to the issuer (the pair's leader);
+// the issuer's wait for it.
+template <bool PAIR>
+__device__ __forceinline__ void release_acc(uint64_t* tempty) {
+  if constexpr (PAIR)
+    ptx::mbar_arrive_cluster(ptx::leader_addr(tempty));
+  else
+    ptx::mbar_arrive(tempty);
+}
+template <bool PAIR>
+__device__ __forceinline__ bool wait_acc(uint64_t* tempty, uint32_t par, long long lim) {
+  if constexpr (PAIR)
+    return ptx::mbar_wait_cluster(tempty, par, lim);
+  else
+    return ptx::mbar_wait(tempty, par, lim);
 }
 
 __device__ __forceinline__ double scale_dir(double x, int e, bool up) {
@@ -89,13 +120,14 @@ __device__ __forceinline__ double pow2_ru(int e) {
 // group, so the CTAs resident at one time share a few A row panels and
 // B column panels (both stay in L2 across the CTAs of one group).
 constexpr int OZ_RASTER = 16;
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int per_group = OZ_RASTER * tiles_n;
+__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn,
+                                            int raster = OZ_RASTER) {
+  const int per_group = raster * tiles_n;
   const int g = tile / per_group;
-  const int rows = min(OZ_RASTER, tiles_m - g * OZ_RASTER);
+  const int rows = min(raster, tiles_m - g * raster);
   const int idx = tile - g * per_group;
   tn = idx / rows;
-  tm = g * OZ_RASTER + idx % rows;
+  tm = g * raster + idx % rows;
 }
 
 // Work items.  MID (slice form): one item per tile, all groups (the groups
@@ -126,9 +158,13 @@ __device__ __forceinline__ int gfind_item(const int* __restrict__ prefix, int np
   return lo;
 }
 
-__device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int ntiles) {
+// PAIR: ntiles and the tile index count pairs of row blocks; `rank` is this
+// CTA's block of the pair.
+template <bool PAIR>
+__device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int ntiles,
+                                              int rank) {
   ItemInfo f;
-  if (a.gp) {
+  if (!PAIR && a.gp) {
     const int p = a.gprob ? a.gprob[item] : gfind_item(a.gitem, a.gnprob, item);
     const OzGProb& q = a.gp[p];
     const int nt = q.tiles_m * q.tiles_n;
@@ -148,7 +184,7 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
     return f;
   }
   int tile = item;
-  if (a.mode == OZ_MID) {
+  if (!PAIR && a.mode == OZ_MID) {
     f.g0 = 0;
     f.g1 = a.pl.ngroups;
   } else {
@@ -156,7 +192,12 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
     f.g1 = f.g0 + 1;
     tile = item - f.g0 * ntiles;
   }
-  tile_coords(tile, a.tiles_m, a.tiles_n, f.tm, f.tn);
+  if (PAIR) {
+    tile_coords(tile, (a.tiles_m + 1) >> 1, a.tiles_n, f.tm, f.tn, OZ_RASTER / 2);
+    f.tm = 2 * f.tm + rank;  // (past the last row block: loads give zeros, all rows are padding)
+  } else {
+    tile_coords(tile, a.tiles_m, a.tiles_n, f.tm, f.tn);
+  }
   f.arow = f.tm * OZ_BM;
   f.bcol = f.tn * OZ_BN;
   f.Mp = a.Mp;
@@ -167,6 +208,17 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
   f.res = a.res;
   f.P = a.P;
   return f;
+}
+
+// The CTA's (or pair's) place among those of the grid; read where it is used,
+// so that the epilogue's registers stay free of it.
+template <bool PAIR>
+__device__ __forceinline__ int worker() {
+  return PAIR ? blockIdx.x >> 1 : blockIdx.x;
+}
+template <bool PAIR>
+__device__ __forceinline__ int nworkers() {
+  return PAIR ? gridDim.x >> 1 : gridDim.x;
 }
 
 // Residue of a one-chunk CRT group on the FP32 pipe (no float-to-int
@@ -183,42 +235,52 @@ __device__ __forceinline__ long long shift_t(int c, int sh) {
   return sh >= 0 ? (v << sh) : (v >> (-sh));
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(NTHREADS, 1)
 oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
+  constexpr int STAGES = PAIR ? PAIR_STAGES : OZ_STAGES;
+  constexpr int STAGE = PAIR ? PAIR_STAGE_BYTES : STAGE_BYTES;
   extern __shared__ uint8_t dsmem_raw[];
-  __shared__ Smem sm;
+  __shared__ Smem<STAGES> sm;
   uint8_t* dsmem = (uint8_t*)(((uintptr_t)dsmem_raw + 1023) & ~(uintptr_t)1023);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntiles = args.tiles_m * args.tiles_n;
-  const int nitems = args.gp ? args.gnitems
-                             : (args.mode == OZ_MID ? ntiles : ntiles * args.pl.ngroups);
+  const int rank = PAIR ? (int)ptx::cluster_rank() : 0;
+  const int ntiles = (PAIR ? (args.tiles_m + 1) >> 1 : args.tiles_m) * args.tiles_n;
+  const int nitems = !PAIR && args.gp
+                         ? args.gnitems
+                         : (!PAIR && args.mode == OZ_MID ? ntiles : ntiles * args.pl.ngroups);
   const int nchunks = (args.Kp + OZ_CHUNK - 1) / OZ_CHUNK;
   const int kblocks = args.Kp / OZ_BK;
   const long long lim = args.timeout_cycles;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < OZ_STAGES; ++i) {
+    for (int i = 0; i < STAGES; ++i) {
       ptx::mbar_init(&sm.full[i], 1);
       ptx::mbar_init(&sm.empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&sm.tfull[i], 1);
-      ptx::mbar_init(&sm.tempty[i], 8);
+      ptx::mbar_init(&sm.tempty[i], PAIR ? 16 : 8);  // the epilogue warps of both CTAs
     }
     ptx::mbar_init(&sm.mma_done, 1);
     sm.abort = 0;
     ptx::fence_mbar_init();
   }
   if (warp == 1) {
-    ptx::tmem_alloc(&sm.tmem_base, TMEM_COLS);
-    ptx::tmem_relinquish();
+    if constexpr (PAIR) {
+      ptx::tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(&sm.tmem_base, TMEM_COLS);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) ptx::cluster_sync();  // the peer's barriers are initialised
   ptx::tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
@@ -228,8 +290,8 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
       uint32_t phase = 0;
       bool ok = true;
       uint32_t used = 0, lastpar = 0;  // per-stage bit masks
-      for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-        const ItemInfo f = item_info(args, item, ntiles);
+      for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
+        const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
         for (int pi = args.pl.gstart[f.g0]; pi < args.pl.gstart[f.g1] && ok; ++pi) {
           const int pa = args.pl.pa[pi], pb = args.pl.pb[pi];
           for (int kb = 0; kb < kblocks; ++kb) {
@@ -238,22 +300,31 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
               ok = false;
               break;
             }
-            uint8_t* sA = dsmem + stage * STAGE_BYTES;
+            uint8_t* sA = dsmem + stage * STAGE;
             uint8_t* sB = sA + A_STAGE;
-            ptx::mbar_expect_tx(&sm.full[stage], A_STAGE + f.nb * B_SUB);
-            ptx::tma_load_3d(sA, &args.tmA, &sm.full[stage], kb * OZ_BK, f.arow, pa);
-            if (args.bsub) {
-              // 64-row boxes land back to back: the same SW128 K-major
-              // layout as one box of 64 nb rows
-              for (int i = 0; i < f.nb; ++i)
-                ptx::tma_load_3d(sB + i * B_SUB, &args.tmB, &sm.full[stage], kb * OZ_BK,
-                                 f.bcol + 64 * i, pb);
+            if constexpr (PAIR) {
+              // both CTAs' bytes count on the leader's barrier, which the
+              // issuer waits for
+              const uint32_t bar = ptx::leader_addr(&sm.full[stage]);
+              if (rank == 0) ptx::mbar_expect_tx(&sm.full[stage], 2 * PAIR_STAGE_BYTES);
+              ptx::tma_load_3d_pair(sA, &args.tmA, bar, kb * OZ_BK, f.arow, pa);
+              ptx::tma_load_3d_pair(sB, &args.tmB, bar, kb * OZ_BK, f.bcol + 128 * rank, pb);
             } else {
-              ptx::tma_load_3d(sB, &args.tmB, &sm.full[stage], kb * OZ_BK, f.bcol, pb);
+              ptx::mbar_expect_tx(&sm.full[stage], A_STAGE + f.nb * B_SUB);
+              ptx::tma_load_3d(sA, &args.tmA, &sm.full[stage], kb * OZ_BK, f.arow, pa);
+              if (args.bsub) {
+                // 64-row boxes land back to back: the same SW128 K-major
+                // layout as one box of 64 nb rows
+                for (int i = 0; i < f.nb; ++i)
+                  ptx::tma_load_3d(sB + i * B_SUB, &args.tmB, &sm.full[stage], kb * OZ_BK,
+                                   f.bcol + 64 * i, pb);
+              } else {
+                ptx::tma_load_3d(sB, &args.tmB, &sm.full[stage], kb * OZ_BK, f.bcol, pb);
+              }
             }
             used |= 1u << stage;
             lastpar = (lastpar & ~(1u << stage)) | (phase << stage);
-            if (++stage == OZ_STAGES) {
+            if (++stage == STAGES) {
               stage = 0;
               phase ^= 1;
             }
@@ -261,25 +332,30 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
         }
       }
       // every issued copy has landed before the CTA may exit (immediate in
-      // the normal case: the MMA thread consumed them all)
-      for (int i = 0; i < OZ_STAGES; ++i)
-        if (used & (1u << i)) ptx::mbar_wait(&sm.full[i], (lastpar >> i) & 1u, lim);
+      // the normal case: the MMA thread consumed them all); of a pair, the
+      // issuer's arrivals on this CTA's empty barriers too
+      for (int i = 0; i < STAGES; ++i)
+        if (used & (1u << i)) {
+          if (rank == 0) ptx::mbar_wait(&sm.full[i], (lastpar >> i) & 1u, lim);
+          if (PAIR) ptx::mbar_wait(&sm.empty[i], (lastpar >> i) & 1u, lim);
+        }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
       int stage = 0;
       uint32_t phase = 0;
       uint32_t acc = 0;  // global chunk counter
       bool ok = true;
-      for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-        const ItemInfo f = item_info(args, item, ntiles);
-        const uint32_t idesc = ptx::idesc_bf16_f32(OZ_BM, 64 * f.nb);
+      for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
+        const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
+        const uint32_t idesc =
+            PAIR ? ptx::idesc_bf16_f32(2 * OZ_BM, OZ_BN) : ptx::idesc_bf16_f32(OZ_BM, 64 * f.nb);
         for (int pi = args.pl.gstart[f.g0]; pi < args.pl.gstart[f.g1] && ok; ++pi) {
           for (int ch = 0; ch < nchunks && ok; ++ch, ++acc) {
             const int buf = acc & 1;
             const uint32_t par = (acc >> 1) & 1;
-            if (*(volatile int*)&sm.abort || !ptx::mbar_wait(&sm.tempty[buf], par ^ 1, lim)) {
+            if (*(volatile int*)&sm.abort || !wait_acc<PAIR>(&sm.tempty[buf], par ^ 1, lim)) {
               if (!*(volatile int*)&sm.abort) raise_timeout(&sm, args.flag, 1);
               ok = false;
               break;
@@ -295,28 +371,44 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
                 break;
               }
               ptx::tc_fence_after();
-              const uint32_t sA = ptx::smem_u32(dsmem + stage * STAGE_BYTES);
+              const uint32_t sA = ptx::smem_u32(dsmem + stage * STAGE);
               const uint32_t sB = sA + A_STAGE;
 #pragma unroll
               for (int kk = 0; kk < OZ_BK / 16; ++kk) {
                 const uint64_t ad = ptx::sw128_kmajor_desc(sA + kk * 32);
                 const uint64_t bd = ptx::sw128_kmajor_desc(sB + kk * 32);
-                ptx::mma_bf16(dt, ad, bd, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+                if constexpr (PAIR)
+                  ptx::mma_bf16_pair(dt, ad, bd, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+                else
+                  ptx::mma_bf16(dt, ad, bd, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
               }
-              ptx::mma_commit(&sm.empty[stage]);
-              if (++stage == OZ_STAGES) {
+              if constexpr (PAIR)
+                ptx::mma_commit_pair(&sm.empty[stage]);
+              else
+                ptx::mma_commit(&sm.empty[stage]);
+              if (++stage == STAGES) {
                 stage = 0;
                 phase ^= 1;
               }
             }
             if (!ok) break;
-            ptx::mma_commit(&sm.tfull[buf]);
+            if constexpr (PAIR)
+              ptx::mma_commit_pair(&sm.tfull[buf]);
+            else
+              ptx::mma_commit(&sm.tfull[buf]);
           }
         }
       }
-      // all MMAs of this thread done before TMEM is released
-      ptx::mma_commit(&sm.mma_done);
+      // all MMAs of this thread done before TMEM is released; of a pair, the
+      // peer's last arrivals on this CTA's barriers too
+      if constexpr (PAIR)
+        ptx::mma_commit_pair(&sm.mma_done);
+      else
+        ptx::mma_commit(&sm.mma_done);
       ptx::mbar_wait(&sm.mma_done, 0, lim);
+      if (PAIR && ok)
+        for (uint32_t a = acc > 2 ? acc - 2 : 0; a < acc; ++a)
+          wait_acc<PAIR>(&sm.tempty[a & 1], (a >> 1) & 1, lim);
     }
   } else {
     // ------------------------------------------------------------ epilogue
@@ -328,8 +420,8 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
     uint32_t acc = 0;
     bool ok = true;
     bool nonfinite = args.flag[0] != 0;
-    for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-      const ItemInfo f = item_info(args, item, ntiles);
+    for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
+      const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
       const int g0 = f.g0, g1 = f.g1;
       const int gi = f.tm * OZ_BM + row_in_tile;
       const int gj0 = f.tn * OZ_BN + half * 128;
@@ -352,7 +444,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
             ptx::tc_fence_after();
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
+            if (lane == 0) release_acc<PAIR>(&sm.tempty[buf]);
           }
         }
         continue;
@@ -395,7 +487,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
             }
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
+            if (lane == 0) release_acc<PAIR>(&sm.tempty[buf]);
             if (++pc == nchunks) {
               pc = 0;
               ++pi;
@@ -464,7 +556,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
           }
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
+          if (lane == 0) release_acc<PAIR>(&sm.tempty[buf]);
           continue;
         }
         if (kind == OZ_CRT) {
@@ -511,7 +603,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
             }
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
+            if (lane == 0) release_acc<PAIR>(&sm.tempty[buf]);
           }
           if (!ok) break;
           uint8_t* rp = f.res + (size_t)args.gres[g] * f.Np * f.Mp + (size_t)gj0 * f.Mp + gi;
@@ -560,7 +652,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
           }
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&sm.tempty[buf]);
+          if (lane == 0) release_acc<PAIR>(&sm.tempty[buf]);
           ++cnt;
           const bool last_of_group = idx == total - 1;
           if (cnt == OZ_FOLD_CHUNKS || last_of_group) {
@@ -616,9 +708,19 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
 
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) {
+    // no CTA leaves while its peer may still signal it (the issuer's last
+    // arrival on the other CTA is that on mma_done)
+    if (rank == 1 && threadIdx.x == 32) ptx::mbar_wait(&sm.mma_done, 0, lim);
+    __syncwarp();
+    ptx::cluster_sync();
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, TMEM_COLS);
+    if constexpr (PAIR)
+      ptx::tmem_dealloc_pair(tmem, TMEM_COLS);
+    else
+      ptx::tmem_dealloc(tmem, TMEM_COLS);
   }
 }
 
@@ -674,6 +776,28 @@ int num_sms() {
   return n;
 }
 
+// CTA pairs for products of several chunks that fill the device: their gain is
+// in the loads of a long inner dimension (single CTAs -> pairs, the GEMM alone:
+// 2048^3 279 -> 263 us, 4096^3 1869 -> 1800, 1225x1225x12544 649 -> 599).
+//   One chunk: within 2 % of each other, either way round (4096x4096x1024 508
+// and 512 us).  Below one item per SM the pair's start-up shows (256x256x4096
+// 97 and 102 us).  An odd last row block costs half a pair: not where that
+// adds more than a tenth of the rounds.
+//   From about 2^42 multiply-adds (4 ms) the power limit sets the clock, and
+// single CTAs do more work at it; whole products in a sustained loop, single
+// CTAs and pairs: 8192x8192x2048 4836 and 4654 us, 3000x3000x16384 5855 and
+// 5780, 6000^3 7130 and 7208, 8192^3 16598 and 17175.
+bool use_pairs(int tiles_m, int tiles_n, int Kp, const OzPairList& pl) {
+  if (tiles_m < 2 || Kp <= OZ_CHUNK) return false;
+  const long sms = num_sms(), pairs = sms / 2;
+  const long tiles = (long)tiles_m * tiles_n, items = tiles * pl.ngroups;
+  if (items < sms || pairs < 1) return false;
+  if ((double)tiles * OZ_BM * OZ_BN * Kp * pl.npairs > 0x1p42) return false;
+  const long one = (items + sms - 1) / sms;
+  const long two = ((long)((tiles_m + 1) / 2) * tiles_n * pl.ngroups + pairs - 1) / pairs;
+  return 10 * two <= 11 * one;
+}
+
 // The radius products and the residue GEMMs in one launch: the A planes are
 // [residues (mpl) | |mA| + rA digits (sr) | rA digits (sr)] at one plane
 // stride, the B planes [residues | rB digits | |mB| digits]; the groups of
@@ -724,7 +848,10 @@ static int oz_gemm_smem_optin() {
   }
   std::lock_guard<std::mutex> lk(mu);
   if (!done[dev]) {
-    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel,
+    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<false>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)oz_dyn_smem()));
+    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)oz_dyn_smem()));
     done[dev] = true;
@@ -775,10 +902,12 @@ int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, 
       a.gres[g] = (int8_t)g;
     }
   if ((st_ = make_tmap(&a.tmA, ap, pb.Kp, pb.Mp, apl, OZ_BM, ws.a_pstride))) return st_;
-  if ((st_ = make_tmap(&a.tmB, bp, pb.Kp, pb.Np, bpl, OZ_BN, ws.b_pstride))) return st_;
-  a.M = pb.M; a.N = pb.N; a.Mp = pb.Mp; a.Np = pb.Np; a.Kp = pb.Kp;
   a.tiles_m = pb.Mp / OZ_BM;
   a.tiles_n = pb.Np / OZ_BN;
+  const bool pair = !mid && use_pairs(a.tiles_m, a.tiles_n, pb.Kp, a.pl);
+  if ((st_ = make_tmap(&a.tmB, bp, pb.Kp, pb.Np, bpl, pair ? OZ_BN / 2 : OZ_BN, ws.b_pstride)))
+    return st_;
+  a.M = pb.M; a.N = pb.N; a.Mp = pb.Mp; a.Np = pb.Np; a.Kp = pb.Kp;
   a.mode = mode;
   a.t_set = t_set >= 0 ? t_set : (mode == OZ_RAD_SET ? 1 : 0);
   a.s = pb.s;
@@ -794,10 +923,28 @@ int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, 
   a.ldc = ldc;
   a.flag = ws.flag;
   a.timeout_cycles = 4000000000LL;  // about 2 s at 2 GHz
+  if (pair) {
+    const int nitems = (a.tiles_m + 1) / 2 * a.tiles_n * a.pl.ngroups;
+    const int pairs = nitems < num_sms() / 2 ? nitems : num_sms() / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = oz_dyn_smem();
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    VCPCU_CUDA_TRY(cudaLaunchKernelEx(&cfg, oz_slice_gemm_kernel<true>, a));
+    VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
+    return VCPCU_OK;
+  }
   const int ntiles = a.tiles_m * a.tiles_n;
   const int nitems = mode == OZ_MID ? ntiles : ntiles * a.pl.ngroups;
   const int grid = nitems < num_sms() ? nitems : num_sms();
-  oz_slice_gemm_kernel<<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
+  oz_slice_gemm_kernel<false><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
   VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
   return VCPCU_OK;
 }
@@ -855,7 +1002,7 @@ int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int mode, int nitems, 
   a.gnprob = b.nprob;
   a.gnitems = nitems;
   const int grid = nitems < num_sms() ? nitems : num_sms();
-  oz_slice_gemm_kernel<<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
+  oz_slice_gemm_kernel<false><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
   VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
   return VCPCU_OK;
 }
