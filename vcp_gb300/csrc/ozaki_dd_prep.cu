@@ -152,8 +152,8 @@ __host__ __device__ __forceinline__ int dd_right_lanes(int Kp) {
   return Kp <= 64 ? 8 : (Kp <= 128 ? 16 : 32);
 }
 
-// Left blocks: rows [32 rb, + 32) x 64 k, a warp 8 rows x 32 k (lane = row +
-// 8 k-group); right blocks as above.  Both end in the same dd_split8: its 32
+// Left blocks: rows [32 rb, + 32) x 64 k, a warp 8 rows x 32 k (lane =
+// k-group + 4 row, as ozaki_prep.cu); right blocks as above.  Both end in the same dd_split8: its 32
 // unrolled residues are most of the kernel's code, and two copies of it
 // overran the instruction cache (160 us against 128 at n = 2048).
 __global__ void __launch_bounds__(NT, 3) dd_split(const __grid_constant__ DdPrepArgs p) {
@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(NT, 3) dd_split(const __grid_constant__ DdPrep
   double2 v[8];
   if (left) {
     const int nrb = (s.lines + 31) >> 5;
-    line = (blockIdx.x % nrb) * 32 + (warp & 3) * 8 + (lane & 7);
-    k = (blockIdx.x / nrb) * 64 + (warp >> 2) * 32 + (lane >> 3) * 8;
+    line = (blockIdx.x % nrb) * 32 + (warp & 3) * 8 + (lane >> 2);
+    k = (blockIdx.x / nrb) * 64 + (warp >> 2) * 32 + (lane & 3) * 8;
 #pragma unroll
     for (int t = 0; t < 8; ++t)
       v[t] = line < s.lines && k + t < p.K

@@ -294,7 +294,8 @@ template <int NL, bool LEFT>
 __device__ __forceinline__ void split8(const double2 (&v)[8], const Line& ln, const PrepArgs& p,
                                        const PrepSide& s, size_t off, bool store, LineSums& sums) {
   unsigned long long h[4][NL];
-  uint32_t b1[4], b0[4], r1[4], r0[4];
+  uint32_t b1[4] = {}, b0[4] = {}, r1[4] = {}, r0[4] = {};
+  const bool digits = p.run1 | p.run2;  // (no radius product: both radii are zero)
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const Ints x = entry_ints<LEFT>(v[2 * t], ln, p.w), y = entry_ints<LEFT>(v[2 * t + 1], ln, p.w);
@@ -307,6 +308,7 @@ __device__ __forceinline__ void split8(const double2 (&v)[8], const Line& ln, co
       sums.hi += (ax >> 32) + (ay >> 32);
       sums.lo += (ax & 0xffffffffULL) + (ay & 0xffffffffULL);
     }
+    if (!digits) continue;
     int xb1, xb0, yb1, yb0, xr1, xr0, yr1, yr0;
     digits16(x.nb, xb1, xb0);
     digits16(y.nb, yb1, yb0);
@@ -367,21 +369,23 @@ __device__ __forceinline__ void add_sums(LineSums x, int lanes, int step, bool f
   if (q3) atomicAdd(&sum[3], (unsigned long long)q3);
 }
 
-// Rows [32 rb, + 32), steps of 64 k from 64 kb0: a warp takes 8 rows x 32 k
-// (lane = row + 8 k-group), so that its loads of one k are whole 128-byte
-// lines of A's columns and its stores 64 contiguous bytes of a plane's rows.
+// Rows [32 rb, + 32), steps of 64 k from 64 kb0: a warp takes 8 rows x 32 k,
+// lane = k-group + 4 row.  The eight lanes that a 16-byte store serves at a
+// time then write two lines of a plane (with rows fastest they wrote eight,
+// and the store pipe, 36 passes an instruction, was the bound: 1225x12544
+// 332 -> 301 us, n = 8192 1441 -> 1311).
 template <int NL>
 __device__ __forceinline__ void split_left(const PrepArgs& p, int rb, int kb0, int steps) {
   const PrepSide& s = p.a;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = rb * 32 + (warp & 3) * 8 + (lane & 7);
+  const int i = rb * 32 + (warp & 3) * 8 + (lane >> 2);
   const bool row = i < s.lines;
   const uint32_t* e = s.e + 3 * (size_t)i;
   const Line ln = row ? make_line(exp_dec(e[0]), exp_dec(e[1]), exp_dec(e[2]), p.w)
                       : make_line(OZ_ZERO_EXP, OZ_ZERO_EXP, OZ_ZERO_EXP, p.w);
   LineSums sums;
   for (int it = 0; it < steps; ++it) {
-    const int k = (kb0 + it) * 64 + (warp >> 2) * 32 + (lane >> 3) * 8;
+    const int k = (kb0 + it) * 64 + (warp >> 2) * 32 + (lane & 3) * 8;
     if ((kb0 + it) * 64 >= p.Kp) break;
     double2 v[8];
 #pragma unroll
@@ -390,7 +394,7 @@ __device__ __forceinline__ void split_left(const PrepArgs& p, int rb, int kb0, i
                                 : make_double2(0.0, 0.0);
     split8<NL, true>(v, ln, p, s, (size_t)(s.line0 + i) * p.Kp + k, row, sums);
   }
-  add_sums<NL, true>(sums, 4, 8, row && lane < 8, s.sum + 4 * (size_t)i);
+  add_sums<NL, true>(sums, 4, 1, row && (lane & 3) == 0, s.sum + 4 * (size_t)i);
 }
 
 // Lanes per column of the right split: as many as its padded length fills
