@@ -21,6 +21,18 @@ constexpr int OZ_MAX_GROUPS = 32;
 // Tile geometry of the slice GEMM.
 constexpr int OZ_BM = 128, OZ_BN = 256, OZ_BK = 64, OZ_STAGES = 4;
 
+// Element offset of (line, k) in an operand plane of the CRT form: tiles of
+// `lines` lines (OZ_BM of A's rows, OZ_BN of B's columns) x 64 k, each
+// contiguous ([line][64], what one box of the slice GEMM loads), the k tiles
+// of a line block one after another.  A block of the preparation then writes
+// 4 KB runs of a plane where whole K-major lines took 32 pieces of 128 bytes
+// a line apart (point factor 16384 x 16384: split 2500 -> 2362 us, and the
+// slice GEMM, which DRAM bounds there, 1436 -> 1323; 1225x1225x12544: split
+// 301 -> 280).
+OZ_HD size_t oz_tile_off(int line, int lines, int k, int Kp) {
+  return (((size_t)(line / lines) * (Kp >> 6) + (k >> 6)) * lines + line % lines) * 64 + (k & 63);
+}
+
 struct OzProblem {
   int M, N, K;     // logical sizes: C (M x N) = A (M x K) * B (K x N)
   int Mp, Np, Kp;  // padded: Mp % 128 == 0, Np % 256 == 0, Kp % 64 == 0
@@ -40,8 +52,10 @@ struct OzOperand {
 
 // Device scratch of one Ozaki-form product (pointers into one allocation).
 struct OzWorkspace {
-  uint16_t *a_mid, *a_p, *a_r;        // left digit planes  [s|sr][Mp][Kp] (bf16)
-  uint16_t *b_mid, *b_r, *b_s;        // right digit planes [s|sr][Np][Kp] (bf16)
+  // left planes [s|sr][Mp][Kp], right planes [s|sr][Np][Kp] (bf16); the CRT
+  // form's in tiles (oz_tile_off)
+  uint16_t *a_mid, *a_p, *a_r;
+  uint16_t *b_mid, *b_r, *b_s;
   int32_t* P;                         // [2 slots][Np][Mp] fp32 folds (bits) of the two radius products
   int* flag;                          // [0] non-finite input, [1] device wait timeout
   // CRT form.  zero .. zero_bytes: the words that the preparation
@@ -126,6 +140,7 @@ struct alignas(128) OzGemmArgs {
   // multiplies only the 64-column blocks that hold columns of its problem
   // (MMA N = 64, 128, 192 or 256); else one 256-row box, N = 256
   int bsub;
+  int tiled;  // the planes are stored in tiles (oz_tile_off; the CRT form's)
   OzPairList pl;
 };
 
@@ -230,7 +245,7 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, cons
 // launches).  Problems with the same padded inner dimension Kp, modulus
 // count and operand width form a bucket (cut into chunks of similar work);
 // the bucket's operand planes are stacked: the rows of problem p occupy rows
-// [rowoff, rowoff + Mp) of the A planes ([plane][Mtot][Kp]) and [coloff,
+// [rowoff, rowoff + Mp) of the A planes ([plane][Mtot][Kp], tiled) and [coloff,
 // coloff + Np) of the B planes ([plane][Ntot][Kp]); its residue bytes and
 // radius folds live at res_off / P_off of the bucket's arrays, laid out as
 // in a single product.  Every kernel of the CRT form has a grouped twin

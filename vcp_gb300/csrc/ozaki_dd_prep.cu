@@ -1,8 +1,8 @@
 // ozaki_dd_prep.cu -- operand preparation of the dd product (ozaki_dd.cu) in
 // two launches over both factors, in the manner of the interval product's
 // (ozaki_prep.cu): the exponents of the largest |a1| of every row of A and
-// column of B, then the residue planes [L][line][Kp] of the w-bit integers of
-// their entries, K-major bf16, k padded with zeros.
+// column of B, then the residue planes (oz_tile_off) of the w-bit integers of
+// their entries, bf16, k padded with zeros.
 //
 // Bound: DRAM (16 bytes read, 2 L written per entry of the split) and the FP32
 // pipe (10 paired instructions per residue and pair of entries).  n = 2048, L =
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(NT, 3) dd_split(const __grid_constant__ DdPrep
     k = k0 + (lane & (lanes - 1)) * 8;
   }
   if (line >= s.lines || k >= p.Kp) return;
-  dd_split8(v, dd_line_exp(s.e[line]), p, s, (size_t)line * p.Kp + k);
+  dd_split8(v, dd_line_exp(s.e[line]), p, s, oz_tile_off(line, left ? OZ_BM : OZ_BN, k, p.Kp));
 }
 
 inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }

@@ -164,6 +164,7 @@ template <bool PAIR>
 __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int ntiles,
                                               int rank) {
   ItemInfo f;
+  const int unit = a.tiled ? a.Kp / OZ_BK : 1;  // rows of the tensor map per line
   if (!PAIR && a.gp) {
     const int p = a.gprob ? a.gprob[item] : gfind_item(a.gitem, a.gnprob, item);
     const OzGProb& q = a.gp[p];
@@ -172,8 +173,8 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
     f.g0 = local / nt;
     f.g1 = f.g0 + 1;
     tile_coords(local - f.g0 * nt, q.tiles_m, q.tiles_n, f.tm, f.tn);
-    f.arow = q.rowoff + f.tm * OZ_BM;
-    f.bcol = q.coloff + f.tn * OZ_BN;
+    f.arow = (q.rowoff + f.tm * OZ_BM) * unit;
+    f.bcol = (q.coloff + f.tn * OZ_BN) * unit;
     f.Mp = q.Mp;
     f.Np = q.Np;
     f.M = q.m;
@@ -198,8 +199,8 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
   } else {
     tile_coords(tile, a.tiles_m, a.tiles_n, f.tm, f.tn);
   }
-  f.arow = f.tm * OZ_BM;
-  f.bcol = f.tn * OZ_BN;
+  f.arow = f.tm * OZ_BM * unit;
+  f.bcol = f.tn * OZ_BN * unit;
   f.Mp = a.Mp;
   f.Np = a.Np;
   f.M = a.M;
@@ -290,6 +291,10 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
       uint32_t phase = 0;
       bool ok = true;
       uint32_t used = 0, lastpar = 0;  // per-stage bit masks
+      // a k-block further: the next tile of the line block (tiled planes), or
+      // 64 entries along the lines
+      const int kx = args.tiled ? 0 : OZ_BK;
+      const int ka = args.tiled ? OZ_BM : 0, kbb = args.tiled ? OZ_BN : 0;
       for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
         const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
         for (int pi = args.pl.gstart[f.g0]; pi < args.pl.gstart[f.g1] && ok; ++pi) {
@@ -307,19 +312,19 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
               // issuer waits for
               const uint32_t bar = ptx::leader_addr(&sm.full[stage]);
               if (rank == 0) ptx::mbar_expect_tx(&sm.full[stage], 2 * PAIR_STAGE_BYTES);
-              ptx::tma_load_3d_pair(sA, &args.tmA, bar, kb * OZ_BK, f.arow, pa);
-              ptx::tma_load_3d_pair(sB, &args.tmB, bar, kb * OZ_BK, f.bcol + 128 * rank, pb);
+              ptx::tma_load_3d_pair(sA, &args.tmA, bar, kb * kx, f.arow + kb * ka, pa);
+              ptx::tma_load_3d_pair(sB, &args.tmB, bar, kb * kx, f.bcol + kb * kbb + 128 * rank, pb);
             } else {
               ptx::mbar_expect_tx(&sm.full[stage], A_STAGE + f.nb * B_SUB);
-              ptx::tma_load_3d(sA, &args.tmA, &sm.full[stage], kb * OZ_BK, f.arow, pa);
+              ptx::tma_load_3d(sA, &args.tmA, &sm.full[stage], kb * kx, f.arow + kb * ka, pa);
               if (args.bsub) {
                 // 64-row boxes land back to back: the same SW128 K-major
                 // layout as one box of 64 nb rows
                 for (int i = 0; i < f.nb; ++i)
-                  ptx::tma_load_3d(sB + i * B_SUB, &args.tmB, &sm.full[stage], kb * OZ_BK,
-                                   f.bcol + 64 * i, pb);
+                  ptx::tma_load_3d(sB + i * B_SUB, &args.tmB, &sm.full[stage], kb * kx,
+                                   f.bcol + kb * kbb + 64 * i, pb);
               } else {
-                ptx::tma_load_3d(sB, &args.tmB, &sm.full[stage], kb * OZ_BK, f.bcol, pb);
+                ptx::tma_load_3d(sB, &args.tmB, &sm.full[stage], kb * kx, f.bcol + kb * kbb, pb);
               }
             }
             used |= 1u << stage;
@@ -743,15 +748,19 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// Map of operand planes, read in boxes of box_rows lines x 64 k: planes of
+// whole lines (the slice form), or tiled ones (oz_tile_off: 64 entries wide,
+// a box one contiguous run).
 int make_tmap(CUtensorMap* m, const void* base, int Kp, int rows, int planes, int box_rows,
-              size_t pstride = 0) {
+              bool tiled, size_t pstride = 0) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return VCPCU_ERR_CUDA;
   }
-  cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t strides[2] = {(cuuint64_t)Kp * 2,
+  const cuuint64_t width = tiled ? OZ_BK : Kp;
+  cuuint64_t dims[3] = {width, (cuuint64_t)rows * (tiled ? Kp / OZ_BK : 1), (cuuint64_t)planes};
+  cuuint64_t strides[2] = {width * 2,
                            (cuuint64_t)(pstride ? pstride : (size_t)Kp * rows) * 2};
   cuuint32_t box[3] = {(cuuint32_t)OZ_BK, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
@@ -901,11 +910,13 @@ int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, 
       a.gkind[g] = (int8_t)mode;
       a.gres[g] = (int8_t)g;
     }
-  if ((st_ = make_tmap(&a.tmA, ap, pb.Kp, pb.Mp, apl, OZ_BM, ws.a_pstride))) return st_;
+  a.tiled = mode == OZ_ALL || mode == OZ_CRT;
+  if ((st_ = make_tmap(&a.tmA, ap, pb.Kp, pb.Mp, apl, OZ_BM, a.tiled, ws.a_pstride))) return st_;
   a.tiles_m = pb.Mp / OZ_BM;
   a.tiles_n = pb.Np / OZ_BN;
   const bool pair = !mid && use_pairs(a.tiles_m, a.tiles_n, pb.Kp, a.pl);
-  if ((st_ = make_tmap(&a.tmB, bp, pb.Kp, pb.Np, bpl, pair ? OZ_BN / 2 : OZ_BN, ws.b_pstride)))
+  if ((st_ = make_tmap(&a.tmB, bp, pb.Kp, pb.Np, bpl, pair ? OZ_BN / 2 : OZ_BN, a.tiled,
+                       ws.b_pstride)))
     return st_;
   a.M = pb.M; a.N = pb.N; a.Mp = pb.Mp; a.Np = pb.Np; a.Kp = pb.Kp;
   a.mode = mode;
@@ -983,8 +994,9 @@ int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int mode, int nitems, 
     for (int l = 0; l < b.Lmax; ++l) a.moduli[l] = OZ_MODULI[l];
   }
   int st_;
-  if ((st_ = make_tmap(&a.tmA, ap, b.Kp, b.Mtot, apl, OZ_BM))) return st_;
-  if ((st_ = make_tmap(&a.tmB, bp, b.Kp, b.Ntot, bpl, 64))) return st_;
+  a.tiled = 1;
+  if ((st_ = make_tmap(&a.tmA, ap, b.Kp, b.Mtot, apl, OZ_BM, true))) return st_;
+  if ((st_ = make_tmap(&a.tmB, bp, b.Kp, b.Ntot, bpl, 64, true))) return st_;
   a.bsub = 1;
   a.Kp = b.Kp;
   a.mode = mode;

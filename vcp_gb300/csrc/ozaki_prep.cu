@@ -9,7 +9,7 @@
 //      integer instructions and nothing is stored but the maxima: the pass
 //      reads each factor once, at memory speed.
 //   2. oz_crt_split: midrad again, and the bf16 planes that the slice GEMM
-//      consumes, K-major, plane[p][line][k]:
+//      consumes, in tiles (oz_tile_off), per line:
 //        left  (per row i):    the L residues of A' = round(mA 2^(w - Em_i));
 //                              two upward digits of P (exponent Ep_i) and of
 //                              rA (Er_i)
@@ -392,7 +392,7 @@ __device__ __forceinline__ void split_left(const PrepArgs& p, int rb, int kb0, i
     for (int t = 0; t < 8; ++t)
       v[t] = row && k + t < p.K ? load_entry(s, (size_t)i + (size_t)(k + t) * s.ld)
                                 : make_double2(0.0, 0.0);
-    split8<NL, true>(v, ln, p, s, (size_t)(s.line0 + i) * p.Kp + k, row, sums);
+    split8<NL, true>(v, ln, p, s, oz_tile_off(s.line0 + i, OZ_BM, k, p.Kp), row, sums);
   }
   add_sums<NL, true>(sums, 4, 1, row && (lane & 3) == 0, s.sum + 4 * (size_t)i);
 }
@@ -442,7 +442,8 @@ __device__ __forceinline__ void split_right(const PrepArgs& p, int cb, int kb) {
 #pragma unroll
   for (int t = 0; t < 8; ++t) v[t] = T[9 * lane + t];
   LineSums sums;
-  split8<NL, false>(v, ln, p, s, (size_t)(s.line0 + j) * p.Kp + k, col && k < p.Kp, sums);
+  split8<NL, false>(v, ln, p, s, oz_tile_off(s.line0 + j, OZ_BN, k, p.Kp), col && k < p.Kp,
+                    sums);
   add_sums<NL, false>(sums, lanes, 1, col && (lane & (lanes - 1)) == 0, s.sum + 4 * (size_t)j);
 }
 
