@@ -135,11 +135,7 @@ struct alignas(128) OzGemmArgs {
   const struct OzGProb* gp;
   const int* gitem;
   const int* gprob;  // item -> problem (one load per item)
-  int gnprob, gnitems;
-  // bsub != 0 (grouped products): tmB has 64-row boxes and a tile loads and
-  // multiplies only the 64-column blocks that hold columns of its problem
-  // (MMA N = 64, 128, 192 or 256); else one 256-row box, N = 256
-  int bsub;
+  int gnitems;
   int tiled;  // the planes are stored in tiles (oz_tile_off; the CRT form's)
   OzPairList pl;
 };
@@ -242,11 +238,12 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, cons
 
 // ---------------------------------------------------------------------------
 // Grouped CRT-form products (a batch of uneven interval products in a few
-// launches).  Problems with the same padded inner dimension Kp, modulus
-// count and operand width form a bucket (cut into chunks of similar work);
-// the bucket's operand planes are stacked: the rows of problem p occupy rows
-// [rowoff, rowoff + Mp) of the A planes ([plane][Mtot][Kp], tiled) and [coloff,
-// coloff + Np) of the B planes ([plane][Ntot][Kp]); its residue bytes and
+// launches).  Problems with the same CRT plan (modulus count, operand width,
+// radius scaling) form a bucket (cut into chunks of similar work), whatever
+// their inner dimensions: a plane of the bucket is the tiles of its problems'
+// planes (oz_tile_off with each one's own Kp) one problem after another, from
+// 64-entry row arow / brow on.  Lines are numbered through the bucket from
+// rowoff / coloff (exponents, sums); problem p's residue bytes and
 // radius folds live at res_off / P_off of the bucket's arrays, laid out as
 // in a single product.  Every kernel of the CRT form has a grouped twin
 // that finds its problem by one load from a block / item -> problem table.
@@ -258,8 +255,9 @@ struct OzGProb {
   long ldb;
   double* C;
   long ldc;
-  int Mp, Np, L, w;
-  int rowoff, coloff;          // stacked rows of the bucket's A / B planes
+  int Mp, Np, Kp, L, w;
+  int rowoff, coloff;          // its first line among the bucket's rows / columns
+  int arow, brow;              // its first 64-entry row of the bucket's A / B planes
   int tiles_m, tiles_n;
   long long res_off, P_off;    // element offsets into the bucket's res / P
   int orig;                    // index in the caller's problem table
@@ -271,24 +269,23 @@ constexpr int OZ_GMAX_SPAN = 256;  // k range of a block of its maxima pass
 
 // Device view of one bucket (all pointers device memory).
 struct OzGBucket {
-  int nprob, Kp, Lmax, Mtot, Ntot;
+  int nprob, Lmax;
+  int Arows, Brows;        // 64-entry rows of an A / B plane
   const OzGProb* probs;
   const int* blk_max;      // [nprob + 1] prefix of the blocks of the maxima pass
   const int* prob_max;     // [blocks] the problem of each
   const int* blk_split;    // [nprob + 1] prefix of the blocks of the split pass
   const int* prob_split;   // [blocks] the problem of each
-  const int* item_rad;     // [nprob + 1] prefix of radius work items (groups x tiles)
-  const int* item_crt;     // [nprob + 1] prefix of residue work items (L x tiles)
-  const int* prob_rad;     // [radius items] the problem of each item
-  const int* prob_crt;     // [residue items] the problem of each item
+  const int* item;         // [nprob + 1] prefix of work items ((radius groups + L) x tiles)
+  const int* prob_item;    // [items] the problem of each item
   const int* blk_asm;      // [nprob + 1] prefix of reassembly blocks (128 rows x OZ_GASM_COLS)
   const int* prob_asm;     // [reassembly blocks] the problem of each block
-  uint16_t* planesA;       // [Lmax + 4][Mtot][Kp]: residues, |mA|+rA digits, rA digits
-  uint16_t* planesB;       // [Lmax + 4][Ntot][Kp]: residues, rB digits, |mB| digits
-  uint32_t* eA;            // [Mtot][3] encoded exponents, as OzWorkspace::eA
-  uint32_t* eB;            // [Ntot][2]
-  unsigned long long* bsum;  // [Ntot][4] as OzWorkspace::bsum
-  unsigned long long* asum;  // [Mtot][4] as OzWorkspace::asum
+  uint16_t* planesA;       // [Lmax + 4][Arows][64]: residues, |mA|+rA digits, rA digits
+  uint16_t* planesB;       // [Lmax + 4][Brows][64]: residues, rB digits, |mB| digits
+  uint32_t* eA;            // [rows][3] encoded exponents, as OzWorkspace::eA
+  uint32_t* eB;            // [columns][2]
+  unsigned long long* bsum;  // [columns][4] as OzWorkspace::bsum
+  unsigned long long* asum;  // [rows][4] as OzWorkspace::asum
   uint8_t* res;
   int32_t* P;
   int* flag;               // [nprob][4]: non-finite input, wait timeout
@@ -301,8 +298,7 @@ struct OzGBucket {
 int oz_gprep(const OzGBucket& b, int nblk_max, int nblk_split, int wmax, cudaStream_t st);
 // Blocks of one problem in the two passes; sets q's left counts.
 void oz_gprep_blocks(int m, int n, int k, int Kp, OzGProb* q, int* max_blocks, int* split_blocks);
-int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int mode, int nitems,
-                 cudaStream_t st);
+int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int nitems, cudaStream_t st);
 // shape: the bucket's plan (every problem of a bucket has the same CRT basis)
 int oz_gassemble(const OzGBucket& b, const OzPlan& shape, const OzRadConst& rc, int nblk,
                  cudaStream_t st);

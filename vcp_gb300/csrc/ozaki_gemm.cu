@@ -140,52 +140,44 @@ struct ItemInfo {
   int arow, bcol;   // TMA row of the A tile / of the B tile in the planes
   int tm, tn, g0, g1;
   int nb;           // 64-column blocks of B the tile multiplies (1..4)
+  int kblocks;      // k-blocks of its problem
   int Mp, Np;       // output layout of this item's problem
   int M, N;         // its valid rows / columns
   uint8_t* res;
   int32_t* P;
 };
 
-__device__ __forceinline__ int gfind_item(const int* __restrict__ prefix, int nprob, int x) {
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (prefix[mid] <= x)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
-}
-
 // PAIR: ntiles and the tile index count pairs of row blocks; `rank` is this
 // CTA's block of the pair.
-template <bool PAIR>
+template <bool PAIR, bool GROUP>
 __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int ntiles,
                                               int rank) {
   ItemInfo f;
-  const int unit = a.tiled ? a.Kp / OZ_BK : 1;  // rows of the tensor map per line
-  if (!PAIR && a.gp) {
-    const int p = a.gprob ? a.gprob[item] : gfind_item(a.gitem, a.gnprob, item);
+  f.kblocks = a.Kp / OZ_BK;
+  if constexpr (GROUP) {
+    const int p = a.gprob[item];
     const OzGProb& q = a.gp[p];
+    f.kblocks = q.Kp / OZ_BK;
     const int nt = q.tiles_m * q.tiles_n;
     const int local = item - a.gitem[p];
     f.g0 = local / nt;
     f.g1 = f.g0 + 1;
     tile_coords(local - f.g0 * nt, q.tiles_m, q.tiles_n, f.tm, f.tn);
-    f.arow = (q.rowoff + f.tm * OZ_BM) * unit;
-    f.bcol = (q.coloff + f.tn * OZ_BN) * unit;
+    f.arow = q.arow + f.tm * OZ_BM * f.kblocks;
+    f.bcol = q.brow + f.tn * OZ_BN * f.kblocks;
     f.Mp = q.Mp;
     f.Np = q.Np;
     f.M = q.m;
     f.N = q.n;
-    f.nb = a.bsub ? min(4, (f.N - f.tn * OZ_BN + 63) >> 6) : 4;
+    // only the 64-column blocks that hold columns of the problem are loaded and
+    // multiplied (tmB has 64-row boxes; MMA N = 64 .. 256)
+    f.nb = min(4, (f.N - f.tn * OZ_BN + 63) >> 6);
     f.res = a.res ? a.res + q.res_off : nullptr;
     f.P = a.P ? a.P + q.P_off : nullptr;
     return f;
   }
   int tile = item;
-  if (!PAIR && a.mode == OZ_MID) {
+  if (!PAIR && !GROUP && a.mode == OZ_MID) {
     f.g0 = 0;
     f.g1 = a.pl.ngroups;
   } else {
@@ -199,6 +191,7 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
   } else {
     tile_coords(tile, a.tiles_m, a.tiles_n, f.tm, f.tn);
   }
+  const int unit = a.tiled ? f.kblocks : 1;  // rows of the tensor map per line
   f.arow = f.tm * OZ_BM * unit;
   f.bcol = f.tn * OZ_BN * unit;
   f.Mp = a.Mp;
@@ -209,6 +202,10 @@ __device__ __forceinline__ ItemInfo item_info(const OzGemmArgs& a, int item, int
   f.res = a.res;
   f.P = a.P;
   return f;
+}
+
+__device__ __forceinline__ int chunks_of(int kblocks) {
+  return (kblocks + OZ_CHUNK / OZ_BK - 1) / (OZ_CHUNK / OZ_BK);
 }
 
 // The CTA's (or pair's) place among those of the grid; read where it is used,
@@ -236,7 +233,8 @@ __device__ __forceinline__ long long shift_t(int c, int sh) {
   return sh >= 0 ? (v << sh) : (v >> (-sh));
 }
 
-template <bool PAIR>
+// GROUP: the products of a batch bucket (never pairs).
+template <bool PAIR, bool GROUP>
 __global__ void __launch_bounds__(NTHREADS, 1)
 oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
   constexpr int STAGES = PAIR ? PAIR_STAGES : OZ_STAGES;
@@ -248,11 +246,8 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = PAIR ? (int)ptx::cluster_rank() : 0;
   const int ntiles = (PAIR ? (args.tiles_m + 1) >> 1 : args.tiles_m) * args.tiles_n;
-  const int nitems = !PAIR && args.gp
-                         ? args.gnitems
-                         : (!PAIR && args.mode == OZ_MID ? ntiles : ntiles * args.pl.ngroups);
-  const int nchunks = (args.Kp + OZ_CHUNK - 1) / OZ_CHUNK;
-  const int kblocks = args.Kp / OZ_BK;
+  const bool mid = !PAIR && !GROUP && args.mode == OZ_MID;
+  const int nitems = GROUP ? args.gnitems : (mid ? ntiles : ntiles * args.pl.ngroups);
   const long long lim = args.timeout_cycles;
 
   if (threadIdx.x == 0) {
@@ -296,10 +291,10 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
       const int kx = args.tiled ? 0 : OZ_BK;
       const int ka = args.tiled ? OZ_BM : 0, kbb = args.tiled ? OZ_BN : 0;
       for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
-        const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
+        const ItemInfo f = item_info<PAIR, GROUP>(args, item, ntiles, rank);
         for (int pi = args.pl.gstart[f.g0]; pi < args.pl.gstart[f.g1] && ok; ++pi) {
           const int pa = args.pl.pa[pi], pb = args.pl.pb[pi];
-          for (int kb = 0; kb < kblocks; ++kb) {
+          for (int kb = 0; kb < f.kblocks; ++kb) {
             if (*(volatile int*)&sm.abort || !ptx::mbar_wait(&sm.empty[stage], phase ^ 1, lim)) {
               if (!*(volatile int*)&sm.abort) raise_timeout(&sm, args.flag, 0);
               ok = false;
@@ -317,7 +312,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
             } else {
               ptx::mbar_expect_tx(&sm.full[stage], A_STAGE + f.nb * B_SUB);
               ptx::tma_load_3d(sA, &args.tmA, &sm.full[stage], kb * kx, f.arow + kb * ka, pa);
-              if (args.bsub) {
+              if constexpr (GROUP) {
                 // 64-row boxes land back to back: the same SW128 K-major
                 // layout as one box of 64 nb rows
                 for (int i = 0; i < f.nb; ++i)
@@ -353,7 +348,8 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
       uint32_t acc = 0;  // global chunk counter
       bool ok = true;
       for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
-        const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
+        const ItemInfo f = item_info<PAIR, GROUP>(args, item, ntiles, rank);
+        const int nchunks = chunks_of(f.kblocks);
         const uint32_t idesc =
             PAIR ? ptx::idesc_bf16_f32(2 * OZ_BM, OZ_BN) : ptx::idesc_bf16_f32(OZ_BM, 64 * f.nb);
         for (int pi = args.pl.gstart[f.g0]; pi < args.pl.gstart[f.g1] && ok; ++pi) {
@@ -368,7 +364,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
             ptx::tc_fence_after();
             const uint32_t dt = tmem + buf * OZ_BN;
             const int kb0 = ch * (OZ_CHUNK / OZ_BK);
-            const int kb1 = min(kblocks, kb0 + OZ_CHUNK / OZ_BK);
+            const int kb1 = min(f.kblocks, kb0 + OZ_CHUNK / OZ_BK);
             for (int kb = kb0; kb < kb1; ++kb) {
               if (*(volatile int*)&sm.abort || !ptx::mbar_wait(&sm.full[stage], phase, lim)) {
                 if (!*(volatile int*)&sm.abort) raise_timeout(&sm, args.flag, 2);
@@ -426,11 +422,12 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
     bool ok = true;
     bool nonfinite = args.flag[0] != 0;
     for (int item = worker<PAIR>(); item < nitems && ok; item += nworkers<PAIR>()) {
-      const ItemInfo f = item_info<PAIR>(args, item, ntiles, rank);
+      const ItemInfo f = item_info<PAIR, GROUP>(args, item, ntiles, rank);
       const int g0 = f.g0, g1 = f.g1;
+      const int nchunks = chunks_of(f.kblocks);
       const int gi = f.tm * OZ_BM + row_in_tile;
       const int gj0 = f.tn * OZ_BN + half * 128;
-      if (args.mode != OZ_MID && f.tm * OZ_BM + quarter * 32 >= f.M) {
+      if (!mid && f.tm * OZ_BM + quarter * 32 >= f.M) {
         // this warp's 32 rows are all past M (padding of the tile): release
         // each accumulator of the item unread -- the reassembly reads no
         // padding row (midpoint folds keep every row)
@@ -629,6 +626,7 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
           }
           continue;
         }
+        if constexpr (PAIR || GROUP) continue;  // (no other kinds there)
         // OZ_MID: the chunks of a digit group as int32 sums, folded into W
         const int t = args.pl.gt[g];
         const int sh = 8 * (args.t_ref - t);
@@ -676,7 +674,8 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
         }
       }
       if (!ok) break;
-      if (args.mode != OZ_MID) continue;  // CRT residues / radius folds: combined later
+      if constexpr (PAIR || GROUP) continue;
+      if (!mid) continue;  // CRT residues / radius folds: combined later
       // ------------------------------------------------------ final epilogue
       const int Ei = (gi < args.M) ? args.Erow[(size_t)args.erow_stride * gi] : OZ_ZERO_EXP;
       double dlt = 0.0;
@@ -857,10 +856,13 @@ static int oz_gemm_smem_optin() {
   }
   std::lock_guard<std::mutex> lk(mu);
   if (!done[dev]) {
-    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<false>,
+    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<false, false>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)oz_dyn_smem()));
-    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<true>,
+    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<true, false>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)oz_dyn_smem()));
+    VCPCU_CUDA_TRY(cudaFuncSetAttribute(oz_slice_gemm_kernel<false, true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)oz_dyn_smem()));
     done[dev] = true;
@@ -948,73 +950,45 @@ int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, 
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    VCPCU_CUDA_TRY(cudaLaunchKernelEx(&cfg, oz_slice_gemm_kernel<true>, a));
+    VCPCU_CUDA_TRY(cudaLaunchKernelEx(&cfg, oz_slice_gemm_kernel<true, false>, a));
     VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
     return VCPCU_OK;
   }
   const int ntiles = a.tiles_m * a.tiles_n;
   const int nitems = mode == OZ_MID ? ntiles : ntiles * a.pl.ngroups;
   const int grid = nitems < num_sms() ? nitems : num_sms();
-  oz_slice_gemm_kernel<false><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
+  oz_slice_gemm_kernel<false, false><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
   VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
   return VCPCU_OK;
 }
 
-// One launch of the slice GEMM over all problems of a bucket: radius product
-// 1 (OZ_RAD_SET), 2 (OZ_RAD_ADD) or the residue GEMMs (OZ_CRT).  `shape`
-// supplies the pair lists (radius digit pairs, Lmax moduli), the fold count
-// and the padded inner dimension shared by the bucket.
-int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int mode, int nitems, cudaStream_t st) {
+// One launch of the slice GEMM over all problems of a bucket: the radius
+// products and the residue GEMMs.  `shape` supplies the pair lists (radius
+// digit pairs, Lmax moduli) and the fold count.
+int oz_grun_gemm(const OzGBucket& b, const OzPlan& shape, int nitems, cudaStream_t st) {
   if (nitems <= 0) return VCPCU_OK;
   if (int e = oz_gemm_smem_optin()) return e;
   OzGemmArgs a;
   memset(&a, 0, sizeof(a));
-  const size_t psA = (size_t)b.Mtot * b.Kp, psB = (size_t)b.Ntot * b.Kp;
-  const uint16_t* ap;
-  const uint16_t* bp;
-  int apl, bpl;
-  if (mode == OZ_RAD_SET) {  // (|mA| + rA) * rB
-    ap = b.planesA + (size_t)b.Lmax * psA;
-    bp = b.planesB + (size_t)b.Lmax * psB;
-    apl = bpl = 2;
-    a.pl = shape.rad;
-    a.t_ref = shape.t_ref_rad;
-  } else if (mode == OZ_RAD_ADD) {  // rA * |mB|
-    ap = b.planesA + (size_t)(b.Lmax + 2) * psA;
-    bp = b.planesB + (size_t)(b.Lmax + 2) * psB;
-    apl = bpl = 2;
-    a.pl = shape.rad;
-    a.t_ref = shape.t_ref_rad;
-  } else {
-    ap = b.planesA;
-    bp = b.planesB;
-    apl = bpl = b.Lmax;
-    a.pl = shape.crt;
-    a.res = b.res;
-    for (int l = 0; l < b.Lmax; ++l) a.moduli[l] = OZ_MODULI[l];
-  }
-  int st_;
+  a.t_ref = shape.t_ref_rad;
+  a.res = b.res;
+  all_groups(shape.rad, shape.crt, b.Lmax, 2, 0, a);
   a.tiled = 1;
-  if ((st_ = make_tmap(&a.tmA, ap, b.Kp, b.Mtot, apl, OZ_BM, true))) return st_;
-  if ((st_ = make_tmap(&a.tmB, bp, b.Kp, b.Ntot, bpl, 64, true))) return st_;
-  a.bsub = 1;
-  a.Kp = b.Kp;
-  a.mode = mode;
+  int st_;
+  if ((st_ = make_tmap(&a.tmA, b.planesA, OZ_BK, b.Arows, b.Lmax + 4, OZ_BM, true))) return st_;
+  if ((st_ = make_tmap(&a.tmB, b.planesB, OZ_BK, b.Brows, b.Lmax + 4, 64, true))) return st_;
+  a.Kp = OZ_BK;  // (each item has its problem's)
+  a.mode = OZ_ALL;
   a.P = b.P;
   a.slot_add = shape.rad_slots;
-  for (int g = 0; g < a.pl.ngroups; ++g) {
-    a.gkind[g] = (int8_t)mode;
-    a.gres[g] = (int8_t)g;
-  }
   a.flag = b.flag;  // problem 0's status words take the (global) timeout bit
   a.timeout_cycles = 4000000000LL;  // about 2 s at 2 GHz
   a.gp = b.probs;
-  a.gitem = mode == OZ_CRT ? b.item_crt : b.item_rad;
-  a.gprob = mode == OZ_CRT ? b.prob_crt : b.prob_rad;
-  a.gnprob = b.nprob;
+  a.gitem = b.item;
+  a.gprob = b.prob_item;
   a.gnitems = nitems;
   const int grid = nitems < num_sms() ? nitems : num_sms();
-  oz_slice_gemm_kernel<false><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
+  oz_slice_gemm_kernel<false, true><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
   VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
   return VCPCU_OK;
 }

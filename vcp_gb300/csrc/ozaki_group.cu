@@ -2,16 +2,20 @@
 // of a batch of uneven products, vcpcu_igemm_batched_dev / the batch
 // graphs).
 //
-// The problems of a batch are bucketed by their padded inner dimension Kp,
-// modulus count L and operand width w (one CRT plan per bucket), and each
+// The problems of a batch are bucketed by modulus count L, operand width w
+// and radius scaling (one CRT plan per bucket, any inner dimensions), and each
 // bucket is cut into chunks of about 0.4 ms of estimated work, so that a
 // problem's latency -- the length of its chunk -- stays short.  A chunk runs
-// in a fixed number of launches whatever its size: row maxima, exponents,
-// left and right splits, the two radius slice GEMMs, the residue slice GEMM,
-// the reassembly and the status merge -- each a grouped twin of the
-// single-product kernel that finds its problem through a prefix array of
-// blocks or work items, or one load from an item -> problem table (the slice
-// GEMM's work items are the (problem, group, tile) triples of the chunk).
+// in four launches whatever its size: maxima, splits, slice GEMM (the radius
+// products and the residue GEMMs) and reassembly -- each a grouped twin of
+// the single-product kernel that finds its problem by one load from a block
+// or item -> problem table (the slice GEMM's work items are the (problem,
+// group, tile) triples of the chunk).
+//   (One bucket per padded inner dimension and a launch each for the radius
+// products and the residues made 17 chunks of 7 launches of 256 products of
+// 32 .. 1024, each launch with a tail of its own: 2103 us, now 1733; 40
+// products of 32 .. 300: 212 us, now 89.  Chunks of 0.2 and 1.6 ms: 1830 and
+// 1685 us.)
 // The results are bit for bit those of one vcpcu_igemm_dev call per problem:
 // the same plan (w, L, moduli, digit pairs, folds) and the same arithmetic
 // per entry.  Chunks run one after another on the stream and share one
@@ -39,7 +43,7 @@ struct BucketHost {
   OzGBucket dev;  // table pointers set at plan time, workspace pointers at record time
   OzPlan shape;   // radius pair list, Lmax-modulus pair list, fold count
   OzRadConst rc;
-  int nblk_max = 0, nblk_split = 0, nitem_rad = 0, nitem_crt = 0, nblk_asm = 0;
+  int nblk_max = 0, nblk_split = 0, nitem = 0, nblk_asm = 0;
   int wmax = 0;  // largest operand width w of the bucket's problems
   // workspace layout (byte offsets; the first zero_bytes are cleared per run)
   size_t offEA = 0, offEB = 0, offAsum = 0, offBsum = 0, offFlag = 0, zero_bytes = 0;
@@ -79,15 +83,16 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
                   int persistent, cudaStream_t s, OzGroupPlan** out) {
   *out = nullptr;
   const int nslices = slices > 0 ? slices : 8;
-  // bucket the selected problems by (Kp, L, w, radius pairs): the problems
-  // of a bucket share one CRT plan (moduli, basis, digit pairs, folds)
-  std::map<std::tuple<int, int, int, int>, std::vector<int>> byKey;
+  // bucket the selected problems by (L, w, radius pairs and scaling): the
+  // problems of a bucket share one CRT plan (moduli, basis, digit pairs, folds)
+  std::map<std::tuple<int, int, int, int, int>, std::vector<int>> byKey;
   std::vector<OzPlan> plans(count);
   for (int i = 0; i < count; ++i) {
     const BatchProblemView& q = problems[i];
     if ((select && !select[i]) || q.m <= 0 || q.n <= 0 || q.k <= 0) continue;
     oz_make_plan(q.m, q.n, q.k, nslices, 2, &plans[i], 1);
-    byKey[std::make_tuple(plans[i].pb.Kp, plans[i].pb.L, plans[i].pb.w, plans[i].rad.npairs)]
+    byKey[std::make_tuple(plans[i].pb.L, plans[i].pb.w, plans[i].rad.npairs, plans[i].t_ref_rad,
+                          plans[i].R_rad)]
         .push_back(i);
   }
   // A bucket runs its kernels one after another, so a problem's latency is
@@ -123,23 +128,27 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     host.resize(off + bytes);
     return off;
   };
-  struct Offs { size_t probs, bmax, bspl, irad, icrt, basm, pmax, pspl, prad, pcrt, pasm; };
+  struct Offs { size_t probs, bmax, bspl, item, basm, pmax, pspl, pitem, pasm; };
   std::vector<Offs> toff;
-  for (const std::vector<int>& ids : chunks) {
+  for (std::vector<int>& ids : chunks) {
+    // longest inner dimensions first: the launches end on short work items
+    std::stable_sort(ids.begin(), ids.end(),
+                     [&](int x, int y) { return plans[x].pb.Kp > plans[y].pb.Kp; });
     const int n = (int)ids.size();
     BucketHost b;
     memset(&b.dev, 0, sizeof(b.dev));
     const OzPlan& p0 = plans[ids[0]];
-    const int Kp = p0.pb.Kp;
     b.shape = p0;
     b.dev.nprob = n;
-    b.dev.Kp = Kp;
     int Lmax = 0;
-    long long Mtot = 0, Ntot = 0;
+    long long Mtot = 0, Ntot = 0, Arows = 0, Brows = 0;
     for (int id : ids) {
-      Lmax = std::max(Lmax, plans[id].pb.L);
-      Mtot += plans[id].pb.Mp;
-      Ntot += plans[id].pb.Np;
+      const OzProblem& pb = plans[id].pb;
+      Lmax = std::max(Lmax, pb.L);
+      Mtot += pb.Mp;
+      Ntot += pb.Np;
+      Arows += (long long)pb.Mp * (pb.Kp / OZ_BK);
+      Brows += (long long)pb.Np * (pb.Kp / OZ_BK);
     }
     // every modulus a group of its own, Lmax of them (a problem uses its first L)
     OzPairList& crt = b.shape.crt;
@@ -158,11 +167,10 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     o.probs = reserve(sizeof(OzGProb) * n);
     o.bmax = reserve(sizeof(int) * (n + 1));
     o.bspl = reserve(sizeof(int) * (n + 1));
-    o.irad = reserve(sizeof(int) * (n + 1));
-    o.icrt = reserve(sizeof(int) * (n + 1));
+    o.item = reserve(sizeof(int) * (n + 1));
     o.basm = reserve(sizeof(int) * (n + 1));
-    long long bmax = 0, bspl = 0, irad = 0, icrt = 0, basm = 0, res = 0, P = 0;
-    int rowoff = 0, coloff = 0;
+    long long bmax = 0, bspl = 0, nitem = 0, basm = 0, res = 0, P = 0;
+    long long rowoff = 0, coloff = 0, arow = 0, brow = 0;
     for (int t = 0; t < n; ++t) {
       const int id = ids[t];
       const BatchProblemView& q = problems[id];
@@ -180,38 +188,40 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       gp.ldc = q.ldc;
       gp.Mp = pl.pb.Mp;
       gp.Np = pl.pb.Np;
+      gp.Kp = pl.pb.Kp;
       gp.L = pl.pb.L;
       gp.w = pl.pb.w;
       b.wmax = std::max(b.wmax, gp.w);
-      gp.rowoff = rowoff;
-      gp.coloff = coloff;
+      gp.rowoff = (int)rowoff;  // (ranges checked below)
+      gp.coloff = (int)coloff;
+      gp.arow = (int)arow;
+      gp.brow = (int)brow;
       gp.tiles_m = pl.pb.Mp / OZ_BM;
       gp.tiles_n = pl.pb.Np / OZ_BN;
       gp.res_off = res;
       gp.P_off = P;
       gp.orig = id;
       int nmax, nspl;
-      oz_gprep_blocks(q.m, q.n, q.k, Kp, &gp, &nmax, &nspl);
+      oz_gprep_blocks(q.m, q.n, q.k, gp.Kp, &gp, &nmax, &nspl);
       memcpy(host.data() + o.probs + sizeof(OzGProb) * t, &gp, sizeof(gp));
       int* v;
       v = (int*)(host.data() + o.bmax); v[t] = (int)bmax;
       v = (int*)(host.data() + o.bspl); v[t] = (int)bspl;
-      v = (int*)(host.data() + o.irad); v[t] = (int)irad;
-      v = (int*)(host.data() + o.icrt); v[t] = (int)icrt;
+      v = (int*)(host.data() + o.item); v[t] = (int)nitem;
       v = (int*)(host.data() + o.basm); v[t] = (int)basm;
       const long long tiles = (long long)gp.tiles_m * gp.tiles_n;
       bmax += nmax;
       bspl += nspl;
-      irad += b.shape.rad.ngroups * tiles;
-      icrt += gp.L * tiles;
+      nitem += (2 * b.shape.rad.ngroups + gp.L) * tiles;
       basm += (long long)((q.m + 127) / 128) * ((q.n + OZ_GASM_COLS - 1) / OZ_GASM_COLS);
       res += (long long)gp.L * gp.Np * gp.Mp;
       P += 2LL * b.shape.rad_slots * gp.Np * gp.Mp;
       rowoff += gp.Mp;
       coloff += gp.Np;
+      arow += (long long)gp.Mp * (gp.Kp / OZ_BK);
+      brow += (long long)gp.Np * (gp.Kp / OZ_BK);
     }
-    if (std::max({bmax, bspl, irad, icrt, basm}) >= INT_MAX || Mtot >= INT_MAX ||
-        Ntot >= INT_MAX) {
+    if (std::max({bmax, bspl, nitem, basm, Mtot, Ntot, Arows, Brows}) >= INT_MAX) {
       delete g;
       set_error("igemm_batched: the tensor-core batch is too large for one group");
       return VCPCU_ERR_INVALID_ARG;
@@ -219,19 +229,16 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     int* v;
     v = (int*)(host.data() + o.bmax); v[n] = (int)bmax;
     v = (int*)(host.data() + o.bspl); v[n] = (int)bspl;
-    v = (int*)(host.data() + o.irad); v[n] = (int)irad;
-    v = (int*)(host.data() + o.icrt); v[n] = (int)icrt;
+    v = (int*)(host.data() + o.item); v[n] = (int)nitem;
     v = (int*)(host.data() + o.basm); v[n] = (int)basm;
     b.nblk_max = (int)bmax;
     b.nblk_split = (int)bspl;
-    b.nitem_rad = (int)irad;
-    b.nitem_crt = (int)icrt;
+    b.nitem = (int)nitem;
     // block / item -> problem maps (one load instead of a binary search over
     // the prefixes above)
     o.pmax = reserve(sizeof(int) * (size_t)(bmax > 0 ? bmax : 1));
     o.pspl = reserve(sizeof(int) * (size_t)(bspl > 0 ? bspl : 1));
-    o.prad = reserve(sizeof(int) * (size_t)(irad > 0 ? irad : 1));
-    o.pcrt = reserve(sizeof(int) * (size_t)(icrt > 0 ? icrt : 1));
+    o.pitem = reserve(sizeof(int) * (size_t)(nitem > 0 ? nitem : 1));
     o.pasm = reserve(sizeof(int) * (size_t)(basm > 0 ? basm : 1));
     {
       auto spread = [&](size_t prefix, size_t map) {
@@ -242,13 +249,12 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
       };
       spread(o.bmax, o.pmax);
       spread(o.bspl, o.pspl);
-      spread(o.irad, o.prad);
-      spread(o.icrt, o.pcrt);
+      spread(o.item, o.pitem);
       spread(o.basm, o.pasm);
     }
     b.nblk_asm = (int)basm;
-    b.dev.Mtot = (int)Mtot;
-    b.dev.Ntot = (int)Ntot;
+    b.dev.Arows = (int)Arows;
+    b.dev.Brows = (int)Brows;
     // workspace layout
     size_t w = 0;
     auto take = [&](size_t bytes) {
@@ -262,8 +268,8 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     b.offBsum = take(sizeof(unsigned long long) * 4 * Ntot);
     b.offFlag = take(sizeof(int) * 4 * (size_t)n);
     b.zero_bytes = w;
-    b.offA = take(sizeof(uint16_t) * (size_t)(Lmax + 4) * Mtot * Kp);
-    b.offB = take(sizeof(uint16_t) * (size_t)(Lmax + 4) * Ntot * Kp);
+    b.offA = take(sizeof(uint16_t) * (size_t)(Lmax + 4) * Arows * OZ_BK);
+    b.offB = take(sizeof(uint16_t) * (size_t)(Lmax + 4) * Brows * OZ_BK);
     b.offRes = take((size_t)res);
     b.offP = take(sizeof(int32_t) * (size_t)P);
     b.ws_bytes = w;
@@ -305,10 +311,8 @@ int oz_group_plan(int count, const BatchProblemView* problems, const char* selec
     d.prob_max = (const int*)(tb + o.pmax);
     d.blk_split = (const int*)(tb + o.bspl);
     d.prob_split = (const int*)(tb + o.pspl);
-    d.item_rad = (const int*)(tb + o.irad);
-    d.item_crt = (const int*)(tb + o.icrt);
-    d.prob_rad = (const int*)(tb + o.prad);
-    d.prob_crt = (const int*)(tb + o.pcrt);
+    d.item = (const int*)(tb + o.item);
+    d.prob_item = (const int*)(tb + o.pitem);
     d.blk_asm = (const int*)(tb + o.basm);
     d.prob_asm = (const int*)(tb + o.pasm);
   }
@@ -340,16 +344,8 @@ int record_chunk(const BucketHost& b, uint8_t* ws, unsigned long long* t_first,
     if ((st = oz_gprep(d, b.nblk_max, b.nblk_split, b.wmax, s))) return st;
   }
   {
-    PhaseTimer t(1, s);
-    if ((st = oz_grun_gemm(d, b.shape, OZ_RAD_SET, b.nitem_rad, s))) return st;
-  }
-  {
-    PhaseTimer t(2, s);
-    if ((st = oz_grun_gemm(d, b.shape, OZ_RAD_ADD, b.nitem_rad, s))) return st;
-  }
-  {
-    PhaseTimer t(3, s);
-    if ((st = oz_grun_gemm(d, b.shape, OZ_CRT, b.nitem_crt, s))) return st;
+    PhaseTimer t(3, s);  // the radius products and the residue GEMMs
+    if ((st = oz_grun_gemm(d, b.shape, b.nitem, s))) return st;
   }
   {
     PhaseTimer t(4, s);  // the reassembly also merges the chunk's status words

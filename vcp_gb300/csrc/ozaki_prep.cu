@@ -466,18 +466,18 @@ __global__ void __launch_bounds__(NT, 3) oz_crt_split(const __grid_constant__ Pr
 
 // ------------------------------------------------------ grouped products
 // The problems of a bucket: block -> problem by a table, its PrepArgs from its
-// descriptor (rows rowoff.., columns coloff.. of the stacked planes).
+// descriptor.
 __device__ __forceinline__ PrepArgs group_args(const OzGBucket& b, const OzGProb& q, int p) {
   PrepArgs a;
-  const size_t psA = (size_t)b.Mtot * b.Kp, psB = (size_t)b.Ntot * b.Kp;
-  a.a = PrepSide{q.A, q.lda, 0, q.m, q.rowoff, psA, b.planesA, b.planesA + b.Lmax * psA,
-                 b.planesA + (b.Lmax + 2) * psA, b.eA + 3 * (size_t)q.rowoff,
-                 b.asum + 4 * (size_t)q.rowoff};
-  a.b = PrepSide{q.B, q.ldb, 0, q.n, q.coloff, psB, b.planesB, b.planesB + b.Lmax * psB,
-                 b.planesB + (b.Lmax + 2) * psB, b.eB + 2 * (size_t)q.coloff,
-                 b.bsum + 4 * (size_t)q.coloff};
+  const size_t psA = (size_t)b.Arows * 64, psB = (size_t)b.Brows * 64;
+  uint16_t* pA = b.planesA + (size_t)q.arow * 64;
+  uint16_t* pB = b.planesB + (size_t)q.brow * 64;
+  a.a = PrepSide{q.A, q.lda, 0, q.m, 0, psA, pA, pA + b.Lmax * psA, pA + (b.Lmax + 2) * psA,
+                 b.eA + 3 * (size_t)q.rowoff, b.asum + 4 * (size_t)q.rowoff};
+  a.b = PrepSide{q.B, q.ldb, 0, q.n, 0, psB, pB, pB + b.Lmax * psB, pB + (b.Lmax + 2) * psB,
+                 b.eB + 2 * (size_t)q.coloff, b.bsum + 4 * (size_t)q.coloff};
   a.K = q.k;
-  a.Kp = b.Kp;
+  a.Kp = q.Kp;
   a.L = q.L;
   a.w = q.w;
   a.run1 = a.run2 = 1;
