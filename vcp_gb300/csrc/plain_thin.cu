@@ -18,8 +18,9 @@
 // passes: interval x point vector 658 -> 290 us, point x interval vector
 // 361 -> 247, |E| x vector 867 -> 251, norm 311 -> 128; at n = 1225 the norm
 // and the interval sums of |X| 230 -> 47 us (three passes before).  The FP64
-// chains alone are 131 us at n = 4096 (64 cycles a step): the integer chain
-// warps, about 120 cycles a step, are the bound.
+// chains alone are 131 us at n = 4096 (64 cycles a step), an integer chain
+// warp takes about 120 cycles a step; with an SM to itself a block therefore
+// runs all four chains in FP64 (thin_launch_as).
 #include "common.cuh"
 #include "dirchain.cuh"
 #include "ozaki_prep.cuh"
@@ -27,6 +28,7 @@
 #include "swfp.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace vcpcu {
 
@@ -132,32 +134,40 @@ __device__ __forceinline__ double2 entry_abs(double2 e) {
 //   0  the round-down midpoint chain, negated into a round-up one
 //      (RD(a b + c) = -RU((-a) b + (-c)), signed zeros included)
 //   1  the round-up midpoint chain
-//   2  RU((|mA| +ru rA) rB)       (integer chain)
-//   3  RU(rA |mB|)                (integer chain)
+//   2  RU((|mA| +ru rA) rB)       (integer chain, F = ChainFactor, or FP64,
+//   3  RU(rA |mB|)                 F = double: thin_launch says where)
 // and T = 2 +ru 3, C = [1st -rd T, 2nd +ru T] as pidblas::mulmm combines them;
 // four producer warps.  A step past K multiplies zeros and leaves every chain
 // unchanged.
-template <int NB>
+template <int NB, class F>
 struct ThinStage {
   double m[TG * TR];
-  ChainFactor f[2][TG * TR];  // P, r
+  F f[2][TG * TR];  // P, r
   double bm[TG][NB];
-  ChainFactor fb[2][TG][NB];  // rB, |mB|
+  F fb[2][TG][NB];  // rB, |mB|
 };
-template <int NB>
+template <int NB, class F>
 struct ThinSmem {
   double2 ring[TSTAGES][TG * TR];
-  ThinStage<NB> st[2];
+  ThinStage<NB, F> st[2];
   double T[2][TR][NB + 1];
 };
 
-template <int NB, int LEFT>
+template <class F>
+__device__ __forceinline__ F thin_factor(double x) {
+  if constexpr (std::is_same_v<F, double>)
+    return x;
+  else
+    return chain_factor(x);
+}
+
+template <int NB, int LEFT, class F>
 __global__ void __launch_bounds__(256)
 interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, long lda,
                           const double* __restrict__ mB, const double* __restrict__ rB,
                           double* __restrict__ C, long ldc) {
   extern __shared__ __align__(16) uint8_t thin_smem[];
-  ThinSmem<NB>& sm = *reinterpret_cast<ThinSmem<NB>*>(thin_smem);
+  ThinSmem<NB, F>& sm = *reinterpret_cast<ThinSmem<NB, F>*>(thin_smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i0 = blockIdx.x * TR, i = i0 + lane, j0 = blockIdx.y * NB;
   const int ng = (K + TG - 1) / TG;
@@ -190,14 +200,14 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
     for (int g = 0; g <= ng; ++g) {
       if (g < ng) {
         cp_wait<TSTAGES - 2>();
-        ThinStage<NB>& st = sm.st[g & 1];
+        ThinStage<NB, F>& st = sm.st[g & 1];
 #pragma unroll
         for (int q = 0; q < QB; ++q) {
           const int x = t + PT * q;
           if (x < TG * NB) {
             st.bm[x % TG][x / TG] = bm[q];
-            st.fb[0][x % TG][x / TG] = chain_factor(br[q]);
-            st.fb[1][x % TG][x / TG] = chain_factor(oz_abs(bm[q]));
+            st.fb[0][x % TG][x / TG] = thin_factor<F>(br[q]);
+            st.fb[1][x % TG][x / TG] = thin_factor<F>(oz_abs(bm[q]));
           }
         }
         load_b(g + 1);
@@ -218,8 +228,8 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
             v = entry_mid(e);
           }
           st.m[x] = v.m;
-          st.f[0][x] = chain_factor(v.P);
-          st.f[1][x] = chain_factor(v.r);
+          st.f[0][x] = thin_factor<F>(v.P);
+          st.f[1][x] = thin_factor<F>(v.r);
         }
         issue(g + TSTAGES - 1);  // (into the slot of stage g - 1, this thread's own)
       }
@@ -228,7 +238,8 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
   } else {
     // FP64 chains of blocks that share an SM on different sub-partitions
     const int role = (warp + 2 * ((blockIdx.x / 152) & 1)) & 3;
-    double c[NB];    // roles 0, 1
+    constexpr bool fp64 = std::is_same_v<F, double>;
+    double c[NB];    // roles 0, 1; FP64 chains of roles 2, 3
     DirChain x[NB];  // roles 2, 3
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
@@ -237,8 +248,18 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
     }
     for (int g = 0; g <= ng; ++g) {
       if (g > 0) {
-        const ThinStage<NB>& st = sm.st[(g - 1) & 1];
-        if (role < 2) {
+        const ThinStage<NB, F>& st = sm.st[(g - 1) & 1];
+        if constexpr (fp64) {
+          const double* fa = (role < 2 ? st.m : st.f[role - 2]) + lane;
+          const double(*fb)[NB] = role < 2 ? st.bm : st.fb[role - 2];
+          const uint64_t neg = role == 0 ? 1ULL << 63 : 0ULL;
+#pragma unroll
+          for (int p = 0; p < TG; ++p) {
+            const double a = sw_double(sw_bits(fa[p * TR]) ^ neg);
+#pragma unroll
+            for (int j = 0; j < NB; ++j) c[j] = __fma_ru(a, fb[p][j], c[j]);
+          }
+        } else if (role < 2) {
 #pragma unroll
           for (int p = 0; p < TG; ++p) {
             const double m = st.m[p * TR + lane], a = role == 0 ? sw_neg(m) : m;
@@ -265,7 +286,7 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
     }
     if (role >= 2) {
 #pragma unroll
-      for (int j = 0; j < NB; ++j) sm.T[role - 2][lane][j] = chain_value(x[j]);
+      for (int j = 0; j < NB; ++j) sm.T[role - 2][lane][j] = fp64 ? c[j] : chain_value(x[j]);
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");  // the four chain warps
     if (role < 2 && i < M) {
@@ -409,15 +430,35 @@ int smem_optin(size_t bytes) {
   return VCPCU_OK;
 }
 
+// All four chains go through the FP64 pipe where the blocks do not outnumber
+// the SMs: each chain warp then has a sub-partition, and its pipe, to itself
+// (64 cycles a step, against about 120 of an integer chain alone on its own).
+// With two blocks an SM the integer chains of one fill the other's pipes.
+// n = 4096, integer -> FP64 radius chains: interval x point vector 285 -> 224
+// us, point x interval vector 243 -> 208, |E| x vector 247 -> 221.  (That is
+// about 105 cycles a step.  Bare chains on all four sub-partitions take 76
+// with operands in registers and 82 with loads from shared memory; twice the
+// producer warps, or a stage's operands loaded ahead of its first step, left
+// the time as it is.)
+template <int NB, int LEFT, class F>
+int thin_launch_as(int M, int N, int K, const double* A, long lda, const double* mB,
+                const double* rB, double* C, long ldc, cudaStream_t s) {
+  constexpr size_t bytes = sizeof(ThinSmem<NB, F>);
+  if (int e = smem_optin<interval_gemm_thin_kernel<NB, LEFT, F>>(bytes)) return e;
+  const dim3 grid((M + TR - 1) / TR, (N + NB - 1) / NB);
+  interval_gemm_thin_kernel<NB, LEFT, F>
+      <<<grid, 256, bytes, s>>>(M, N, K, A, lda, mB, rB, C, ldc);
+  VCPCU_LAUNCH_CHECK("interval_gemm_thin_kernel");
+  return VCPCU_OK;
+}
+
 template <int NB, int LEFT>
 int thin_launch(int M, int N, int K, const double* A, long lda, const double* mB,
                 const double* rB, double* C, long ldc, cudaStream_t s) {
-  constexpr size_t bytes = sizeof(ThinSmem<NB>);
-  if (int e = smem_optin<interval_gemm_thin_kernel<NB, LEFT>>(bytes)) return e;
-  const dim3 grid((M + TR - 1) / TR, (N + NB - 1) / NB);
-  interval_gemm_thin_kernel<NB, LEFT><<<grid, 256, bytes, s>>>(M, N, K, A, lda, mB, rB, C, ldc);
-  VCPCU_LAUNCH_CHECK("interval_gemm_thin_kernel");
-  return VCPCU_OK;
+  const long blocks = (long)((M + TR - 1) / TR) * ((N + NB - 1) / NB);
+  if (blocks <= 152)
+    return thin_launch_as<NB, LEFT, double>(M, N, K, A, lda, mB, rB, C, ldc, s);
+  return thin_launch_as<NB, LEFT, ChainFactor>(M, N, K, A, lda, mB, rB, C, ldc, s);
 }
 
 template <int NB>
