@@ -52,6 +52,51 @@ struct Scratch {
   ~Scratch();
 };
 
+// Chains of kernels: with `chained` the kernel may start while its
+// predecessor on the stream, a kernel of the same call that ends its own
+// prologue with dep_ready(), still runs, and begins with dep_wait(), which
+// returns when that one has completed and its writes are visible (every kernel
+// of a chain waits, so all earlier ones have completed too).  Takes the launch
+// latency out of the gap between two kernels: the product 61 x 48 x 97 34.8 ->
+// 28.9 us, the eigenvalue verification at n = 1225 897 -> 873 us.  Not
+// for the chunks of a batch: on their two streams the waiting blocks hold
+// places that the other stream's kernels would take (1743 -> 1874 us).
+// Without `chained`, an ordinary launch (and dep_wait() returns at once).
+#ifdef __CUDACC__
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_ready() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class T>
+struct SameType {
+  using type = T;
+};
+template <class... P>
+cudaError_t launch_dep(bool chained, int cluster, void (*kernel)(P...), dim3 grid, dim3 block,
+                       size_t smem, cudaStream_t s, typename SameType<P>::type... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  unsigned n = 0;
+  if (chained) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = (unsigned)cluster;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#endif
+
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 }  // namespace vcpcu

@@ -330,7 +330,7 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, cons
     // CRT form: the radius products and the residue GEMMs in one launch
     // (phase 3 times all of them)
     PhaseTimer t(3, s);
-    if ((st = oz_run_gemm(plan, OZ_ALL, ws, nullptr, 0, s))) return st;
+    if ((st = oz_run_gemm(plan, OZ_ALL, ws, nullptr, 0, s, -1, true))) return st;
   } else {
     if (!(plan.point_mask & 2)) {
       PhaseTimer t(1, s);
@@ -346,7 +346,7 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, cons
   }
   if (plan.pb.crt) {
     PhaseTimer t(4, s);
-    if ((st = oz_crt_assemble(plan, ws, C, ldc, s, true, Cup))) return st;
+    if ((st = oz_crt_assemble(plan, ws, C, ldc, s, true, Cup, true))) return st;
   } else {
     oz_merge_status(ws.flag, s);
     VCPCU_LAUNCH_CHECK("oz_status_merge");

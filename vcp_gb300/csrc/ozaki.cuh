@@ -178,7 +178,8 @@ int oz_radius_T(const OzPlan& plan, const OzWorkspace& ws, cudaStream_t st);
 int oz_make_plan(int M, int N, int K, int s, int sr, OzPlan* plan, int crt = 0);
 // merge_status: the kernel also merges ws.flag into the sticky status.
 int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long ldc,
-                    cudaStream_t st, bool merge_status, double* Cup = nullptr);
+                    cudaStream_t st, bool merge_status, double* Cup = nullptr,
+                    bool chained = false);
 // Operand planes of the CRT form (ozaki_prep.cu): both factors of a product
 // whose radius products point_mask leaves out (OzPlan::point_mask), or, after
 // oz_prepare_begin, the rows [i0, i0 + rows) of the left one (i0 a multiple of
@@ -193,10 +194,11 @@ int oz_prepare_right_cols(const OzProblem& pb, const OzOperand& B, int j0, int c
 // Operand planes of the slice form (ozaki_split.cu).
 int oz_prepare_slices(const OzProblem& pb, const double* A, long lda, const double* B, long ldb,
                       OzWorkspace& ws, cudaStream_t st);
+// chained: the preparation precedes it on st (launch_dep).
 // t_set < 0: the radius product of OZ_RAD_SET writes T, that of OZ_RAD_ADD
 // adds to it; 0 / 1 force add / write.
 int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, long ldc,
-                cudaStream_t st, int t_set = -1);
+                cudaStream_t st, int t_set = -1, bool chained = false);
 size_t oz_workspace_bytes(const OzProblem& pb);
 int oz_carve_workspace(const OzProblem& pb, void* base, OzWorkspace* ws);
 

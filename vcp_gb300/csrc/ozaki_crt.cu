@@ -489,6 +489,7 @@ oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
                        const int* __restrict__ flag, int merge,
                        const __grid_constant__ CrtBasis cc, const __grid_constant__ OzRadConst rc) {
   __shared__ AsmTile t;
+  dep_wait();
   const int f0 = flag[0], f1 = flag[1];
   if (merge && (f0 | f1) && blockIdx.x == 0 && threadIdx.x == 0)
     atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
@@ -558,7 +559,7 @@ int oz_take_status(cudaStream_t s, int* status) {
 }
 
 int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long ldc,
-                    cudaStream_t st, bool merge_status, double* Cup) {
+                    cudaStream_t st, bool merge_status, double* Cup, bool chained) {
   const OzProblem& pb = plan.pb;
   if (pb.M <= 0 || pb.N <= 0) return VCPCU_OK;
   const int tm = (pb.M + ASM_ROWS - 1) / ASM_ROWS;
@@ -568,15 +569,11 @@ int oz_crt_assemble(const OzPlan& plan, const OzWorkspace& ws, double* C, long l
   while (CB > 8 && (long)tm * ((pb.N + CB - 1) / CB) < 608) CB >>= 1;
   const unsigned grid = (unsigned)tm * (unsigned)((pb.N + CB - 1) / CB);
   const OzRadConst rc = oz_rad_const(plan);
-  auto launch = [&](auto kernel) {
-    kernel<<<grid, ASM_NT, 0, st>>>(pb.M, pb.N, pb.K, pb.Mp, pb.L, pb.w, CB, ws.res,
-                                    (size_t)pb.Np * pb.Mp, ws.eA, ws.eB, ws.asum, ws.bsum, ws.P,
-                                    C, Cup, ldc, ws.flag, merge_status ? 1 : 0, plan.basis, rc);
-  };
-  if (rc.lowb)
-    launch(oz_crt_assemble_kernel<true>);
-  else
-    launch(oz_crt_assemble_kernel<false>);
+  const auto kernel = rc.lowb ? oz_crt_assemble_kernel<true> : oz_crt_assemble_kernel<false>;
+  VCPCU_CUDA_TRY(launch_dep(chained, 1, kernel, dim3(grid), dim3(ASM_NT), 0, st, pb.M, pb.N, pb.K,
+                            pb.Mp, pb.L, pb.w, CB, ws.res, (size_t)pb.Np * pb.Mp, ws.eA, ws.eB,
+                            ws.asum, ws.bsum, ws.P, C, Cup, ldc, ws.flag, merge_status ? 1 : 0,
+                            plan.basis, rc));
   VCPCU_LAUNCH_CHECK("oz_crt_assemble_kernel");
   return VCPCU_OK;
 }

@@ -181,6 +181,7 @@ dd_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, const uint8_t*
                        const uint32_t* __restrict__ eB, double* __restrict__ C, long ldc,
                        double* __restrict__ Cerr, long lde, const int* __restrict__ flag,
                        const __grid_constant__ DdBasis cc) {
+  dep_wait();
   const bool bad = flag[0] != 0 || flag[1] != 0;
   const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= M) return;
@@ -343,16 +344,16 @@ int ozaki_ddgemm(int m, int n, int k, const double* A, long lda, const double* B
   }
   {
     PhaseTimer t(3, s);
-    if ((st = oz_run_gemm(plan, OZ_CRT, ws, nullptr, 0, s))) return st;
+    if ((st = oz_run_gemm(plan, OZ_CRT, ws, nullptr, 0, s, -1, true))) return st;
   }
   oz_profile_add_flops(2LL * m * n * (long long)(k > 0 ? k : 0) * L);
   {
     PhaseTimer t(4, s);
     const int gx = (m + 511) / 512;
     const int gy = n < 65535 ? n : 65535;
-    dd_crt_assemble_kernel<<<dim3(gx, gy), 128, 0, s>>>(m, n, k, pb.Mp, L, w, ws.res,
-                                                        (size_t)pb.Np * pb.Mp, eA, eB, C, ldc,
-                                                        Cerr, lde, ws.flag, cc);
+    VCPCU_CUDA_TRY(launch_dep(true, 1, dd_crt_assemble_kernel, dim3(gx, gy), dim3(128), 0, s, m, n,
+                              k, pb.Mp, L, w, ws.res, (size_t)pb.Np * pb.Mp, eA, eB, C, ldc, Cerr,
+                              lde, ws.flag, cc));
     VCPCU_LAUNCH_CHECK("dd_crt_assemble_kernel");
   }
   oz_merge_status(ws.flag, s);

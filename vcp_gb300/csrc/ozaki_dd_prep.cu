@@ -105,6 +105,7 @@ __device__ __forceinline__ void dd_max_right(const DdSide& s, int k0, int k1, in
 }
 
 __global__ void __launch_bounds__(NT) dd_maxima(const __grid_constant__ DdPrepArgs p) {
+  dep_ready();
   int local = blockIdx.x;
   if (local < p.nA) {
     const int nrb = (p.a.lines + 31) >> 5;
@@ -158,6 +159,8 @@ __host__ __device__ __forceinline__ int dd_right_lanes(int Kp) {
 // overran the instruction cache (160 us against 128 at n = 2048).
 __global__ void __launch_bounds__(NT, 3) dd_split(const __grid_constant__ DdPrepArgs p) {
   __shared__ double2 turn[NT / 32][288];
+  dep_wait();
+  dep_ready();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool left = (int)blockIdx.x < p.nA;
   const DdSide& s = left ? p.a : p.b;
@@ -229,7 +232,8 @@ int dd_prepare(int M, int N, int K, int Mp, int Np, int Kp, int L, int w, const 
   }
   p.nA = nrb * cdiv(Kp, 64);
   const int lanes = dd_right_lanes(Kp);
-  dd_split<<<p.nA + cdiv(N, 8 * (32 / lanes)) * cdiv(Kp, 8 * lanes), NT, 0, st>>>(p);
+  const int blocks = p.nA + cdiv(N, 8 * (32 / lanes)) * cdiv(Kp, 8 * lanes);
+  VCPCU_CUDA_TRY(launch_dep(K > 0, 1, dd_split, dim3(blocks), dim3(NT), 0, st, p));
   VCPCU_LAUNCH_CHECK("dd_split");
   return VCPCU_OK;
 }

@@ -277,6 +277,10 @@ oz_slice_gemm_kernel(const __grid_constant__ OzGemmArgs args) {
   if constexpr (PAIR) ptx::cluster_sync();  // the peer's barriers are initialised
   ptx::tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
+  if constexpr (!GROUP) {
+    dep_wait();  // the planes are there
+    dep_ready();
+  }
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
@@ -871,7 +875,7 @@ static int oz_gemm_smem_optin() {
 }
 
 int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, long ldc,
-                cudaStream_t st, int t_set) {
+                cudaStream_t st, int t_set, bool chained) {
   const OzProblem& pb = plan.pb;
   if (int e = oz_gemm_smem_optin()) return e;
   OzGemmArgs a;
@@ -939,25 +943,16 @@ int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, 
   if (pair) {
     const int nitems = (a.tiles_m + 1) / 2 * a.tiles_n * a.pl.ngroups;
     const int pairs = nitems < num_sms() / 2 ? nitems : num_sms() / 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = oz_dyn_smem();
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    VCPCU_CUDA_TRY(cudaLaunchKernelEx(&cfg, oz_slice_gemm_kernel<true, false>, a));
+    VCPCU_CUDA_TRY(launch_dep(chained, 2, oz_slice_gemm_kernel<true, false>, dim3(2 * pairs),
+                              dim3(NTHREADS), oz_dyn_smem(), st, a));
     VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
     return VCPCU_OK;
   }
   const int ntiles = a.tiles_m * a.tiles_n;
   const int nitems = mode == OZ_MID ? ntiles : ntiles * a.pl.ngroups;
   const int grid = nitems < num_sms() ? nitems : num_sms();
-  oz_slice_gemm_kernel<false, false><<<grid, NTHREADS, oz_dyn_smem(), st>>>(a);
+  VCPCU_CUDA_TRY(launch_dep(chained, 1, oz_slice_gemm_kernel<false, false>, dim3(grid),
+                            dim3(NTHREADS), oz_dyn_smem(), st, a));
   VCPCU_LAUNCH_CHECK("oz_slice_gemm_kernel");
   return VCPCU_OK;
 }

@@ -239,6 +239,7 @@ __device__ __forceinline__ void maxima_block(const PrepArgs& p, int local) {
 }
 
 __global__ void __launch_bounds__(NT) oz_crt_maxima(const __grid_constant__ PrepArgs p) {
+  dep_ready();
   maxima_block(p, blockIdx.x);
 }
 
@@ -503,6 +504,8 @@ __device__ __forceinline__ void split_block(const PrepArgs& p, int local) {
 
 template <int NL>
 __global__ void __launch_bounds__(NT, 3) oz_crt_split(const __grid_constant__ PrepArgs p) {
+  dep_wait();
+  dep_ready();
   split_block<NL>(p, blockIdx.x);
 }
 
@@ -557,6 +560,7 @@ inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 // Launches both passes over the factors of p (either may have no lines).
 int prepare(PrepArgs& p, cudaStream_t st) {
+  bool after_maxima = false;  // a kernel of this call precedes the split
   const int nrb = cdiv(p.a.lines, 32), ncb = cdiv(p.b.lines, 8);
   if (p.K > 0) {
     // k range of a block: about eight blocks for each of the 152 SMs, so that
@@ -573,6 +577,7 @@ int prepare(PrepArgs& p, cudaStream_t st) {
     if (blocks > 0) {
       oz_crt_maxima<<<(unsigned)blocks, NT, 0, st>>>(p);
       VCPCU_LAUNCH_CHECK("oz_crt_maxima");
+      after_maxima = true;
     }
   }
   // 64-k steps of a left block: four (fewer additions to the row sums) where
@@ -584,12 +589,8 @@ int prepare(PrepArgs& p, cudaStream_t st) {
   if (blocks <= 0) return VCPCU_OK;
   // |A'|, |B'| <= 2^(w-1): four 14-bit limbs up to w = 56, five 12-bit limbs
   // up to w = 61, six up to 73
-  if (p.w <= 56)
-    oz_crt_split<4><<<(unsigned)blocks, NT, 0, st>>>(p);
-  else if (p.w <= 61)
-    oz_crt_split<5><<<(unsigned)blocks, NT, 0, st>>>(p);
-  else
-    oz_crt_split<6><<<(unsigned)blocks, NT, 0, st>>>(p);
+  const auto split = p.w <= 56 ? oz_crt_split<4> : (p.w <= 61 ? oz_crt_split<5> : oz_crt_split<6>);
+  VCPCU_CUDA_TRY(launch_dep(after_maxima, 1, split, dim3((unsigned)blocks), dim3(NT), 0, st, p));
   VCPCU_LAUNCH_CHECK("oz_crt_split");
   return VCPCU_OK;
 }
