@@ -464,11 +464,12 @@ def run_ours(args, ws, rank, local):
     pk, pk_kind = peaks()
     if form == pidcuda.FORM_PLAIN:
         fp64_peak, fp64_kind = measure_fp64_peak(dev)
-        achieved = 8.0 * n ** 3 / (ms * 1e-3) / 1e12
+        achieved = 4.0 * n ** 3 / (ms * 1e-3) / 1e12
         roof = {"bound": "fp64", "kernel": "interval_gemm_kernel", "achieved": achieved,
                 "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
                 "traffic": None, "peak_kind": fp64_kind,
-                "algorithmic": "8 n^3 FP64 flops per launch (4 directed FMA chains)"}
+                "algorithmic": "4 n^3 FP64 flops per launch (2 directed FMA chains; the two "
+                               "radius chains run on the integer pipe)"}
     else:
         roof = ozaki_roofline(phases, tc_flops, args.steps, pk, pk_kind, n,
                               slices == 8 | pidcuda.SLICES_FAST_RADIUS)
@@ -551,8 +552,8 @@ def measure_fp64_peak(dev):
 # n = 8192 product at 8 slices with the fast radius products (2 x 3 radius
 # digit pairs and 16 residue GEMMs in one launch), from a one-pass ncu
 # capture of dram__bytes_read.sum and dram__bytes_write.sum on a GB300
-# (21.30 + 2.06 GB).
-GEMM_TRAFFIC_N8192 = 23.36e9
+# (21.62 + 1.82 GB).
+GEMM_TRAFFIC_N8192 = 23.44e9
 
 
 def ozaki_roofline(phases, tc_flops, steps, pk, pk_kind, n=8192, fast8=True):

@@ -354,8 +354,8 @@ typedef struct {
  * would be a pidblas::mulmm call).  Form PLAIN: one persistent grouped
  * launch over all problems' 64 x 64 tiles (work counter, no waits),
  * bit-identical per problem to vcpcu_igemm_dev PLAIN.  Form OZAKI: grouped
- * products -- the problems bucketed by padded inner dimension, nine launches
- * per bucket over all its problems -- bit-identical per problem to
+ * products -- the problems with one CRT plan together, cut into chunks of a
+ * memset and four launches -- bit-identical per problem to
  * vcpcu_igemm_dev OZAKI.  OZAKI_SLICES: product by product on forked
  * streams.  AUTO: each problem in the form the cost model picks for a batch
  * problem (vcpcu_autotune_choice with batched = 1), both parts concurrent.
