@@ -39,6 +39,7 @@
 #include "swfp.cuh"
 
 #include <cstring>
+#include <type_traits>
 
 namespace vcpcu {
 
@@ -324,6 +325,25 @@ __device__ __forceinline__ void digits16(int n, int& d1, int& d0) {
   d1 = (n + 128) >> 8;
 }
 
+// An entry of a point factor where no radius product runs: its integer alone.
+static __device__ __noinline__ long long point_general(double x, int E, int w) {
+  return sw_finite(x) ? crt_int(x, E, w) : 0;
+}
+__device__ __forceinline__ long long point_int(double x, const Line& ln, int w) {
+  const Words b = words(x);
+  if (ln.direct && ((uint32_t)iv_exp(b) - 64u <= 1982u || ((b.hi << 1) | b.lo) == 0))
+    return __double2ll_rn(__dmul_rn(x, ln.scale));
+  return point_general(x, ln.E, w);
+}
+__device__ __forceinline__ double load_split(const PrepSide& s, size_t at, double) {
+  return s.X[at];
+}
+__device__ __forceinline__ double2 load_split(const PrepSide& s, size_t at, double2) {
+  return load_entry(s, at);
+}
+__device__ __forceinline__ void zero_split(double& v) { v = 0.0; }
+__device__ __forceinline__ void zero_split(double2& v) { v = make_double2(0.0, 0.0); }
+
 // Sums of a thread's entries.
 struct LineSums {
   unsigned long long hi = 0, lo = 0;  // sum |A'| = hi 2^32 + lo
@@ -333,15 +353,25 @@ struct LineSums {
 // Eight consecutive k of one line: digit planes (dst1 / dst2: products 1 /
 // 2), residue planes, sums.  off is the element offset of the first within a
 // plane; store false (a line past the last) writes nothing.
-template <int NL, bool LEFT>
-__device__ __forceinline__ void split8(const double2 (&v)[8], const Line& ln, const PrepArgs& p,
+// V: double2, or double (POINT kernels: both factors plain doubles and no
+// radius product, so no digits).
+template <int NL, bool LEFT, class V>
+__device__ __forceinline__ void split8(const V (&v)[8], const Line& ln, const PrepArgs& p,
                                        const PrepSide& s, size_t off, bool store, LineSums& sums) {
+  constexpr bool POINT = std::is_same_v<V, double>;
   unsigned long long h[4][NL];
   uint32_t b1[4] = {}, b0[4] = {}, r1[4] = {}, r0[4] = {};
-  const bool digits = p.run1 | p.run2;  // (no radius product: both radii are zero)
+  const bool digits = !POINT && (p.run1 | p.run2);  // (no radius product: both radii are zero)
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    const Ints x = entry_ints<LEFT>(v[2 * t], ln, p.w), y = entry_ints<LEFT>(v[2 * t + 1], ln, p.w);
+    Ints x, y;
+    if constexpr (POINT) {
+      x = Ints{point_int(v[2 * t], ln, p.w), 0, 0};
+      y = Ints{point_int(v[2 * t + 1], ln, p.w), 0, 0};
+    } else {
+      x = entry_ints<LEFT>(v[2 * t], ln, p.w);
+      y = entry_ints<LEFT>(v[2 * t + 1], ln, p.w);
+    }
     limbs_pair<NL>(x.a, y.a, h[t]);
     const unsigned long long ax = (unsigned long long)(x.a < 0 ? -x.a : x.a),
                              ay = (unsigned long long)(y.a < 0 ? -y.a : y.a);
@@ -368,11 +398,11 @@ __device__ __forceinline__ void split8(const double2 (&v)[8], const Line& ln, co
   auto put = [&](uint16_t* plane, const uint32_t (&x)[4]) {
     *reinterpret_cast<uint4*>(plane + off) = make_uint4(x[0], x[1], x[2], x[3]);
   };
-  if (p.run1) {  // (|mA| + rA) rB
+  if (!POINT && p.run1) {  // (|mA| + rA) rB
     put(s.p1, LEFT ? b1 : r1);
     put(s.p1 + s.pstride, LEFT ? b0 : r0);
   }
-  if (p.run2) {  // rA |mB|
+  if (!POINT && p.run2) {  // rA |mB|
     put(s.p2, LEFT ? r1 : b1);
     put(s.p2 + s.pstride, LEFT ? r0 : b0);
   }
@@ -417,7 +447,7 @@ __device__ __forceinline__ void add_sums(LineSums x, int lanes, int step, bool f
 // time then write two lines of a plane (with rows fastest they wrote eight,
 // and the store pipe, 36 passes an instruction, was the bound: 1225x12544
 // 332 -> 301 us, n = 8192 1441 -> 1311).
-template <int NL>
+template <int NL, class V>
 __device__ __forceinline__ void split_left(const PrepArgs& p, int rb, int kb0, int steps) {
   const PrepSide& s = p.a;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -430,11 +460,12 @@ __device__ __forceinline__ void split_left(const PrepArgs& p, int rb, int kb0, i
   for (int it = 0; it < steps; ++it) {
     const int k = (kb0 + it) * 64 + (warp >> 2) * 32 + (lane & 3) * 8;
     if ((kb0 + it) * 64 >= p.Kp) break;
-    double2 v[8];
+    V v[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
-      v[t] = row && k + t < p.K ? load_entry(s, (size_t)i + (size_t)(k + t) * s.ld)
-                                : make_double2(0.0, 0.0);
+    for (int t = 0; t < 8; ++t) {
+      zero_split(v[t]);
+      if (row && k + t < p.K) v[t] = load_split(s, (size_t)i + (size_t)(k + t) * s.ld, V());
+    }
     split8<NL, true>(v, ln, p, s, oz_tile_off(s.line0 + i, OZ_BM, k, p.Kp), row, sums);
   }
   add_sums<NL, true>(sums, 4, 1, row && (lane & 3) == 0, s.sum + 4 * (size_t)i);
@@ -451,23 +482,23 @@ __host__ __device__ __forceinline__ int right_lanes(int Kp) {
 // lane through shared memory (one 16-byte slot of padding per 8 entries: no
 // bank conflicts), so that a plane's store is 16 bytes per lane, contiguous
 // along each column.
-template <int NL>
+template <int NL, class V>
 __device__ __forceinline__ void split_right(const PrepArgs& p, int cb, int kb) {
-  __shared__ double2 turn[NT / 32][288];
+  __shared__ V turn[NT / 32][288];
   const PrepSide& s = p.b;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lanes = right_lanes(p.Kp), per = 8 * lanes;  // lanes and k per column
   const int col0 = (cb * 8 + warp) * (32 / lanes);
   if (col0 >= s.lines) return;  // whole warps only (no block barrier below)
   const int k0 = kb * per;
-  double2* T = turn[warp];
+  V* T = turn[warp];
   {
-    double2 v[8];
+    V v[8];
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
       const int x = 32 * t + lane, j = col0 + x / per, k = k0 + (x & (per - 1));
-      v[t] = j < s.lines && k < p.K ? load_entry(s, (size_t)k + (size_t)j * s.ld)
-                                    : make_double2(0.0, 0.0);
+      zero_split(v[t]);
+      if (j < s.lines && k < p.K) v[t] = load_split(s, (size_t)k + (size_t)j * s.ld, V());
     }
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
@@ -481,7 +512,7 @@ __device__ __forceinline__ void split_right(const PrepArgs& p, int cb, int kb) {
   const uint32_t* e = s.e + 2 * (size_t)j;
   const int Fm = col ? exp_dec(e[0]) : OZ_ZERO_EXP, Fr = col ? exp_dec(e[1]) : OZ_ZERO_EXP;
   const Line ln = make_line(Fm, Fm, Fr, p.w);
-  double2 v[8];
+  V v[8];
 #pragma unroll
   for (int t = 0; t < 8; ++t) v[t] = T[9 * lane + t];
   LineSums sums;
@@ -490,23 +521,29 @@ __device__ __forceinline__ void split_right(const PrepArgs& p, int cb, int kb) {
   add_sums<NL, false>(sums, lanes, 1, col && (lane & (lanes - 1)) == 0, s.sum + 4 * (size_t)j);
 }
 
-template <int NL>
+template <int NL, class V>
 __device__ __forceinline__ void split_block(const PrepArgs& p, int local) {
   if (local < p.nA) {
     const int nrb = (p.a.lines + 31) >> 5;
-    split_left<NL>(p, local % nrb, (local / nrb) * p.spanA, p.spanA);
+    split_left<NL, V>(p, local % nrb, (local / nrb) * p.spanA, p.spanA);
   } else {
     local -= p.nA;
     const int nkb = (p.Kp + 8 * right_lanes(p.Kp) - 1) / (8 * right_lanes(p.Kp));
-    split_right<NL>(p, local / nkb, local % nkb);
+    split_right<NL, V>(p, local / nkb, local % nkb);
   }
 }
 
-template <int NL>
-__global__ void __launch_bounds__(NT, 3) oz_crt_split(const __grid_constant__ PrepArgs p) {
+// Two point factors without a radius product (the directed point product) hold
+// one double an entry, no digits and no width test: 62 registers, so that a
+// fourth block fits an SM, and 16384 x 16384 takes 1600 us where the general
+// kernel took 2360 (10.7 GB: 6.7 TB/s; 4.5 before).  The general kernel at four
+// blocks spills (n = 8192 1.25 -> 1.43 ms), at two it is 12 % slower.
+template <int NL, class V>
+__global__ void __launch_bounds__(NT, std::is_same_v<V, double> && NL < 6 ? 4 : 3)
+oz_crt_split(const __grid_constant__ PrepArgs p) {
   dep_wait();
   dep_ready();
-  split_block<NL>(p, blockIdx.x);
+  split_block<NL, V>(p, blockIdx.x);
 }
 
 // ------------------------------------------------------ grouped products
@@ -553,7 +590,7 @@ __global__ void __launch_bounds__(NT, 3) oz_crt_split_g(const __grid_constant__ 
   PrepArgs a = group_args(b, q, p);
   a.nA = q.split_left;
   a.spanA = 1;
-  split_block<NL>(a, blockIdx.x - b.blk_split[p]);
+  split_block<NL, double2>(a, blockIdx.x - b.blk_split[p]);
 }
 
 inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
@@ -589,7 +626,12 @@ int prepare(PrepArgs& p, cudaStream_t st) {
   if (blocks <= 0) return VCPCU_OK;
   // |A'|, |B'| <= 2^(w-1): four 14-bit limbs up to w = 56, five 12-bit limbs
   // up to w = 61, six up to 73
-  const auto split = p.w <= 56 ? oz_crt_split<4> : (p.w <= 61 ? oz_crt_split<5> : oz_crt_split<6>);
+  const bool point = p.a.raw && p.b.raw && !p.run1 && !p.run2;
+  const auto split =
+      point ? (p.w <= 56 ? oz_crt_split<4, double>
+                         : (p.w <= 61 ? oz_crt_split<5, double> : oz_crt_split<6, double>))
+            : (p.w <= 56 ? oz_crt_split<4, double2>
+                         : (p.w <= 61 ? oz_crt_split<5, double2> : oz_crt_split<6, double2>));
   VCPCU_CUDA_TRY(launch_dep(after_maxima, 1, split, dim3((unsigned)blocks), dim3(NT), 0, st, p));
   VCPCU_LAUNCH_CHECK("oz_crt_split");
   return VCPCU_OK;
