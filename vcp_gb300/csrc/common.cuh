@@ -62,6 +62,9 @@ struct Scratch {
 // for the chunks of a batch: on their two streams the waiting blocks hold
 // places that the other stream's kernels would take (1743 -> 1874 us).
 // Without `chained`, an ordinary launch (and dep_wait() returns at once).
+// A chained kernel lives while its predecessors write, so it must not take what
+// they write through __restrict__ pointers to const or __ldg: the read-only path
+// that these allow is only for data constant during the kernel's whole life.
 #ifdef __CUDACC__
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_ready() {

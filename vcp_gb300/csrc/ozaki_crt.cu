@@ -119,7 +119,7 @@ __device__ __forceinline__ void big_to_dir(const uint32_t (&mag)[4], int neg, in
 // one fp32 fold per product (slot 0 and slot nslot = 1), the slice GEMM
 // epilogue's upward sum of every chunk weighted by its digit pair -- an
 // upper bound of the exact integer W of the product.
-__device__ __forceinline__ void rad_folds(const int32_t* __restrict__ P, size_t plane,
+__device__ __forceinline__ void rad_folds(const int32_t* P, size_t plane,
                                           size_t e0, const OzRadConst& rc, float (&S1)[4],
                                           float (&S2)[4]) {
   const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -263,10 +263,9 @@ __device__ __forceinline__ double asum_ru(unsigned long long ah, unsigned long l
 // The rows [i0, i0 + nr) and columns [j0, j0 + nc) of the tile.  eA, asum, eB
 // and bsum point at row / column 0 of the product.
 __device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j0, int nc, int K,
-                                               int w, int lowb, const uint32_t* __restrict__ eA,
-                                               const unsigned long long* __restrict__ asum,
-                                               const uint32_t* __restrict__ eB,
-                                               const unsigned long long* __restrict__ bsum) {
+                                               int w, int lowb, const uint32_t* eA,
+                                               const unsigned long long* asum, const uint32_t* eB,
+                                               const unsigned long long* bsum) {
   for (int x = threadIdx.x; x < ASM_ROWS + ASM_COLS; x += ASM_NT) {
     if (x < ASM_ROWS) {
       double sA = 0.0;
@@ -477,16 +476,16 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
 
 // One product: blocks over the column ranges of CB columns, then over the
 // 128-row tiles (one dimension: no limit on either).  Block 0 merges the
-// status words.
+// status words.  (No __restrict__, here and in what it calls: the kernel may
+// start while the ones before it still write res, P and flag, and read-only
+// loads are not ordered by dep_wait().)
 template <bool LOWB>
 __global__ void __launch_bounds__(ASM_NT, 3)
-oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB,
-                       const uint8_t* __restrict__ res, size_t plane,
-                       const uint32_t* __restrict__ eA, const uint32_t* __restrict__ eB,
-                       const unsigned long long* __restrict__ asum,
-                       const unsigned long long* __restrict__ bsum, const int32_t* __restrict__ P,
-                       double* __restrict__ C, double* __restrict__ Cup, long ldc,
-                       const int* __restrict__ flag, int merge,
+oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB, const uint8_t* res,
+                       size_t plane, const uint32_t* eA, const uint32_t* eB,
+                       const unsigned long long* asum, const unsigned long long* bsum,
+                       const int32_t* P, double* C, double* Cup, long ldc, const int* flag,
+                       int merge,
                        const __grid_constant__ CrtBasis cc, const __grid_constant__ OzRadConst rc) {
   __shared__ AsmTile t;
   dep_wait();

@@ -174,12 +174,13 @@ __device__ double scale_ru_slow(double x, int e) {
 // instructions.  Three residues meet in one 32-bit value before the eight-limb
 // products (ozaki_dd.cuh; one product per residue before), and the two words
 // of the result come from five leading words picked by selections: n = 2048,
-// L = 28, 250 -> 113 us.
+// L = 28, 250 -> 113 us.  (No __restrict__: the kernel may start while the ones
+// before it still write res and flag, and read-only loads are not ordered by
+// dep_wait().)
 __global__ void __launch_bounds__(128, 6)
-dd_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, const uint8_t* __restrict__ res,
-                       size_t plane, const uint32_t* __restrict__ eA,
-                       const uint32_t* __restrict__ eB, double* __restrict__ C, long ldc,
-                       double* __restrict__ Cerr, long lde, const int* __restrict__ flag,
+dd_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, const uint8_t* res,
+                       size_t plane, const uint32_t* eA, const uint32_t* eB, double* C, long ldc,
+                       double* Cerr, long lde, const int* flag,
                        const __grid_constant__ DdBasis cc) {
   dep_wait();
   const bool bad = flag[0] != 0 || flag[1] != 0;
