@@ -169,7 +169,8 @@ int vcpcu_udmatmul_ozaki(int m, int n, int k, const double* A, const double* B,
  *     (the classic Ozaki splitting) with a rigorous truncation bound.
  *   form == VCPCU_FORM_AUTO: the autotuner picks the form and slice count.
  * Device pointers; stream-ordered; scratch comes from the stream-ordered
- * allocator of the current device. */
+ * allocator of the current device.  C may overlap A or B: both are read to
+ * the end before C is written. */
 int vcpcu_igemm_dev(int m, int n, int k, const double* A, int lda,
                     const double* B, int ldb, double* C, int ldc,
                     int form, int slices, void* stream);
@@ -200,7 +201,7 @@ int vcpcu_igemm(int m, int n, int k, const double* A, const double* B,
  * Point matrices are plain doubles, intervals kv pairs.  The plain form is
  * bit-identical to pidblas over a sequential-chain dgemm (lC = RD(mid*P),
  * uC = RU(mid*P), temp = RU(rad*|P|), uC +=RU temp, lC -=RD temp); the
- * Ozaki forms enclose the same product. */
+ * Ozaki forms enclose the same product.  C may overlap L or R. */
 int vcpcu_igemm_point_dev(int interval_side, int m, int n, int k,
                           const double* L, int ldl, const double* R, int ldr,
                           double* C, int ldc, int form, int slices, void* stream);

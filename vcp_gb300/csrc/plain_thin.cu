@@ -495,6 +495,21 @@ int launch_interval_gemm_thin(int M, int N, int K, const double* A, long lda, Th
     return VCPCU_ERR_INVALID_ARG;
   }
   if (K < 0) K = 0;
+  // The kernel reads A while blocks of the same rows and other columns store C:
+  // where the two overlap (a product in place), it reads a copy.
+  Scratch copy;
+  if (K > 0) {
+    const size_t esz = left == THIN_POINT ? 8 : 16;
+    const uintptr_t a0 = (uintptr_t)A, a1 = a0 + esz * ((size_t)(K - 1) * lda + M);
+    const uintptr_t c0 = (uintptr_t)C, c1 = c0 + 16 * ((size_t)(N - 1) * ldc + M);
+    if (a0 < c1 && c0 < a1) {
+      if (int e = copy.alloc(esz * (size_t)M * K, s)) return e;
+      VCPCU_CUDA_TRY(cudaMemcpy2DAsync(copy.ptr, esz * M, A, esz * lda, esz * M, K,
+                                       cudaMemcpyDeviceToDevice, s));
+      A = (const double*)copy.ptr;
+      lda = M;
+    }
+  }
   double* mB = ws;
   double* rB = mB + (size_t)K * N;
   if (K > 0) {
