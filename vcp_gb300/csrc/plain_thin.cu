@@ -7,20 +7,26 @@
 // Both are bound by their chains, one per row and kind, in ascending column
 // order: GB300's FP64 pipe takes 64 cycles for a warp instruction whatever
 // its active lanes, and 64 for the next one of the same chain.  So every
-// chain has a lane of its own, the chains of a kind share a warp, the two
-// FP64 chains of a product sit on two sub-partitions of an SM, and all chains
-// of non-negative terms run on the integer pipe (dirchain.cuh) on the other
-// two.  Everything that is not the chain -- midrad, kv |.|, significands and
+// chain has a lane of its own and the chains of a kind share a warp.  The four
+// chains of a product run in FP64, one kind on each sub-partition of an SM; the
+// row sums, of non-negative terms, on the integer pipe (dirchain.cuh).
+// Everything that is not the chain -- midrad, kv |.|, significands and
 // exponents -- is done ahead of it by four producer warps, which stream the
 // matrix through a ring of cp.async stages and leave one processed stage of 16
 // columns for the chain warps per barrier.  Measured at n = 4096, against two
 // FP64 chains per lane (two lanes a row) and separate midrad, shift and |.|
-// passes: interval x point vector 658 -> 290 us, point x interval vector
-// 361 -> 247, |E| x vector 867 -> 251, norm 311 -> 128; at n = 1225 the norm
-// and the interval sums of |X| 230 -> 47 us (three passes before).  The FP64
-// chains alone are 131 us at n = 4096 (64 cycles a step), an integer chain
-// warp takes about 120 cycles a step; with an SM to itself a block therefore
-// runs all four chains in FP64 (thin_launch_as).
+// passes: interval x point vector 658 -> 224 us, point x interval vector
+// 361 -> 208, |E| x vector 867 -> 221, norm 311 -> 128; at n = 1225 the norm
+// and the interval sums of |X| 230 -> 47 us (three passes before).  (About 105
+// cycles a step; bare chains on all four sub-partitions take 76 with operands
+// in registers and 82 with loads from shared memory.  Twice the producer warps,
+// or a stage's operands loaded ahead of its first step, left the time as it is.)
+//   With the radius chains of the product on the integer pipe a chain's terms
+// that outgrow its unit cost steps of their own, one lane's for all 32: an inner
+// dimension of 64 (100000 x 16) took 2653 us where two lanes a row had taken 940
+// and this form takes 724, exponents over +-600 (4000 x 3, k = 4000) 2099 for
+// 1954 and now 410.  Narrow spreads at k = 4096: 3 columns 535 and 418 us, 8
+// columns 917 and 1057, 16 columns 1965 and 1912.
 #include "common.cuh"
 #include "dirchain.cuh"
 #include "ozaki_prep.cuh"
@@ -28,7 +34,6 @@
 #include "swfp.cuh"
 
 #include <mutex>
-#include <type_traits>
 
 namespace vcpcu {
 
@@ -134,40 +139,32 @@ __device__ __forceinline__ double2 entry_abs(double2 e) {
 //   0  the round-down midpoint chain, negated into a round-up one
 //      (RD(a b + c) = -RU((-a) b + (-c)), signed zeros included)
 //   1  the round-up midpoint chain
-//   2  RU((|mA| +ru rA) rB)       (integer chain, F = ChainFactor, or FP64,
-//   3  RU(rA |mB|)                 F = double: thin_launch says where)
+//   2  RU((|mA| +ru rA) rB)
+//   3  RU(rA |mB|)
 // and T = 2 +ru 3, C = [1st -rd T, 2nd +ru T] as pidblas::mulmm combines them;
 // four producer warps.  A step past K multiplies zeros and leaves every chain
 // unchanged.
-template <int NB, class F>
+template <int NB>
 struct ThinStage {
   double m[TG * TR];
-  F f[2][TG * TR];  // P, r
+  double f[2][TG * TR];  // P, r
   double bm[TG][NB];
-  F fb[2][TG][NB];  // rB, |mB|
+  double fb[2][TG][NB];  // rB, |mB|
 };
-template <int NB, class F>
+template <int NB>
 struct ThinSmem {
   double2 ring[TSTAGES][TG * TR];
-  ThinStage<NB, F> st[2];
+  ThinStage<NB> st[2];
   double T[2][TR][NB + 1];
 };
 
-template <class F>
-__device__ __forceinline__ F thin_factor(double x) {
-  if constexpr (std::is_same_v<F, double>)
-    return x;
-  else
-    return chain_factor(x);
-}
-
-template <int NB, int LEFT, class F>
+template <int NB, int LEFT>
 __global__ void __launch_bounds__(256)
 interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, long lda,
                           const double* __restrict__ mB, const double* __restrict__ rB,
                           double* __restrict__ C, long ldc) {
   extern __shared__ __align__(16) uint8_t thin_smem[];
-  ThinSmem<NB, F>& sm = *reinterpret_cast<ThinSmem<NB, F>*>(thin_smem);
+  ThinSmem<NB>& sm = *reinterpret_cast<ThinSmem<NB>*>(thin_smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i0 = blockIdx.x * TR, i = i0 + lane, j0 = blockIdx.y * NB;
   const int ng = (K + TG - 1) / TG;
@@ -200,14 +197,14 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
     for (int g = 0; g <= ng; ++g) {
       if (g < ng) {
         cp_wait<TSTAGES - 2>();
-        ThinStage<NB, F>& st = sm.st[g & 1];
+        ThinStage<NB>& st = sm.st[g & 1];
 #pragma unroll
         for (int q = 0; q < QB; ++q) {
           const int x = t + PT * q;
           if (x < TG * NB) {
             st.bm[x % TG][x / TG] = bm[q];
-            st.fb[0][x % TG][x / TG] = thin_factor<F>(br[q]);
-            st.fb[1][x % TG][x / TG] = thin_factor<F>(oz_abs(bm[q]));
+            st.fb[0][x % TG][x / TG] = br[q];
+            st.fb[1][x % TG][x / TG] = oz_abs(bm[q]);
           }
         }
         load_b(g + 1);
@@ -228,65 +225,36 @@ interval_gemm_thin_kernel(int M, int N, int K, const double* __restrict__ A, lon
             v = entry_mid(e);
           }
           st.m[x] = v.m;
-          st.f[0][x] = thin_factor<F>(v.P);
-          st.f[1][x] = thin_factor<F>(v.r);
+          st.f[0][x] = v.P;
+          st.f[1][x] = v.r;
         }
         issue(g + TSTAGES - 1);  // (into the slot of stage g - 1, this thread's own)
       }
       __syncthreads();  // stage g is there; stage g - 1 has been used
     }
   } else {
-    // FP64 chains of blocks that share an SM on different sub-partitions
-    const int role = (warp + 2 * ((blockIdx.x / 152) & 1)) & 3;
-    constexpr bool fp64 = std::is_same_v<F, double>;
-    double c[NB];    // roles 0, 1; FP64 chains of roles 2, 3
-    DirChain x[NB];  // roles 2, 3
+    const int role = warp;
+    double c[NB];
 #pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      c[j] = role == 0 ? -0.0 : 0.0;
-      x[j] = chain_zero();
-    }
+    for (int j = 0; j < NB; ++j) c[j] = role == 0 ? -0.0 : 0.0;
     for (int g = 0; g <= ng; ++g) {
       if (g > 0) {
-        const ThinStage<NB, F>& st = sm.st[(g - 1) & 1];
-        if constexpr (fp64) {
-          const double* fa = (role < 2 ? st.m : st.f[role - 2]) + lane;
-          const double(*fb)[NB] = role < 2 ? st.bm : st.fb[role - 2];
-          const uint64_t neg = role == 0 ? 1ULL << 63 : 0ULL;
+        const ThinStage<NB>& st = sm.st[(g - 1) & 1];
+        const double* fa = (role < 2 ? st.m : st.f[role - 2]) + lane;
+        const double(*fb)[NB] = role < 2 ? st.bm : st.fb[role - 2];
+        const uint64_t neg = role == 0 ? 1ULL << 63 : 0ULL;
 #pragma unroll
-          for (int p = 0; p < TG; ++p) {
-            const double a = sw_double(sw_bits(fa[p * TR]) ^ neg);
+        for (int p = 0; p < TG; ++p) {
+          const double a = sw_double(sw_bits(fa[p * TR]) ^ neg);
 #pragma unroll
-            for (int j = 0; j < NB; ++j) c[j] = __fma_ru(a, fb[p][j], c[j]);
-          }
-        } else if (role < 2) {
-#pragma unroll
-          for (int p = 0; p < TG; ++p) {
-            const double m = st.m[p * TR + lane], a = role == 0 ? sw_neg(m) : m;
-#pragma unroll
-            for (int j = 0; j < NB; ++j) c[j] = __fma_ru(a, st.bm[p][j], c[j]);
-          }
-        } else {
-          const ChainFactor* fa = st.f[role - 2] + lane;
-          const ChainFactor(*fb)[NB] = st.fb[role - 2];
-#pragma unroll 1
-          for (int p0 = 0; p0 < TG; p0 += TB) {
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-              auto get = [&](int p, ChainFactor* u, ChainFactor* v) {
-                *u = fa[(p0 + p) * TR];
-                *v = fb[p0 + p][j];
-              };
-              chain_fma_n<TB>(x[j], get, get);
-            }
-          }
+          for (int j = 0; j < NB; ++j) c[j] = __fma_ru(a, fb[p][j], c[j]);
         }
       }
       __syncthreads();
     }
     if (role >= 2) {
 #pragma unroll
-      for (int j = 0; j < NB; ++j) sm.T[role - 2][lane][j] = fp64 ? c[j] : chain_value(x[j]);
+      for (int j = 0; j < NB; ++j) sm.T[role - 2][lane][j] = c[j];
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");  // the four chain warps
     if (role < 2 && i < M) {
@@ -430,35 +398,43 @@ int smem_optin(size_t bytes) {
   return VCPCU_OK;
 }
 
-// All four chains go through the FP64 pipe where the blocks do not outnumber
-// the SMs: each chain warp then has a sub-partition, and its pipe, to itself
-// (64 cycles a step, against about 120 of an integer chain alone on its own).
-// With two blocks an SM the integer chains of one fill the other's pipes.
-// n = 4096, integer -> FP64 radius chains: interval x point vector 285 -> 224
-// us, point x interval vector 243 -> 208, |E| x vector 247 -> 221.  (That is
-// about 105 cycles a step.  Bare chains on all four sub-partitions take 76
-// with operands in registers and 82 with loads from shared memory; twice the
-// producer warps, or a stage's operands loaded ahead of its first step, left
-// the time as it is.)
-template <int NB, int LEFT, class F>
-int thin_launch_as(int M, int N, int K, const double* A, long lda, const double* mB,
+template <int NB, int LEFT>
+int thin_launch(int M, int N, int K, const double* A, long lda, const double* mB,
                 const double* rB, double* C, long ldc, cudaStream_t s) {
-  constexpr size_t bytes = sizeof(ThinSmem<NB, F>);
-  if (int e = smem_optin<interval_gemm_thin_kernel<NB, LEFT, F>>(bytes)) return e;
+  constexpr size_t bytes = sizeof(ThinSmem<NB>);
+  if (int e = smem_optin<interval_gemm_thin_kernel<NB, LEFT>>(bytes)) return e;
   const dim3 grid((M + TR - 1) / TR, (N + NB - 1) / NB);
-  interval_gemm_thin_kernel<NB, LEFT, F>
-      <<<grid, 256, bytes, s>>>(M, N, K, A, lda, mB, rB, C, ldc);
+  interval_gemm_thin_kernel<NB, LEFT><<<grid, 256, bytes, s>>>(M, N, K, A, lda, mB, rB, C, ldc);
   VCPCU_LAUNCH_CHECK("interval_gemm_thin_kernel");
   return VCPCU_OK;
 }
 
-template <int NB, int LEFT>
-int thin_launch(int M, int N, int K, const double* A, long lda, const double* mB,
-                const double* rB, double* C, long ldc, cudaStream_t s) {
-  const long blocks = (long)((M + TR - 1) / TR) * ((N + NB - 1) / NB);
-  if (blocks <= 152)
-    return thin_launch_as<NB, LEFT, double>(M, N, K, A, lda, mB, rB, C, ldc, s);
-  return thin_launch_as<NB, LEFT, ChainFactor>(M, N, K, A, lda, mB, rB, C, ldc, s);
+// Columns of a block (1, 2, 4, 8 or 16) from an estimate of the cycles: a
+// block keeps each sub-partition's FP64 pipe for 64 cycles a step and column,
+// the pipes are shared by the up to three blocks of an SM (two from four columns
+// on: shared memory), and the blocks of a last wave land together on the SMs that
+// are free first; a wave's fill and end take about 4000 cycles.  Single columns
+// come out up to a quarter better than that: a tenth in their favour.  us for 1 /
+// 2 / 4 / 8 / 16 columns, the estimate's choice in brackets: 4096 x 16, k = 4096
+// [1914] 2373 2086 2071 2478; 4096 x 8 1089 1585 [1051] 1255; 8192 x 2, k = 8192
+// 1260 [1077]; 5000 x 3, k = 5000 [783] 973 1279; 10000 x 16, k = 1000 [1123]
+// 1184 1196 1398 1650; 100000 x 16, k = 16 341 271 253 226 [224].
+inline int thin_cols(int M, int N, int K) {
+  const long rb = (M + TR - 1) / TR;
+  int best = 1;
+  double cost = 0.0;
+  for (int nb = 1; nb < 2 * N && nb <= kThinN; nb <<= 1) {
+    const long blocks = rb * ((N + nb - 1) / nb), per = nb <= 2 ? 3 : 2;
+    const long waves = (blocks + 152 * per - 1) / (152 * per);
+    const long depth = waves == 1 ? (blocks + 151) / 152 : per * waves;
+    const double c =
+        (nb == 1 ? 64.0 : 70.4 * nb) * (double)depth * K + 4000.0 * (double)waves;
+    if (nb == 1 || c < cost) {
+      best = nb;
+      cost = c;
+    }
+  }
+  return best;
 }
 
 template <int NB>
@@ -521,11 +497,7 @@ int launch_interval_gemm_thin(int M, int N, int K, const double* A, long lda, Th
       thin_prep_right<false><<<blocks, 256, 0, s>>>(K, N, B, ldb, mB, rB);
     VCPCU_LAUNCH_CHECK("thin_prep_right");
   }
-  // columns per block: as few as keep two blocks on each of the 152 SMs (the
-  // columns of a block follow one another on its FP64 chains)
-  const long rb = (M + TR - 1) / TR;
-  int nb = 1;
-  while (nb < N && rb * ((N + nb - 1) / nb) > 304) nb <<= 1;
+  const int nb = thin_cols(M, N, K);
   if (nb == 1) return thin_launch_left<1>(left, M, N, K, A, lda, mB, rB, C, ldc, s);
   if (nb == 2) return thin_launch_left<2>(left, M, N, K, A, lda, mB, rB, C, ldc, s);
   if (nb == 4) return thin_launch_left<4>(left, M, N, K, A, lda, mB, rB, C, ldc, s);
