@@ -85,7 +85,7 @@ static __device__ __noinline__ Exps entry_exponents_general(double lo, double up
   Exps x{0, 0, 0, false};
   if (!sw_finite(lo) || !sw_finite(up)) return x;
   double m, r, p;
-  sw_midrad(lo, up, m, r, p);
+  if (!sw_midrad_wide(lo, up, m, r, p)) sw_midrad_hw(lo, up, m, r, p);
   x.m = exp_enc(oz_exponent(oz_abs(m)));
   x.p = exp_enc(oz_exponent(p));
   x.r = exp_enc(oz_exponent(r));
@@ -295,7 +295,7 @@ static __device__ __noinline__ Ints entry_general(double lo, double up, int E, i
   Ints x{0, 0, 0};
   if (!sw_finite(lo) || !sw_finite(up)) return x;  // the whole result is NaN then
   double m, r, p;
-  sw_midrad(lo, up, m, r, p);
+  if (!sw_midrad_wide(lo, up, m, r, p)) sw_midrad_hw(lo, up, m, r, p);
   x.a = crt_int(m, E, w);
   if (Eb != OZ_ZERO_EXP) x.nb = (int)oz_scaled_int64(LEFT ? p : oz_abs(m), Eb, 16, 1);
   if (Er != OZ_ZERO_EXP) x.nr = (int)oz_scaled_int64(r, Er, 16, 1);

@@ -13,7 +13,7 @@
 //                  power of two itself).
 // An entry that is the same zero at both ends goes the same way (all of it
 // zero).
-// Other entries take the general midrad (swfp.cuh).
+// Other entries take sw_midrad_wide (swfp.cuh).
 #pragma once
 #include "ozaki_common.cuh"
 

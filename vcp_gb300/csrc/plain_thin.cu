@@ -102,7 +102,7 @@ struct Mid {
 };
 static __device__ __noinline__ Mid entry_mid_general(double lo, double up) {
   Mid x;
-  sw_midrad(lo, up, x.m, x.r, x.P);
+  if (!sw_midrad_wide(lo, up, x.m, x.r, x.P)) sw_midrad_hw(lo, up, x.m, x.r, x.P);
   return x;
 }
 __device__ __forceinline__ Mid entry_mid(double2 v) {

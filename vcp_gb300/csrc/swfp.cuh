@@ -2,10 +2,7 @@
 //
 // GB300 issues FP64 at 1/64 of the FP32 rate, so the operand preparation of
 // the tensor-core form (one kv midrad per interval entry) is bound by the
-// FP64 pipe when it uses FP64 instructions.  (A single FP64 instruction per
-// entry beside integer-bound work is cheaper on the FP64 pipe, which runs in
-// parallel: the upward additions |m| + r of the splits and of the radius
-// term stay FP64 instructions.)  The functions below compute the
+// FP64 pipe when it uses FP64 instructions.  The functions below compute the
 // same bits with integer operations for the common case -- both endpoints
 // normal, of one sign, binary exponents at most one apart (an interval
 // narrower than its midpoint) -- and fall back to the FP64 instructions
@@ -158,11 +155,34 @@ __device__ __forceinline__ void sw_midrad_hw(double lo, double up, double& m, do
   p = __dadd_ru(fabs(m), r);
 }
 
+// The same three values of any finite lo <= up whose sum does not overflow, with
+// the four FP64 instructions that round: the sum, m - lo, up - m and |m| + r.
+// The half of the sum is an integer operation (an exponent one lower or, where
+// the half may be subnormal, its bit pattern halved to nearest even), the larger
+// difference the larger bit pattern.  False: the caller takes sw_midrad_hw.
+//   For the entries that the callers' own narrow path leaves over (around zero,
+// ends of two exponents).  sw_midrad's integer attempt and then the seven FP64
+// instructions of sw_midrad_hw, 64 cycles of the pipe each and one after
+// another, bounded whole products of such entries: 2000 x 1, k = 2000 553 -> 250
+// us (318 as a pass of its own over the matrix), n = 2048 on the tensor cores 729
+// -> 544 (749 with its midpoints stored), 1225 x 1225 x 12544 2033 -> 1348 (1974).
+__device__ __forceinline__ bool sw_midrad_wide(double lo, double up, double& m, double& r,
+                                               double& p) {
+  const unsigned long long s = sw_bits(__dadd_rn(lo, up)), b = s & 0x7fffffffffffffffULL;
+  const uint32_t es = (uint32_t)(b >> 52);
+  const unsigned long long h = es >= 2 ? b - (1ULL << 52) : (b >> 1) + (b & (b >> 1) & 1ULL);
+  m = sw_double(h | (s ^ b));
+  const unsigned long long d1 = sw_bits(__dsub_ru(m, lo)), d2 = sw_bits(__dsub_ru(up, m));
+  r = sw_double(d1 > d2 ? d1 : d2);
+  p = __dadd_ru(sw_double(h), r);
+  return es != 0x7ffu && ((d1 | d2) >> 63) == 0;
+}
+
 // The FP64 fallbacks are out of line: inlined, the compiler may issue their
 // first FP64 instruction speculatively on the common path.
 static __device__ __noinline__ void sw_midrad_slow(double lo, double up, double& m, double& r,
                                             double& p) {
-  sw_midrad_hw(lo, up, m, r, p);
+  if (!sw_midrad_wide(lo, up, m, r, p)) sw_midrad_hw(lo, up, m, r, p);
 }
 
 __device__ __forceinline__ void sw_midrad(double lo, double up, double& m, double& r,
