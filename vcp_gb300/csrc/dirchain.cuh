@@ -242,10 +242,10 @@ OZ_HD void chain_add_n(DirChain& x, GET get, VALUE value) {
   chain_batch<UP, N>(x, y);
 }
 
-// c = RU(c + a_p b_p), p ascending; get(p, &fa, &fb) gives the factors, again
-// (p not a constant: from memory) for the single steps.
-template <int N, typename GET, typename AGAIN>
-OZ_HD void chain_fma_n(DirChain& x, GET get, AGAIN again) {
+// c = RU(c + a_p b_p), p ascending, get(p, &fa, &fb) the factors: the whole
+// batch at once, or false and x as it was.
+template <int N, typename GET>
+OZ_HD bool chain_fma_batch(DirChain& x, GET get) {
   long long y[N];
   int sm = 1;
   const int U = x.U + 1023;
@@ -259,16 +259,36 @@ OZ_HD void chain_fma_n(DirChain& x, GET get, AGAIN again) {
     const long long t1 = (long long)fa.h * fb.l + ((long long)fa.l * fb.h + (t0 >> 26));
     y[p] = chain_shr((long long)fa.h * fb.h + (t1 >> 26), s);
   }
-  if (sm < 1 || x.U > CHAIN_TOP || x.U < 1) {
-#pragma unroll 1
+  if (sm < 1 || x.U > CHAIN_TOP || x.U < 1) return false;
+  chain_batch<true, N>(x, y);
+  return true;
+}
+// Its steps one by one (p not a constant: get from memory).  fp64: all of them
+// the FP64 instruction, for a young chain -- a term outgrows its unit so often
+// that some lane of a warp takes an FP64 step at nearly every p anyway.
+template <int N, typename GET>
+OZ_HD void chain_fma_steps(DirChain& x, GET get, bool fp64) {
+  if (fp64) {
+    double c = chain_value(x);
+#pragma unroll
     for (int p = 0; p < N; ++p) {
       ChainFactor fa, fb;
-      again(p, &fa, &fb);
-      chain_fma(x, fa, fb);
+      get(p, &fa, &fb);
+      c = chain_fma_ru(chain_factor_value(fa), chain_factor_value(fb), c);
     }
+    x = chain_of(c);
     return;
   }
-  chain_batch<true, N>(x, y);
+#pragma unroll 1
+  for (int p = 0; p < N; ++p) {
+    ChainFactor fa, fb;
+    get(p, &fa, &fb);
+    chain_fma(x, fa, fb);
+  }
+}
+template <int N, typename GET, typename AGAIN>
+OZ_HD void chain_fma_n(DirChain& x, GET get, AGAIN again) {
+  if (!chain_fma_batch<N>(x, get)) chain_fma_steps<N>(x, again, false);
 }
 
 }  // namespace vcpcu

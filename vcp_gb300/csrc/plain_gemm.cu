@@ -233,9 +233,18 @@ namespace {
 // bound, the integer warps take about half the issue slots beside it.  The
 // radius chains' states live in shared memory between batches (their code is
 // one loop over the columns).  n = 512: 64 x 64 tiles with four FP64 chains
-// 2.07 ms, this 0.66; n = 1024 8.24 and
+// 2.07 ms, this 0.64; n = 1024 8.24 and
 // 4.4 ms (3.5 at the FP64 rate).
 constexpr int ITN = 384;  // threads
+// Stages of BKI steps in which a radius chain takes the FP64 instructions:
+// always (some lane's terms outgrow its unit), and where a batch does not go
+// through.  With the single steps instead, one of them in FP64 for the warp at
+// nearly every k, short inner dimensions were slower than four FP64 chains:
+// 3000 x 3000, exponents over +-8, k = 16 / 32 / 64 / 256 1372 / 2490 / 4442 /
+// 12603 us, now 1066 / 2036 / 3670 / 11649 (four FP64 chains 1063 / 2022 / 3940 /
+// 15457); n = 1000 1152 us at k = 256 and narrow exponents, now 1136.  Batches
+// tried in the second stage: 1073 / 2116 / 3776; FP64 up to stage 8: 3970 at 64.
+constexpr int INEW = 2, IYOUNG = 4;
 template <int CW>
 struct ITile {
   struct Stage {
@@ -247,6 +256,21 @@ struct ITile {
   long long c[2][4 * CW][TROWS];
   int U[2][4 * CW][TROWS];
 };
+
+// A stage's steps of a chain one by one; out of line, for the registers of the
+// batches.
+template <int COLS>
+static __device__ __noinline__ DirChain chain_steps(DirChain x, const ChainFactor* a,
+                                                    const ChainFactor* b, bool young) {
+  chain_fma_steps<BKI>(
+      x,
+      [&](int p, ChainFactor* u, ChainFactor* v) {
+        *u = a[p * TROWS];
+        *v = b[p * COLS];
+      },
+      young);
+  return x;
+}
 
 template <int CW>
 __global__ void __launch_bounds__(ITN, 2)
@@ -333,16 +357,11 @@ interval_gemm_kernel(int M, int N, int K, const double* __restrict__ mA,
 #pragma unroll 1
       for (int j = w0; j < w0 + CW; ++j) {
         DirChain x{sm.c[h][j][lane], sm.U[h][j][lane]};
-        chain_fma_n<BKI>(
-            x,
-            [&](int p, ChainFactor* u, ChainFactor* v) {
+        if (t < INEW || !chain_fma_batch<BKI>(x, [&](int p, ChainFactor* u, ChainFactor* v) {
               *u = fa[p];
               *v = fb[p][j];
-            },
-            [&](int p, ChainFactor* u, ChainFactor* v) {
-              *u = a[p * TROWS];
-              *v = fb[p][j];
-            });
+            }))
+          x = chain_steps<COLS>(x, a, &fb[0][j], t < IYOUNG);
         sm.c[h][j][lane] = x.c;
         sm.U[h][j][lane] = x.U;
       }
