@@ -4,7 +4,10 @@
 //   plain  t = 8 m n k / fp64_rate + t_launch
 //   Ozaki  t = (L + 6) 2 Mp Np Kp / tc_rate            (slice GEMMs; L moduli,
 //                                                       2 x 3 radius digit pairs)
-//            + 16 (m k + k n) / prep_bw + 12 t_launch    (operand preparation)
+//            + 16 (m k + k n) / prep_bw + 12 t_launch    (operand preparation;
+//                                                         a product takes five
+//                                                         launches, so small ones
+//                                                         are on the plain side)
 // with the constants measured on this device by vcpcu_autotune (timing one
 // plain and two Ozaki products), kept for the process and optionally stored
 // in / loaded from the file named by VCPCU_AUTOTUNE_CACHE.  Until a
@@ -319,7 +322,7 @@ extern "C" int vcpcu_autotune(void* stream, double* constants) {
   double b = t2 - a * w2;
   if (b < 0) b = 0;
   m.tc_rate = 1.0 / a;
-  // fixed cost b ~ preparation of 2 n2^2 entries + 12 launches
+  // fixed cost b ~ preparation of 2 n2^2 entries + the model's 12 launches
   m.t_launch = 5e-6;
   const double prep_t = b - 12.0 * m.t_launch;
   m.prep_bw = prep_t > 0 ? 16.0 * 2.0 * n2 * (double)n2 / prep_t : 5e12;

@@ -330,7 +330,7 @@ int oz_run_product(const OzPlan& plan, OzWorkspace& ws, const OzOperand& A, cons
     // CRT form: the radius products and the residue GEMMs in one launch
     // (phase 3 times all of them)
     PhaseTimer t(3, s);
-    if ((st = oz_run_gemm(plan, OZ_ALL, ws, nullptr, 0, s, -1, true))) return st;
+    if ((st = oz_run_gemm(plan, OZ_ALL, ws, nullptr, 0, s, true))) return st;
   } else {
     if (!(plan.point_mask & 2)) {
       PhaseTimer t(1, s);

@@ -94,7 +94,7 @@ struct OzPairList {
 };
 
 // OZ_RAD_SET: radius product 1, (|mA| + rA) * rB; OZ_RAD_ADD: radius
-// product 2, rA * |mB|.  Each writes T or adds to it (OzGemmArgs::t_set).
+// product 2, rA * |mB|.  Each leaves its folds in its half of OzWorkspace::P.
 
 enum OzMode { OZ_RAD_SET = 0, OZ_RAD_ADD = 1, OZ_MID = 2, OZ_CRT = 3, OZ_ALL = 4 };
 // OZ_ALL (CRT form): both radius products and the residue GEMMs in one
@@ -109,7 +109,6 @@ struct alignas(128) OzGemmArgs {
   int tiles_m, tiles_n;
   int t_ref, R;     // W unit 2^(E_i + F_j - 8 t_ref); R = floor-shifted folds
   int mode;
-  int t_set;        // radius modes: 1 T = product, 0 T +=RU product
   int s;            // midpoint slices (OZ_MID truncation bound)
   const int* Erow;  // row exponent of the left operand:  Erow[erow_stride * i]
   int erow_stride;
@@ -195,10 +194,8 @@ int oz_prepare_right_cols(const OzProblem& pb, const OzOperand& B, int j0, int c
 int oz_prepare_slices(const OzProblem& pb, const double* A, long lda, const double* B, long ldb,
                       OzWorkspace& ws, cudaStream_t st);
 // chained: the preparation precedes it on st (launch_dep).
-// t_set < 0: the radius product of OZ_RAD_SET writes T, that of OZ_RAD_ADD
-// adds to it; 0 / 1 force add / write.
 int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, long ldc,
-                cudaStream_t st, int t_set = -1, bool chained = false);
+                cudaStream_t st, bool chained = false);
 size_t oz_workspace_bytes(const OzProblem& pb);
 int oz_carve_workspace(const OzProblem& pb, void* base, OzWorkspace* ws);
 

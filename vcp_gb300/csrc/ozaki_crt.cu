@@ -502,8 +502,8 @@ oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB, const 
 }
 
 // Grouped reassembly.  The problems of a bucket share one CRT plan (the
-// bucket is keyed by padded K, modulus count and operand width), so the
-// basis comes in the launch parameters as for one product.  A block takes a
+// bucket is keyed by modulus count, operand width, radius pairs and scaling), so
+// the basis comes in the launch parameters as for one product.  A block takes a
 // tile of up to 128 rows and OZ_GASM_COLS columns of one problem, found with
 // one load (prob_asm); it stamps the problem's end and merges its status
 // words into the sticky status.  A device-wait timeout of the slice

@@ -7,8 +7,8 @@
 // Here each dd entry hi + lo is scaled per row (A) / column (B) to a w-bit
 // integer (w = 8 * slices, default 112 bits), the integer product A'B' is
 // formed exactly from its residues modulo L <= 32 pairwise-coprime moduli
-// <= 256 (one bf16 tensor-core GEMM per modulus, exact fp32 chunks, int32
-// folds), recovered by Chinese remaindering in 256-bit arithmetic, and
+// <= 256 (one bf16 tensor-core GEMM per modulus, exact fp32 chunks, their
+// residues summed in fp32), recovered by Chinese remaindering in 256-bit arithmetic, and
 // rounded to a dd midpoint C = chi + clo.  A rigorous upward-rounded bound
 //   |A B - C| <= K 2^(E+F-w) (1 + 2^-40) + ulp-level conversion error
 // is returned alongside (Cerr).  Inputs and outputs use kv::dd layout:
@@ -345,7 +345,7 @@ int ozaki_ddgemm(int m, int n, int k, const double* A, long lda, const double* B
   }
   {
     PhaseTimer t(3, s);
-    if ((st = oz_run_gemm(plan, OZ_CRT, ws, nullptr, 0, s, -1, true))) return st;
+    if ((st = oz_run_gemm(plan, OZ_CRT, ws, nullptr, 0, s, true))) return st;
   }
   oz_profile_add_flops(2LL * m * n * (long long)(k > 0 ? k : 0) * L);
   {

@@ -875,7 +875,7 @@ static int oz_gemm_smem_optin() {
 }
 
 int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, long ldc,
-                cudaStream_t st, int t_set, bool chained) {
+                cudaStream_t st, bool chained) {
   const OzProblem& pb = plan.pb;
   if (int e = oz_gemm_smem_optin()) return e;
   OzGemmArgs a;
@@ -926,7 +926,6 @@ int oz_run_gemm(const OzPlan& plan, int mode, const OzWorkspace& ws, double* C, 
     return st_;
   a.M = pb.M; a.N = pb.N; a.Mp = pb.Mp; a.Np = pb.Np; a.Kp = pb.Kp;
   a.mode = mode;
-  a.t_set = t_set >= 0 ? t_set : (mode == OZ_RAD_SET ? 1 : 0);
   a.s = pb.s;
   a.erow_stride = 3;
   a.fcol_stride = 2;

@@ -23,9 +23,9 @@
 // by the second).  Measured at n = 8192, L = 16, against the passes they
 // replace (midrad planes stored and read back, 204 and 317 integer
 // instructions per entry): maxima 0.95 -> 0.32 ms (6.6 TB/s), splits 1.62 ->
-// 1.42 ms (5.3 TB/s).  1225 x 1225 x 12544: 376 -> 82 us and 399 -> 334 us
+// 1.26 ms (6.0 TB/s).  1225 x 1225 x 12544: 376 -> 82 us and 399 -> 280 us
 // (one warp took a whole column before).  n = 512: 13 launches before the
-// slice GEMM and after it, 5 now; the call 98 -> 53 us.
+// slice GEMM and after it, 5 now; the call 98 -> 47 us.
 //
 // A factor may also be given as plain doubles (a point matrix: m = x, r = 0).
 // The digit planes of a radius product that does not run are not written.
