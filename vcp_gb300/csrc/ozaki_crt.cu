@@ -218,9 +218,19 @@ oz_radius_T_kernel(int M, int N, int Mp, size_t plane, const int32_t* __restrict
 // per SM, a few words spilled) 756 us at n = 8192, 128 registers 815 us.
 
 constexpr int ASM_ROWS = 128, ASM_COLS = 64, ASM_NT = 256;
-// Exponents within +-ASM_EXP keep every value of an entry a normal double:
-// the path below that adds to exponent fields without looking.
-constexpr int ASM_EXP = 400;
+// The direct path below adds to exponent fields without looking: every value of
+// an entry has to be a normal double (or 0).  With |X| in [1, 2^(2w + 18)], sA in
+// [2^(w - 2), 2^(w + 20)], beta in [2^(F - 2), 2^(F + 20)] (k <= 2^20) and folds in
+// [2^-16, 2^52] that holds where the exponents of a factor pair sum up to
+//   E + F in [2 w - 1020, ASM_HI],  Ep + Fr and Er + F in [ASM_RAD_LO, ASM_HI]
+// and F, for beta itself, lies in [ASM_COL_LO, ASM_COL_HI].  A zero radius row or
+// column has zero folds: any exponent gives its 0.  Entries of a zero row or column
+// take the general path, which has little to do there; a block looks at its columns
+// one by one only where not all of them are in range.  (Limits of +-400 on each
+// exponent, and the general path an entry at a time after the direct one: 3000 x
+// 3000, k = 64, a zero row in four 605 us, now 310; factors over 2^450 690, now 279;
+// rows and columns over 2^+-600 866, now 613.)
+constexpr int ASM_HI = 990, ASM_RAD_LO = -970, ASM_COL_LO = -1020, ASM_COL_HI = 1003;
 
 // (rows as one array per quantity: a thread reads its 4 as one vector, a
 // warp's vectors lie side by side, free of bank conflicts)
@@ -234,14 +244,26 @@ struct AsmCol {
   int Fm, Fr;
   float q1, q2;     // roots of the low digits' squares of rB, |mB|
 };
+// What the entries of a product read and write.  res and P point at row /
+// column 0 of the product (plane = Np Mp of its layout).
+struct AsmArgs {
+  int M, Mp, L, w;
+  const uint8_t* res;
+  size_t plane;
+  const int32_t* P;
+  double* C;
+  double* Cup;  // not null: plain matrices, lower ends to C, upper ends to Cup
+  long ldc;
+  bool nonfinite, al16;
+};
 struct AsmTile {
   AsmRows row;
   AsmCol col[ASM_COLS];
+  // of each warp's 32 columns: least and largest Fm, Fr of those that have one;
+  // a zero column
+  int minF[2], maxF[2], minR[2], maxR[2], zeroF[2];
+  AsmArgs args;  // for the general path, which takes pointers
 };
-
-__device__ __forceinline__ bool asm_exp_ok(int e) { return e >= -ASM_EXP && e <= ASM_EXP; }
-// a zero radius row or column has zero folds: any exponent gives its 0
-__device__ __forceinline__ bool asm_rad_ok(int e) { return e == OZ_ZERO_EXP || asm_exp_ok(e); }
 
 // RU of asum_hi 2^32 + asum_lo (exact below 2^96).
 __device__ __forceinline__ double asum_ru(unsigned long long ah, unsigned long long al) {
@@ -266,93 +288,119 @@ __device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j
                                                int w, int lowb, const uint32_t* eA,
                                                const unsigned long long* asum, const uint32_t* eB,
                                                const unsigned long long* bsum) {
-  for (int x = threadIdx.x; x < ASM_ROWS + ASM_COLS; x += ASM_NT) {
-    if (x < ASM_ROWS) {
-      double sA = 0.0;
-      int E = OZ_ZERO_EXP, Ep = OZ_ZERO_EXP, Er = OZ_ZERO_EXP;
-      float qp = 0.0f, qr = 0.0f;
-      if (x < nr) {
-        const int i = i0 + x;
-        E = exp_dec(eA[3 * i]);
-        Ep = exp_dec(eA[3 * i + 1]);
-        Er = exp_dec(eA[3 * i + 2]);
-        sA = asum_ru(asum[4 * i], asum[4 * i + 1]);
-        if (lowb) {
-          qp = lowpair_root(asum[4 * i + 2], 0x1p-8f);
-          qr = lowpair_root(asum[4 * i + 3], 0x1p-8f);
-        }
+  const int x = threadIdx.x;
+  if (x < ASM_ROWS) {
+    double sA = 0.0;
+    int E = OZ_ZERO_EXP, Ep = OZ_ZERO_EXP, Er = OZ_ZERO_EXP;
+    float qp = 0.0f, qr = 0.0f;
+    if (x < nr) {
+      const int i = i0 + x;
+      E = exp_dec(eA[3 * i]);
+      Ep = exp_dec(eA[3 * i + 1]);
+      Er = exp_dec(eA[3 * i + 2]);
+      sA = asum_ru(asum[4 * i], asum[4 * i + 1]);
+      if (lowb) {
+        qp = lowpair_root(asum[4 * i + 2], 0x1p-8f);
+        qr = lowpair_root(asum[4 * i + 3], 0x1p-8f);
       }
-      t.row.sA[x] = sA;
-      t.row.E[x] = E;
-      t.row.Ep[x] = Ep;
-      t.row.Er[x] = Er;
-      t.row.qp[x] = qp;
-      t.row.qr[x] = qr;
-    } else if (x - ASM_ROWS < nc) {
-      const int j = j0 + x - ASM_ROWS;
-      AsmCol c;
-      c.Fm = exp_dec(eB[2 * j]);
-      c.Fr = exp_dec(eB[2 * j + 1]);
-      c.beta = 0.0;
-      if (c.Fm != OZ_ZERO_EXP) {
-        const double v =
-            __fma_ru((double)bsum[4 * j], 0x1p32,
-                     (double)(bsum[4 * j + 1] + (unsigned long long)(K + 1) / 2));
-        c.beta = scale_dir2(v, c.Fm - w, true);
-      }
-      c.q1 = lowb ? lowpair_root(bsum[4 * j + 2], 1.0f) : 0.0f;
-      c.q2 = lowb ? lowpair_root(bsum[4 * j + 3], 1.0f) : 0.0f;
-      t.col[x - ASM_ROWS] = c;
+    }
+    t.row.sA[x] = sA;
+    t.row.E[x] = E;
+    t.row.Ep[x] = Ep;
+    t.row.Er[x] = Er;
+    t.row.qp[x] = qp;
+    t.row.qr[x] = qr;
+  } else if (x < ASM_ROWS + ASM_COLS) {  // two warps
+    const int jc = x - ASM_ROWS, j = j0 + jc;
+    const bool in = jc < nc;
+    AsmCol c;
+    c.Fm = in ? exp_dec(eB[2 * j]) : OZ_ZERO_EXP;
+    c.Fr = in ? exp_dec(eB[2 * j + 1]) : OZ_ZERO_EXP;
+    c.beta = 0.0;
+    c.q1 = c.q2 = 0.0f;
+    const bool zF = c.Fm == OZ_ZERO_EXP, zR = c.Fr == OZ_ZERO_EXP;
+    if (!zF) {
+      const double v = __fma_ru((double)bsum[4 * j], 0x1p32,
+                                (double)(bsum[4 * j + 1] + (unsigned long long)(K + 1) / 2));
+      c.beta = scale_dir2(v, c.Fm - w, true);
+    }
+    if (lowb && in) {
+      c.q1 = lowpair_root(bsum[4 * j + 2], 1.0f);
+      c.q2 = lowpair_root(bsum[4 * j + 3], 1.0f);
+    }
+    if (in) t.col[jc] = c;
+    const unsigned all = 0xffffffffu;
+    const int v0 = __reduce_min_sync(all, zF ? 30000 : c.Fm), v1 = __reduce_max_sync(all, c.Fm),
+              v2 = __reduce_min_sync(all, zR ? 30000 : c.Fr), v3 = __reduce_max_sync(all, c.Fr),
+              v4 = __any_sync(all, in && zF);
+    if ((x & 31) == 0) {
+      const int h = jc >> 5;
+      t.minF[h] = v0;
+      t.maxF[h] = v1;
+      t.minR[h] = v2;
+      t.maxR[h] = v3;
+      t.zeroF[h] = v4;
     }
   }
   __syncthreads();
 }
 
-// What the entries of a product read and write.  res and P point at row /
-// column 0 of the product (plane = Np Mp of its layout).
-struct AsmArgs {
-  int M, Mp, L, w;
-  const uint8_t* res;
-  size_t plane;
-  const int32_t* P;
-  double* C;
-  double* Cup;  // not null: plain matrices, lower ends to C, upper ends to Cup
-  long ldc;
-  bool nonfinite, al16;
-};
-
-// One entry (row x of the tile, column *col, element e of its planes) whose
-// exponents leave the direct path: the same operations with every range
-// looked at, from its residues again.  Out of line, so that neither its
-// registers nor its FP64 instructions weigh on the direct path.
-static __device__ __noinline__ double2 asm_entry_general(const AsmArgs* a, size_t e,
-                                                         const AsmRows* row, int x,
-                                                         const AsmCol* col, const CrtBasis* cc,
-                                                         const OzRadConst* rc) {
-  double lo = 0.0, up = 0.0, tr = 0.0;
-  const int E = row->E[x], F = col->Fm, w = a->w;
-  if (E != OZ_ZERO_EXP && F != OZ_ZERO_EXP) {
-    uint32_t V[OZ_CRT_GROUPS], mag[4];
-#pragma unroll
-    for (int g = 0; g < OZ_CRT_GROUPS; ++g) {
-      V[g] = 0;
-#pragma unroll
-      for (int l = 0; l < 3; ++l)
-        if (3 * g + l < a->L) V[g] += a->res[(size_t)(3 * g + l) * a->plane + e] * cc->a[g][l];
-    }
-    crt_reduce(V, *cc, mag);
-    const int neg = crt_abs(mag);
-    big_to_dir(mag, neg, E + F - 2 * w - cc->z, lo, up);
-    const double t1 = scale_pow2(col->beta, E - w - 1, true);
-    const double t2 = scale_pow2(row->sA[x], E + F - 2 * w - 1, true);
-    tr = __dadd_ru(t1, t2);
+__device__ __forceinline__ void asm_store(const AsmArgs& a, size_t c, double2 r) {
+  if (a.nonfinite) r.x = r.y = __longlong_as_double(0x7ff8000000000000LL);
+  if (a.Cup) {
+    a.C[c] = r.x;
+    a.Cup[c] = r.y;
+  } else if (a.al16) {
+    reinterpret_cast<double2*>(a.C)[c] = r;
+  } else {  // C may be only 8-byte aligned
+    a.C[2 * c] = r.x;
+    a.C[2 * c + 1] = r.y;
   }
-  const float S1 = rc->run1 ? __int_as_float(a->P[e]) : 0.0f,
-              S2 = rc->run2 ? __int_as_float(a->P[(size_t)rc->nslot * a->plane + e]) : 0.0f;
-  const double T = rad_T(S1, S2, row->Ep[x], row->Er[x], F, col->Fr, *rc,
-                         __fmul_ru(row->qp[x], col->q1), __fmul_ru(row->qr[x], col->q2));
-  const double err = __dadd_ru(tr, T);
-  return make_double2(__dsub_rd(lo, err), __dadd_ru(up, err));
+}
+
+// Entries of a column (rows i0 + q4 + u for the bits u of `rows`, column j, *col)
+// that the direct path leaves out: the same operations with every range looked at.  Out
+// of line, so that neither its registers nor its FP64 instructions weigh on the
+// direct path; everything by pointers into shared memory and the parameters.
+static __device__ __noinline__ void asm_quad_general(const AsmTile* t, int i0, int q4, int j,
+                                                     int rows, const AsmCol* col,
+                                                     const CrtBasis* cc, const OzRadConst* rc) {
+  const AsmArgs& a = t->args;
+  const int w = a.w, F = col->Fm;
+  const size_t e0 = (size_t)j * a.Mp + i0 + q4;
+  uint32_t pk[3 * OZ_CRT_GROUPS];
+#pragma unroll
+  for (int l = 0; l < 3 * OZ_CRT_GROUPS; ++l)
+    pk[l] = l < a.L ? *reinterpret_cast<const uint32_t*>(a.res + (size_t)l * a.plane + e0) : 0u;
+#pragma unroll 1
+  for (int u = 0; u < 4; ++u) {
+    if (!((rows >> u) & 1) || i0 + q4 + u >= a.M) continue;
+    const int x = q4 + u, E = t->row.E[x];
+    double lo = 0.0, up = 0.0, tr = 0.0;
+    if (E != OZ_ZERO_EXP && F != OZ_ZERO_EXP) {
+      uint32_t V[OZ_CRT_GROUPS], mag[4];
+      const uint32_t sel = 0x4440u + (uint32_t)u;
+#pragma unroll
+      for (int g = 0; g < OZ_CRT_GROUPS; ++g)
+        V[g] = __byte_perm(pk[3 * g], 0u, sel) * cc->a[g][0] +
+               __byte_perm(pk[3 * g + 1], 0u, sel) * cc->a[g][1] +
+               __byte_perm(pk[3 * g + 2], 0u, sel) * cc->a[g][2];
+      crt_reduce(V, *cc, mag);
+      const int neg = crt_abs(mag);
+      big_to_dir(mag, neg, E + F - 2 * w - cc->z, lo, up);
+      const double t1 = scale_pow2(col->beta, E - w - 1, true);
+      const double t2 = scale_pow2(t->row.sA[x], E + F - 2 * w - 1, true);
+      tr = __dadd_ru(t1, t2);
+    }
+    const float S1 = rc->run1 ? __int_as_float(a.P[e0 + u]) : 0.0f,
+                S2 = rc->run2 ? __int_as_float(a.P[(size_t)rc->nslot * a.plane + e0 + u]) : 0.0f;
+    const double T =
+        rad_T(S1, S2, t->row.Ep[x], t->row.Er[x], F, col->Fr, *rc,
+              __fmul_ru(t->row.qp[x], col->q1), __fmul_ru(t->row.qr[x], col->q2));
+    const double err = __dadd_ru(tr, T);
+    asm_store(a, (size_t)(i0 + x) + (size_t)j * a.ldc,
+              make_double2(__dsub_rd(lo, err), __dadd_ru(up, err)));
+  }
 }
 
 // RU(s) 2^x of a fold s >= 0 as a double (0 for 0): e20 = (x + 896) << 20.
@@ -366,7 +414,7 @@ __device__ __forceinline__ double asm_fold(float s, int e20) {
 // All entries of a thread: rows i0 + 4 q .. + 3 (q = thread % Rq) of the
 // columns j0 + thread / Rq + CW c of its block.  The 4 entries of a column run
 // the direct path together without a branch between them (their FP64
-// additions overlap); where exponents leave its range they are redone.
+// additions overlap).
 template <bool LOWB>
 __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int i0, int nr,
                                          int j0, int nc, const CrtBasis& cc,
@@ -375,28 +423,60 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
   const int slot = (int)threadIdx.x / Rq, q4 = 4 * ((int)threadIdx.x - slot * Rq);
   if (slot >= CW) return;
   const int i = i0 + q4;
-  // per-row words of the direct path
+  // per-row words of the direct path, zero rows (bits), and the column
+  // exponents that it takes: Fm in [loF, hiF], Fr in [loR, hiR]
   int E20[4], P20[4], R20[4], sAh[4], sAl[4];
   float qp[4], qr[4];
-  bool rows_ok = rc.R == 0;
+  int loF = ASM_COL_LO, hiF = ASM_COL_HI, loR = OZ_ZERO_EXP, hiR = -OZ_ZERO_EXP, zero = 0;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const int E = t.row.E[q4 + u], Ep = t.row.Ep[q4 + u], Er = t.row.Er[q4 + u];
     // (rows past M hold the zero exponent; they are not stored)
-    rows_ok = rows_ok && ((asm_exp_ok(E) && asm_rad_ok(Ep) && asm_rad_ok(Er)) || i + u >= a.M);
+    int E = t.row.E[q4 + u], Ep = t.row.Ep[q4 + u], Er = t.row.Er[q4 + u];
+    if (E == OZ_ZERO_EXP) {
+      zero |= 1 << u;
+      E = 0;
+    } else {
+      loF = max(loF, 2 * a.w - 1020 - E);
+      hiF = min(hiF, ASM_HI - E);
+    }
+    if (Er == OZ_ZERO_EXP) {
+      Er = 0;
+    } else {
+      loF = max(loF, ASM_RAD_LO - Er);
+      hiF = min(hiF, ASM_HI - Er);
+    }
+    if (Ep == OZ_ZERO_EXP) {
+      Ep = 0;
+    } else {
+      loR = max(loR, ASM_RAD_LO - Ep);
+      hiR = min(hiR, ASM_HI - Ep);
+    }
     E20[u] = E << 20;
-    P20[u] = ((Ep == OZ_ZERO_EXP ? 0 : Ep) - 8 * rc.t_ref + 896) << 20;
-    R20[u] = ((Er == OZ_ZERO_EXP ? 0 : Er) - 8 * rc.t_ref + 896) << 20;
+    P20[u] = (Ep - 8 * rc.t_ref + 896) << 20;
+    R20[u] = (Er - 8 * rc.t_ref + 896) << 20;
     const long long sb = __double_as_longlong(t.row.sA[q4 + u]);
     sAh[u] = (int)(sb >> 32) + ((E - 2 * a.w - 1) << 20);  // sA 2^(E - 2 w - 1)
     sAl[u] = (int)sb;
     qp[u] = LOWB ? t.row.qp[q4 + u] : 0.0f;
     qr[u] = LOWB ? t.row.qr[q4 + u] : 0.0f;
   }
+  // every column in range and none zero: nothing to look at column by column
+  const bool special = zero || t.zeroF[0] || t.zeroF[1] || rc.R != 0 ||
+                       min(t.minF[0], t.minF[1]) < loF || max(t.maxF[0], t.maxF[1]) > hiF ||
+                       min(t.minR[0], t.minR[1]) < loR || max(t.maxR[0], t.maxR[1]) > hiR;
   const int cX = (1149 - 2 * a.w - cc.z) << 20;
   for (int c = slot; c < nc; c += CW) {
     const int j = j0 + c;
     const AsmCol& col = t.col[c];
+    const int Fm = col.Fm, Fr = col.Fr;
+    if (special) {
+      const bool zF = Fm == OZ_ZERO_EXP, zR = Fr == OZ_ZERO_EXP;
+      const bool direct = rc.R == 0 && !zF && Fm >= loF && Fm <= hiF &&
+                          (zR || (Fr >= loR && Fr <= hiR));
+      const int redo = direct ? zero : 15;
+      if (redo) asm_quad_general(&t, i0, q4, j, redo, &col, &cc, &rc);
+      if (redo == 15) continue;
+    }
     const size_t e0 = (size_t)j * a.Mp + i;
     uint32_t pk[3 * OZ_CRT_GROUPS];
 #pragma unroll
@@ -414,8 +494,6 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
         V[u][g] = ((pk[3 * g] >> (8 * u)) & 255u) * a0 + ((pk[3 * g + 1] >> (8 * u)) & 255u) * a1 +
                   ((pk[3 * g + 2] >> (8 * u)) & 255u) * a2;
     }
-    const int Fm = col.Fm, Fr = col.Fr;
-    const bool direct = rows_ok && asm_exp_ok(Fm) && asm_rad_ok(Fr);
     const int F20 = Fm << 20, Fr20 = (Fr == OZ_ZERO_EXP ? 0 : Fr) << 20;
     const long long bb = __double_as_longlong(col.beta);
     const int bh = (int)(bb >> 32) - ((a.w + 1) << 20), bl = (int)bb;  // beta 2^(-w - 1)
@@ -450,27 +528,10 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
         err = __dadd_ru(err, b2);
       r[u] = make_double2(__dsub_rd(lo, err), __dadd_ru(hi, err));
     }
-    if (!direct) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (i + u < a.M)
-          r[u] = asm_entry_general(&a, e0 + u, &t.row, q4 + u, &col, &cc, &rc);
-    }
     const size_t c0 = (size_t)i + (size_t)j * a.ldc;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (a.nonfinite) r[u].x = r[u].y = __longlong_as_double(0x7ff8000000000000LL);
-      if (i + u >= a.M) continue;
-      if (a.Cup) {
-        a.C[c0 + u] = r[u].x;
-        a.Cup[c0 + u] = r[u].y;
-      } else if (a.al16) {
-        reinterpret_cast<double2*>(a.C)[c0 + u] = r[u];
-      } else {  // C may be only 8-byte aligned
-        a.C[2 * (c0 + u)] = r[u].x;
-        a.C[2 * (c0 + u) + 1] = r[u].y;
-      }
-    }
+    for (int u = 0; u < 4; ++u)
+      if (i + u < a.M && !((zero >> u) & 1)) asm_store(a, c0 + u, r[u]);
   }
 }
 
@@ -495,9 +556,10 @@ oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB, const 
   const int ncb = (N + CB - 1) / CB;
   const int i0 = (int)(blockIdx.x / ncb) * ASM_ROWS, nr = min(ASM_ROWS, M - i0);
   const int j0 = (int)(blockIdx.x % ncb) * CB, nc = min(CB, N - j0);
-  asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, eA, asum, eB, bsum);
   const AsmArgs a{M, Mp, L, w, res, plane, P, C, Cup, ldc, f0 != 0 || f1 != 0,
                   (((uintptr_t)C) & 15) == 0};
+  if (threadIdx.x == 0) t.args = a;
+  asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, eA, asum, eB, bsum);
   asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
 }
 
@@ -520,11 +582,12 @@ oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ C
   const int i0 = (local % tm) * ASM_ROWS, nr = min(ASM_ROWS, m - i0);
   const int j0 = (local / tm) * OZ_GASM_COLS, nc = min(OZ_GASM_COLS, n - j0);
   const int f0 = b.flag[4 * p], f1 = b.flag[4 * p + 1];
+  const AsmArgs a{m, q.Mp, q.L, q.w, b.res + q.res_off, (size_t)q.Np * q.Mp, b.P + q.P_off, q.C,
+                  nullptr, q.ldc, f0 != 0 || b.flag[1] != 0, (((uintptr_t)q.C) & 15) == 0};
+  if (threadIdx.x == 0) t.args = a;
   asm_tile_setup(t, i0, nr, j0, nc, q.k, q.w, LOWB, b.eA + 3 * (size_t)q.rowoff,
                  b.asum + 4 * (size_t)q.rowoff, b.eB + 2 * (size_t)q.coloff,
                  b.bsum + 4 * (size_t)q.coloff);
-  const AsmArgs a{m, q.Mp, q.L, q.w, b.res + q.res_off, (size_t)q.Np * q.Mp, b.P + q.P_off, q.C,
-                  nullptr, q.ldc, f0 != 0 || b.flag[1] != 0, (((uintptr_t)q.C) & 15) == 0};
   asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
   if (threadIdx.x == 0 && (f0 | f1)) atomicOr(&g_oz_status, (f0 ? 1 : 0) | (f1 ? 2 : 0));
   if (b.t_last) {
@@ -538,6 +601,7 @@ oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ C
 }
 
 static_assert(OZ_GASM_COLS <= ASM_COLS, "column data of a grouped tile");
+static_assert(ASM_ROWS + ASM_COLS <= ASM_NT && ASM_COLS == 64, "one thread a row or column");
 
 }  // namespace
 
