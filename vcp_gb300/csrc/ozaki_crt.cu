@@ -215,7 +215,7 @@ oz_radius_T_kernel(int M, int N, int Mp, size_t plane, const int32_t* __restrict
 // 128-bit product per residue, 8 columns a thread and a branch per entry:
 // n = 8192 1.49 -> 0.76 ms, n = 512 48 -> 10 us (64 blocks before), 17 chunks
 // of a 256-problem batch 1.30 -> 0.54 ms summed.  80 registers (three blocks
-// per SM, a few words spilled) 756 us at n = 8192, 128 registers 815 us.
+// per SM, a few words spilled) 752 us at n = 8192, 128 registers 815 us.
 
 constexpr int ASM_ROWS = 128, ASM_COLS = 64, ASM_NT = 256;
 // The direct path below adds to exponent fields without looking: every value of
@@ -225,11 +225,10 @@ constexpr int ASM_ROWS = 128, ASM_COLS = 64, ASM_NT = 256;
 //   E + F in [2 w - 1020, ASM_HI],  Ep + Fr and Er + F in [ASM_RAD_LO, ASM_HI]
 // and F, for beta itself, lies in [ASM_COL_LO, ASM_COL_HI].  A zero radius row or
 // column has zero folds: any exponent gives its 0.  Entries of a zero row or column
-// take the general path, which has little to do there; a block looks at its columns
-// one by one only where not all of them are in range.  (Limits of +-400 on each
+// take the general path, which has little to do there.  (Limits of +-400 on each
 // exponent, and the general path an entry at a time after the direct one: 3000 x
-// 3000, k = 64, a zero row in four 605 us, now 310; factors over 2^450 690, now 279;
-// rows and columns over 2^+-600 866, now 613.)
+// 3000, k = 64, a zero row in four 605 us, now 351; factors over 2^450 690, now 267;
+// rows and columns over 2^+-600 866, now 623.)
 constexpr int ASM_HI = 990, ASM_RAD_LO = -970, ASM_COL_LO = -1020, ASM_COL_HI = 1003;
 
 // (rows as one array per quantity: a thread reads its 4 as one vector, a
@@ -258,6 +257,10 @@ struct AsmArgs {
 };
 struct AsmTile {
   AsmRows row;
+  // of each quad of rows: the column exponents that its direct path takes, Fm in
+  // [x, y] and Fr in [z, w]; its zero rows (bits)
+  int4 takes[ASM_ROWS / 4];
+  int zero[ASM_ROWS / 4];
   AsmCol col[ASM_COLS];
   // of each warp's 32 columns: least and largest Fm, Fr of those that have one;
   // a zero column
@@ -310,6 +313,30 @@ __device__ __forceinline__ void asm_tile_setup(AsmTile& t, int i0, int nr, int j
     t.row.Er[x] = Er;
     t.row.qp[x] = qp;
     t.row.qr[x] = qr;
+    const unsigned all = 0xffffffffu;
+    const bool z = E == OZ_ZERO_EXP;
+    int loF = z ? ASM_COL_LO : max(ASM_COL_LO, 2 * w - 1020 - E),
+        hiF = z ? ASM_COL_HI : min(ASM_COL_HI, ASM_HI - E), loR = OZ_ZERO_EXP, hiR = -OZ_ZERO_EXP;
+    if (Er != OZ_ZERO_EXP) {
+      loF = max(loF, ASM_RAD_LO - Er);
+      hiF = min(hiF, ASM_HI - Er);
+    }
+    if (Ep != OZ_ZERO_EXP) {
+      loR = ASM_RAD_LO - Ep;
+      hiR = ASM_HI - Ep;
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      loF = max(loF, __shfl_xor_sync(all, loF, o));
+      hiF = min(hiF, __shfl_xor_sync(all, hiF, o));
+      loR = max(loR, __shfl_xor_sync(all, loR, o));
+      hiR = min(hiR, __shfl_xor_sync(all, hiR, o));
+    }
+    const unsigned zb = __ballot_sync(all, z && x < nr);
+    if ((x & 3) == 0) {
+      t.takes[x >> 2] = make_int4(loF, hiF, loR, hiR);
+      t.zero[x >> 2] = (zb >> (x & 28)) & 15;
+    }
   } else if (x < ASM_ROWS + ASM_COLS) {  // two warps
     const int jc = x - ASM_ROWS, j = j0 + jc;
     const bool in = jc < nc;
@@ -415,64 +442,41 @@ __device__ __forceinline__ double asm_fold(float s, int e20) {
 // columns j0 + thread / Rq + CW c of its block.  The 4 entries of a column run
 // the direct path together without a branch between them (their FP64
 // additions overlap).
-template <bool LOWB>
-__device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int i0, int nr,
-                                         int j0, int nc, const CrtBasis& cc,
-                                         const OzRadConst& rc) {
-  const int Rq = (nr + 3) >> 2, CW = ASM_NT / Rq;
-  const int slot = (int)threadIdx.x / Rq, q4 = 4 * ((int)threadIdx.x - slot * Rq);
-  if (slot >= CW) return;
+// SPECIAL: some row or column of the thread's may leave the direct path.  A copy
+// of its own and out of line (asm_entries_special), so that the loop of the others
+// holds neither the tests nor a call: n = 4096, k = 64 196 us, 211 with the tests in
+// one loop and 213 with the general path's calls at its end; the 256-problem batch
+// 1687, 1765 and 1707.  (Inlined beside the other, its registers cost the loop 323.)
+template <bool LOWB, bool SPECIAL>
+__device__ __forceinline__ void asm_entries(const AsmTile& t, const AsmArgs& a, int i0,
+                                            int q4, int slot, int CW, int j0, int nc,
+                                            const CrtBasis& cc, const OzRadConst& rc) {
   const int i = i0 + q4;
-  // per-row words of the direct path, zero rows (bits), and the column
-  // exponents that it takes: Fm in [loF, hiF], Fr in [loR, hiR]
+  // per-row words of the direct path (those of a zero row or radius go unused)
   int E20[4], P20[4], R20[4], sAh[4], sAl[4];
   float qp[4], qr[4];
-  int loF = ASM_COL_LO, hiF = ASM_COL_HI, loR = OZ_ZERO_EXP, hiR = -OZ_ZERO_EXP, zero = 0;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    // (rows past M hold the zero exponent; they are not stored)
-    int E = t.row.E[q4 + u], Ep = t.row.Ep[q4 + u], Er = t.row.Er[q4 + u];
-    if (E == OZ_ZERO_EXP) {
-      zero |= 1 << u;
-      E = 0;
-    } else {
-      loF = max(loF, 2 * a.w - 1020 - E);
-      hiF = min(hiF, ASM_HI - E);
-    }
-    if (Er == OZ_ZERO_EXP) {
-      Er = 0;
-    } else {
-      loF = max(loF, ASM_RAD_LO - Er);
-      hiF = min(hiF, ASM_HI - Er);
-    }
-    if (Ep == OZ_ZERO_EXP) {
-      Ep = 0;
-    } else {
-      loR = max(loR, ASM_RAD_LO - Ep);
-      hiR = min(hiR, ASM_HI - Ep);
-    }
+    const int E = t.row.E[q4 + u];
     E20[u] = E << 20;
-    P20[u] = (Ep - 8 * rc.t_ref + 896) << 20;
-    R20[u] = (Er - 8 * rc.t_ref + 896) << 20;
+    P20[u] = (t.row.Ep[q4 + u] - 8 * rc.t_ref + 896) << 20;
+    R20[u] = (t.row.Er[q4 + u] - 8 * rc.t_ref + 896) << 20;
     const long long sb = __double_as_longlong(t.row.sA[q4 + u]);
     sAh[u] = (int)(sb >> 32) + ((E - 2 * a.w - 1) << 20);  // sA 2^(E - 2 w - 1)
     sAl[u] = (int)sb;
     qp[u] = LOWB ? t.row.qp[q4 + u] : 0.0f;
     qr[u] = LOWB ? t.row.qr[q4 + u] : 0.0f;
   }
-  // every column in range and none zero: nothing to look at column by column
-  const bool special = zero || t.zeroF[0] || t.zeroF[1] || rc.R != 0 ||
-                       min(t.minF[0], t.minF[1]) < loF || max(t.maxF[0], t.maxF[1]) > hiF ||
-                       min(t.minR[0], t.minR[1]) < loR || max(t.maxR[0], t.maxR[1]) > hiR;
+  const int zero = SPECIAL ? t.zero[q4 >> 2] : 0;
   const int cX = (1149 - 2 * a.w - cc.z) << 20;
   for (int c = slot; c < nc; c += CW) {
     const int j = j0 + c;
     const AsmCol& col = t.col[c];
     const int Fm = col.Fm, Fr = col.Fr;
-    if (special) {
-      const bool zF = Fm == OZ_ZERO_EXP, zR = Fr == OZ_ZERO_EXP;
-      const bool direct = rc.R == 0 && !zF && Fm >= loF && Fm <= hiF &&
-                          (zR || (Fr >= loR && Fr <= hiR));
+    if (SPECIAL) {
+      const int4 f = t.takes[q4 >> 2];
+      const bool direct = rc.R == 0 && Fm >= f.x && Fm <= f.y &&  // (a zero column's is below)
+                          (Fr == OZ_ZERO_EXP || (Fr >= f.z && Fr <= f.w));
       const int redo = direct ? zero : 15;
       if (redo) asm_quad_general(&t, i0, q4, j, redo, &col, &cc, &rc);
       if (redo == 15) continue;
@@ -494,7 +498,7 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
         V[u][g] = ((pk[3 * g] >> (8 * u)) & 255u) * a0 + ((pk[3 * g + 1] >> (8 * u)) & 255u) * a1 +
                   ((pk[3 * g + 2] >> (8 * u)) & 255u) * a2;
     }
-    const int F20 = Fm << 20, Fr20 = (Fr == OZ_ZERO_EXP ? 0 : Fr) << 20;
+    const int F20 = Fm << 20, Fr20 = Fr << 20;
     const long long bb = __double_as_longlong(col.beta);
     const int bh = (int)(bb >> 32) - ((a.w + 1) << 20), bl = (int)bb;  // beta 2^(-w - 1)
     double2 r[4];
@@ -535,6 +539,28 @@ __device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int
   }
 }
 
+template <bool LOWB>
+static __device__ __noinline__ void asm_entries_special(const AsmTile* t, int i0, int q4, int slot,
+                                                        int CW, int j0, int nc, const CrtBasis* cc,
+                                                        const OzRadConst* rc) {
+  asm_entries<LOWB, true>(*t, t->args, i0, q4, slot, CW, j0, nc, *cc, *rc);
+}
+template <bool LOWB>
+__device__ __forceinline__ void asm_tile(const AsmTile& t, const AsmArgs& a, int i0, int nr,
+                                         int j0, int nc, const CrtBasis& cc,
+                                         const OzRadConst& rc) {
+  const int Rq = (nr + 3) >> 2, CW = ASM_NT / Rq;
+  const int slot = (int)threadIdx.x / Rq, q4 = 4 * ((int)threadIdx.x - slot * Rq);
+  if (slot >= CW) return;
+  const int4 in = t.takes[q4 >> 2];
+  if (t.zero[q4 >> 2] || t.zeroF[0] || t.zeroF[1] || rc.R != 0 ||
+      min(t.minF[0], t.minF[1]) < in.x || max(t.maxF[0], t.maxF[1]) > in.y ||
+      min(t.minR[0], t.minR[1]) < in.z || max(t.maxR[0], t.maxR[1]) > in.w)
+    asm_entries_special<LOWB>(&t, i0, q4, slot, CW, j0, nc, &cc, &rc);
+  else
+    asm_entries<LOWB, false>(t, a, i0, q4, slot, CW, j0, nc, cc, rc);
+}
+
 // One product: blocks over the column ranges of CB columns, then over the
 // 128-row tiles (one dimension: no limit on either).  Block 0 merges the
 // status words.  (No __restrict__, here and in what it calls: the kernel may
@@ -558,7 +584,7 @@ oz_crt_assemble_kernel(int M, int N, int K, int Mp, int L, int w, int CB, const 
   const int j0 = (int)(blockIdx.x % ncb) * CB, nc = min(CB, N - j0);
   const AsmArgs a{M, Mp, L, w, res, plane, P, C, Cup, ldc, f0 != 0 || f1 != 0,
                   (((uintptr_t)C) & 15) == 0};
-  if (threadIdx.x == 0) t.args = a;
+  if (threadIdx.x == ASM_NT - 1) t.args = a;  // (no row or column of its own)
   asm_tile_setup(t, i0, nr, j0, nc, K, w, LOWB, eA, asum, eB, bsum);
   asm_tile<LOWB>(t, a, i0, nr, j0, nc, cc, rc);
 }
@@ -584,7 +610,7 @@ oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ C
   const int f0 = b.flag[4 * p], f1 = b.flag[4 * p + 1];
   const AsmArgs a{m, q.Mp, q.L, q.w, b.res + q.res_off, (size_t)q.Np * q.Mp, b.P + q.P_off, q.C,
                   nullptr, q.ldc, f0 != 0 || b.flag[1] != 0, (((uintptr_t)q.C) & 15) == 0};
-  if (threadIdx.x == 0) t.args = a;
+  if (threadIdx.x == ASM_NT - 1) t.args = a;  // (no row or column of its own)
   asm_tile_setup(t, i0, nr, j0, nc, q.k, q.w, LOWB, b.eA + 3 * (size_t)q.rowoff,
                  b.asum + 4 * (size_t)q.rowoff, b.eB + 2 * (size_t)q.coloff,
                  b.bsum + 4 * (size_t)q.coloff);
@@ -601,7 +627,7 @@ oz_crt_assemble_g(const __grid_constant__ OzGBucket b, const __grid_constant__ C
 }
 
 static_assert(OZ_GASM_COLS <= ASM_COLS, "column data of a grouped tile");
-static_assert(ASM_ROWS + ASM_COLS <= ASM_NT && ASM_COLS == 64, "one thread a row or column");
+static_assert(ASM_ROWS + ASM_COLS < ASM_NT && ASM_COLS == 64, "one thread a row or column");
 
 }  // namespace
 
